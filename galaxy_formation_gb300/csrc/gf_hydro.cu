@@ -668,7 +668,7 @@ void ForceEngine::hydro(const ForceArgs& a, cudaStream_t s) {
         GF_CUDA(cudaMemsetAsync(&sc->knn_iters, 0, sizeof(unsigned long long), s));
         // the gas of the last full search, moved (same count): rebuild without a host round trip
         knn_exact(knn_tree, ng, gp, kq, rg, nullptr, nullptr, &sc->knn_iters, s, nb, kCand, d31, kNgb - 1,
-                  features ? &hg : nullptr, order_ng == ng, vsel_);
+                  features ? &hg : nullptr, order_ng == ng, vsel_, hguess == 1);
         if (collect) {
             const long long take = std::min<long long>(ng, (collect_cap - collect_n) / 2);  // two rows each
             if (take > 0) {

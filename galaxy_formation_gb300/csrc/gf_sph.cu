@@ -14,8 +14,9 @@
 //                              from hi/lo split coordinates) until the count lies in
 //                              [k, 128] — the radius iteration, Newton steps on
 //                              count ~ R^3 from a guess (2.5 x the previous h, 1.06 x the
-//                              learned guess of the k-th-neighbour distance, or the leaf's
-//                              cell density). The collected points are sorted,
+//                              learned guess of the k-th-neighbour distance, a rank of the
+//                              distances to the points next to the query in the tree's
+//                              order, or the leaf's cell density). The collected points are sorted,
 //                              the k nearest plus near-ties at the boundary are re-measured
 //                              in float64 and sorted again, so the result is the exact
 //                              float64 kNN.
@@ -291,6 +292,8 @@ struct KnnArgs {
     uint32_t* status;
     unsigned long long* iters;
     const int* wparent;     // breadth-first parent of each node (-1 for the root)
+    int window_rank;        // without r_guess: start at this rank of the distances to the points
+                            // next to the query in tree order (0: at the leaf's cell density)
     int exact_order;        // 1: float64 re-sort of the k nearest; 0: float32 order, float64
                             //    only to settle the neighbour at dsel_col (the h boundary)
 };
@@ -298,7 +301,8 @@ struct KnnArgs {
 // Collects, for each of the warp's (up to) two queries that is on, the points within its radius
 // into S.key[i] (the first kKnnCap of them) and their number into cnt[i]; one walk serves both:
 // a node is opened when it meets either sphere, and each point of an opened leaf is tested
-// against both. Returns false on stack overflow. The two queries of a warp are neighbours in
+// against both. A query with more than kKnnCap points is done with this radius: its sphere opens
+// no further nodes (cnt[i] then is only known to exceed kKnnCap). Returns false on stack overflow. The two queries of a warp are neighbours in
 // the tree's order (usually in one leaf), so their walks share most nodes.
 __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2], int leaf, int (&cnt)[2]) {
     const int lane = threadIdx.x & 31;
@@ -322,10 +326,11 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2]
     }
     if (start < 0) start = 0;
     cnt[0] = cnt[1] = 0;
+    bool live[2] = {Q[0].on, Q[1].on};  // still collecting (warp-uniform)
     int sp = 1;
     if (lane == 0) S.stack[0] = (start << 4) | 1;
     __syncwarp();
-    for (int rounds = 0; sp > 0; ++rounds) {
+    for (int rounds = 0; sp > 0 && (live[0] || live[1]); ++rounds) {
         if (rounds > A.nn) return false;  // each node is popped at most once
         // pop up to 64 nodes (two per lane: their loads overlap)
         int node[2];
@@ -352,7 +357,7 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2]
                 const float lim = g.w + 2e-6f * (fabsf(g.x) + fabsf(g.y) + fabsf(g.z) + g.w) + 1e-30f;
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    if (!Q[i].on) continue;
+                    if (!live[i]) continue;
                     const float ex = fmaxf(fabsf((g.x - Q[i].xh.x) - Q[i].xl.x) - lim, 0.f);
                     const float ey = fmaxf(fabsf((g.y - Q[i].xh.y) - Q[i].xl.y) - lim, 0.f);
                     const float ez = fmaxf(fabsf((g.z - Q[i].xh.z) - Q[i].xl.z) - lim, 0.f);
@@ -397,7 +402,7 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2]
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                if (!Q[i].on) continue;
+                if (!live[i]) continue;
                 const float dx = (ph.x - Q[i].xh.x) + (pl.x - Q[i].xl.x);
                 const float dy = (ph.y - Q[i].xh.y) + (pl.y - Q[i].xl.y);
                 const float dz = (ph.z - Q[i].xh.z) + (pl.z - Q[i].xl.z);
@@ -411,6 +416,8 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2]
                 cnt[i] += __popc(hm);
             }
         }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) live[i] = live[i] && cnt[i] <= kKnnCap;
         }  // any leaf
         __syncwarp();
     }
@@ -540,19 +547,97 @@ __device__ void knn_fail_output(const KnnArgs& A, int q, bool stack) {
     if (A.dsel_idx && lane == 0) A.dsel_idx[oq] = -1;
 }
 
-// Radius step of the count-to-k iteration: Newton on count ~ R^3 until the count is
-// bracketed by [lo, hi], bisection afterwards.
-__device__ __forceinline__ float knn_next_radius(float R, int cnt, int k, int cap, float& lo, float& hi) {
-    float next;
-    if (cnt < k) {
-        lo = R;
-        next = R * (cnt >= 4 ? cbrtf(1.3f * float(k) / float(cnt)) : 2.0f);
-    } else {
-        hi = R;
-        next = R * cbrtf(0.75f * float(cap) / float(cnt));
+// Radius from the density of the query's leaf cell.
+__device__ __forceinline__ float knn_cell_radius(const KnnArgs& A, int q) {
+    const int lf = A.leaf_of[q];
+    const float half = A.wgeo[lf].w;
+    const int c = max(1, -__float_as_int(A.wb[lf].z));
+    return 2.0f * half * cbrtf(float(A.k) / float(c));
+}
+
+// A radius that encloses at least `rank` of kPer * 32 points, kPer per lane, given as the upper
+// kKnnRankBits bits of their float32 squared distances (their order is the bits' order; all ones:
+// no point): bisection on those bits, each step one compare per point and one warp sum. The
+// radius is the upper edge of the bucket that reaches the rank.
+constexpr int kKnnRankBits = 12;  // exponent and 4 bits of mantissa: 6 % in d^2, 3 % in the radius
+constexpr int kKnnRankShift = 31 - kKnnRankBits;  // the sign bit is 0
+
+template <int kPer>
+__device__ __forceinline__ float knn_rank_radius(const unsigned (&b)[kPer], int rank) {
+    unsigned lo = 0, hi = (1u << kKnnRankBits) - 1u;
+    while (lo < hi) {
+        const unsigned mid = (lo + hi) >> 1;
+        int c = 0;
+#pragma unroll
+        for (int t = 0; t < kPer; ++t) c += b[t] <= mid ? 1 : 0;
+        if (__reduce_add_sync(0xffffffffu, c) >= rank)
+            hi = mid;
+        else
+            lo = mid + 1;
     }
-    if (lo > 0.f && hi < INFINITY) next = 0.5f * (lo + hi);
-    return next;
+    // padded so that a distance tied with the edge to rounding is inside
+    return sqrtf(__uint_as_float((lo + 1) << kKnnRankShift)) * 1.0001f;
+}
+
+// Starting radii of a warp's two queries without a previous h: the kKnnWindow points around them
+// in tree order hold most of the nearest ones, so the radius that encloses window_rank of them
+// encloses about k of all points. The first search of the 1M disk's 500k gas is bound by the
+// points its spheres collect: from the leaf's cell density, whose one to eight points say little,
+// spheres held hundreds to thousands of them (8.70 ms); from here, with collections that stop at the
+// cap, 3.22 ms (2.10 ms with a previous h).
+constexpr int kKnnWindow = 128;
+
+__device__ __forceinline__ void knn_window_radii(const KnnArgs& A, int q0, KnnQuery (&Q)[2]) {
+    constexpr int kPer = kKnnWindow / 32;
+    const int lane = threadIdx.x & 31;
+    const int w0 = max(0, min(q0 - kKnnWindow / 2 + 1, A.n - kKnnWindow));
+    unsigned b[2][kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        const int j = w0 + 32 * t + lane;
+        b[0][t] = b[1][t] = 0xffffffffu;
+        if (j < A.n) {
+            const float4 ph = A.p4[j], pl = A.plo[j];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (!Q[i].on) continue;
+                const float dx = (ph.x - Q[i].xh.x) + (pl.x - Q[i].xl.x);
+                const float dy = (ph.y - Q[i].xh.y) + (pl.y - Q[i].xl.y);
+                const float dz = (ph.z - Q[i].xh.z) + (pl.z - Q[i].xl.z);
+                b[i][t] = __float_as_uint(dx * dx + dy * dy + dz * dz) >> kKnnRankShift;
+            }
+        }
+    }
+    const int rank = min(A.window_rank, min(A.n, kKnnWindow));
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        if (Q[i].on) Q[i].R = knn_rank_radius<kPer>(b[i], rank);
+}
+
+// Next radius of a query whose sphere holds more than kKnnCap points (key: kKnnCap of them): the
+// sphere around k + kKnnShrink of those, or smaller than R by what one point too many implies.
+constexpr int kKnnShrink = 8;
+
+__device__ __forceinline__ float knn_shrunk_radius(const unsigned long long* key, int k, float R) {
+    constexpr int kPer = kKnnCap / 32;
+    const int lane = threadIdx.x & 31;
+    unsigned b[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) b[t] = unsigned(key[32 * t + lane] >> 32) >> kKnnRankShift;
+    return fminf(knn_rank_radius<kPer>(b, k + kKnnShrink), 0.9f * R);
+}
+
+// Radius step of the count-to-k iteration: Newton on count ~ R^3 below k, a rank of the
+// collected distances above the cap, until the count is bracketed; bisection afterwards.
+__device__ __forceinline__ float knn_next_radius(float R, int cnt, int k, const unsigned long long* key, float& lo,
+                                                 float& hi) {
+    if (cnt < k)
+        lo = R;
+    else
+        hi = R;
+    if (lo > 0.f && hi < INFINITY) return 0.5f * (lo + hi);
+    if (cnt < k) return R * (cnt >= 4 ? cbrtf(1.3f * float(k) / float(cnt)) : 2.0f);
+    return knn_shrunk_radius(key, k, R);
 }
 
 // One warp per pair of consecutive queries (tree order): walk from the smallest ancestor cell
@@ -570,7 +655,9 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 4) k_knn(KnnArgs A) {
     for (int q0 = 2 * (blockIdx.x * kKnnWarps + (threadIdx.x >> 5)); q0 < A.n; q0 += 2 * nwarps) {
         KnnQuery Q[2];
         float lo[2], hi[2];
-        int it[2] = {0, 0};
+        int it[2] = {0, 0}, total = 0;
+        const bool window = !A.r_guess && A.window_rank > 0;
+        bool from_window[2] = {window, window};
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int q = q0 + i;
@@ -580,18 +667,13 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 4) k_knn(KnnArgs A) {
             if (!Q[i].on) continue;
             Q[i].xh = A.p4[q];
             Q[i].xl = A.plo[q];
-            float R;
-            if (A.r_guess) {
-                R = A.r_guess[A.perm[q]];
-            } else {  // from the density of the particle's leaf cell
-                const int lf = A.leaf_of[q];
-                const float half = A.wgeo[lf].w;
-                const int c = max(1, -__float_as_int(A.wb[lf].z));
-                R = 2.0f * half * cbrtf(float(k) / float(c));
-            }
-            if (!(R > 0.f) || !isfinite(R)) R = 1e-3f;
-            Q[i].R = R;
-            Q[i].R2 = R * R;
+            if (!window) Q[i].R = A.r_guess ? A.r_guess[A.perm[q]] : knn_cell_radius(A, q);
+        }
+        if (window) knn_window_radii(A, q0, Q);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (!(Q[i].R > 0.f) || !isfinite(Q[i].R)) Q[i].R = 1e-3f;
+            Q[i].R2 = Q[i].R * Q[i].R;
         }
         while (Q[0].on || Q[1].on) {
             int cnt[2];
@@ -601,22 +683,28 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 4) k_knn(KnnArgs A) {
             for (int i = 0; i < 2; ++i) {
                 if (!Q[i].on) continue;
                 ++it[i];
-                if (!ok_walk) {
-                    knn_fail_output(A, q0 + i, true);
-                    Q[i].on = false;
-                } else if (cnt[i] >= k && cnt[i] <= cap) {
+                ++total;
+                if (ok_walk && cnt[i] >= k && cnt[i] <= cap) {
                     knn_finish(A, S.key[i], S.dd, S.di, cnt[i], q0 + i);
                     Q[i].on = false;
-                } else if (it[i] >= 48) {
-                    knn_fail_output(A, q0 + i, false);
-                    Q[i].on = false;
-                } else {
-                    Q[i].R = knn_next_radius(Q[i].R, cnt[i], k, cap, lo[i], hi[i]);
+                } else if (ok_walk && it[i] < 48) {
+                    Q[i].R = knn_next_radius(Q[i].R, cnt[i], k, S.key[i], lo[i], hi[i]);
                     Q[i].R2 = Q[i].R * Q[i].R;
+                } else if (from_window[i]) {  // once more, from the cell density
+                    from_window[i] = false;
+                    it[i] = 0;
+                    lo[i] = 0.f;
+                    hi[i] = INFINITY;
+                    Q[i].R = knn_cell_radius(A, q0 + i);
+                    if (!(Q[i].R > 0.f) || !isfinite(Q[i].R)) Q[i].R = 1e-3f;
+                    Q[i].R2 = Q[i].R * Q[i].R;
+                } else {
+                    knn_fail_output(A, q0 + i, !ok_walk);
+                    Q[i].on = false;
                 }
             }
         }
-        if (lane == 0 && A.iters) atomicAdd(A.iters, (unsigned long long)(it[0] + it[1]));
+        if (lane == 0 && A.iters) atomicAdd(A.iters, (unsigned long long)total);
     }
 }
 
@@ -700,9 +788,14 @@ __global__ void k_guess_from_logdk(int n, const float* __restrict__ Y, float* __
     if (i < n) rg[i] = kFarMargin * expf(Y[i]);
 }
 
+// Rank of the window distances that a search without a previous h starts at: 3/4 of k, since the
+// window misses a part of the sphere (36 for the 48 nearest: 34 and 38 are 0.5 % and 3 % slower,
+// 46 15 %), and at least 24 (any count from k to the cap settles a query).
+static int knn_window_rank(int k) { return std::max(24, (3 * k + 3) / 4); }
+
 void knn_exact(Octree& T, int n, const double* pos, int k, const float* r_guess, int64_t* nb,
                double* dist, unsigned long long* d_iters, cudaStream_t s, int* nb32, int ld32,
-               double* dsel, int dsel_col, const HGuess* hg, bool same_set, int* dsel_idx) {
+               double* dsel, int dsel_col, const HGuess* hg, bool same_set, int* dsel_idx, bool cell_start) {
     if (n <= 0) return;
     // same_set (the caller's point set drifted since the last search): the synchronisation-free
     // rebuild inside the node buffers of the last regular build (no host round trip in the middle
@@ -752,6 +845,7 @@ void knn_exact(Octree& T, int n, const double* pos, int k, const float* r_guess,
     A.status = ctx().d_status;
     A.iters = d_iters;
     A.wparent = T.w_parent.as<int>();
+    A.window_rank = cell_start ? 0 : knn_window_rank(k);
     ProfScope ps(kStKnn, s);
     const int blocks = std::min(div_up(n, 2 * kKnnWarps), 16 * ctx().sms);  // two queries per warp
     k_knn<<<blocks, kKnnWarps * 32, 0, s>>>(A);

@@ -58,7 +58,9 @@ void knn_from_candidates(int n, int m, const double* pos, const int64_t* cand, i
                          double* dist, int* d_ok, cudaStream_t s);
 
 // Exact float64 k nearest neighbours of every point (itself included), ascending; builds
-// the point octree in T. r_guess (caller order, optional): starting search radius.
+// the point octree in T. r_guess (caller order, optional): starting search radius; without it
+// each query starts at a rank of the distances to the points next to it in the tree's order, or
+// (cell_start) at the radius its leaf cell's density implies.
 // Outputs either nb/dist (n,k) int64/float64, or nb32 (n, ld32) int32 plus the distance of
 // neighbour `dsel_col` in dsel (n,) — or, with dsel_idx, that neighbour's index (the caller
 // measures its float64 distance; -1 for a failed query). same_set: the points are those of the
@@ -66,7 +68,7 @@ void knn_from_candidates(int n, int m, const double* pos, const int64_t* cand, i
 void knn_exact(Octree& T, int n, const double* pos, int k, const float* r_guess, int64_t* nb,
                double* dist, unsigned long long* d_iters, cudaStream_t s, int* nb32 = nullptr,
                int ld32 = 0, double* dsel = nullptr, int dsel_col = -1, const HGuess* hg = nullptr,
-               bool same_set = false, int* dsel_idx = nullptr);
+               bool same_set = false, int* dsel_idx = nullptr, bool cell_start = false);
 
 void direct_sum(int n, const double* pos, const double* mass, int nt, const int64_t* targets,
                 double* acc, double eps, cudaStream_t s);

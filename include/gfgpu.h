@@ -346,10 +346,12 @@ int gf_cool(int n, const double* u, const double* T, const double* rho, const do
  *                           keeps its own tree; nbody_accel_active is never affected. */
 #define GF_OPT_GRAVITY_QUAD 1
 /*   GF_OPT_HGUESS       start of the neighbour-count iteration of a full search:
- *                       0 = 2.5 x the previous h (default), falling back to the density of the
- *                       particle's tree cell when there is none (the first search of a particle
- *                       set); 1 = the cell density only; 2 = 2.5 x the previous h, and the
- *                       learned guess (gf_mlp_*) where there is none. The iteration always runs
+ *                       0 = 2.5 x the previous h (default), falling back to a rank of the
+ *                       distances to the points next to it in the tree's order when there is
+ *                       none (the first search of a particle set); 1 = the density of the
+ *                       particle's tree cell only; 2 = 2.5 x the
+ *                       previous h, and the learned guess (gf_mlp_*) where there is none (without
+ *                       a network: as 0). The iteration always runs
  *                       to the exact 48 nearest, so only the iteration count changes. */
 #define GF_OPT_HGUESS 2
 /*   GF_OPT_COLLECT      capacity (rows) of a device buffer that every later full search with a
