@@ -107,17 +107,27 @@ __device__ __forceinline__ int warp_sum(int v) {
     return v;
 }
 
+// Segments laid end to end, in lane order, over a row of slots: the lane that holds a segment
+// (has) starting at slot `start` marks it, and slot `first_slot + lane` learns how many segments
+// start at or before it (`before` of them before first_slot), minus one: the rank of its own
+// segment. One OR-reduction of the 32 slots' start marks and a population count, where a binary
+// search over the prefix sums takes five dependent shuffles.
+__device__ __forceinline__ unsigned segment_marks(bool has, int start, int first_slot) {
+    const unsigned rel = unsigned(start - first_slot);
+    return __reduce_or_sync(0xffffffffu, has && rel < 32u ? 1u << rel : 0u);
+}
+
 // One round of a warp's tree walk over a shared-memory stack of child ranges (entry =
 // first << 4 | count, count 1..8, top at sp - 1): takes whole ranges from the top while they fit
 // in 32 * NPL node slots and the head of the next one (the rest of that range stays on the
 // stack). Slot s = lane + 32 i gets node[i] (-1 when empty); returns the number of nodes taken.
-// The node of a slot is found by a binary search over the ranges' inclusive sums (shuffles
-// only, no shared-memory staging), so the slots past the first 32 cost nothing in rounds that
-// fill fewer. The caller synchronises the warp before the stack is read again.
+// The range of a slot is found from the ranges' start marks (segment_marks). The caller
+// synchronises the warp before the stack is read again.
 template <int NPL>
 __device__ __forceinline__ int pop_round(int* stack, int& sp, int (&node)[NPL]) {
     constexpr int kRound = 32 * NPL;
     const int lane = threadIdx.x & 31;
+    const unsigned lt = lanemask_lt();
     const int kk = min(sp, 32);
     int e = 0, c = 0;
     if (lane < kk) {
@@ -137,22 +147,17 @@ __device__ __forceinline__ int pop_round(int* stack, int& sp, int (&node)[NPL]) 
         }
     }
     sp -= nfull;
-    const int incl2 = min(incl, kRound);
-    const int first = e >> 4;
+    const int off = (e >> 4) - excl;  // node of slot s in this range: off + s
+    int before = -1;
 #pragma unroll
     for (int i = 0; i < NPL; ++i) {
         node[i] = -1;
         if (32 * i < nnodes) {  // warp-uniform
+            const unsigned marks = segment_marks(lane < kk, excl, 32 * i);
             const int slot = lane + 32 * i;
-            int src = 0;  // ranges ending at or before the slot
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const int v = __shfl_sync(0xffffffffu, incl2, src + step - 1);
-                if (v <= slot) src += step;
-            }
-            const int f = __shfl_sync(0xffffffffu, first, src);
-            const int x = __shfl_sync(0xffffffffu, excl, src);
-            if (slot < nnodes) node[i] = f + (slot - x);
+            const int o = __shfl_sync(0xffffffffu, off, before + __popc(marks & (lt | (1u << lane))));
+            if (slot < nnodes) node[i] = o + slot;
+            if (i + 1 < NPL) before += __popc(marks);
         }
     }
     return nnodes;

@@ -260,6 +260,7 @@ struct KnnSmem {
     unsigned long long key[2][kKnnCap];  // the collected points of the warp's two queries
     unsigned long long dd[64];  // float64 squared distances as bit patterns
     int di[64];
+    int seg[64];                // opened leaves of a round: first particle minus first slot
 };
 
 // A query of a neighbour walk: position (hi/lo), radius; `on` (warp-uniform) false for a slot
@@ -379,24 +380,24 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2]
         const int lincl = warp_incl_scan(lc);
         const int lexcl = lincl - lc;
         const int ltot = __shfl_sync(0xffffffffu, lincl, 31);
+        const bool has0 = lcs[0] > 0, has1 = lcs[1] > 0;
+        const int start1 = lexcl + lcs[0];
+        const int rank0 = __popc(__ballot_sync(0xffffffffu, has0) & lt) + __popc(__ballot_sync(0xffffffffu, has1) & lt);
+        if (has0) S.seg[rank0] = first[0] - lexcl;
+        if (has1) S.seg[rank0 + (has0 ? 1 : 0)] = first[1] - start1;
+        __syncwarp();
+        int before = -1;
         for (int base = 0; base < ltot; base += 32) {
             const int o = base + lane;
-            int src = 0;  // lanes whose inclusive end is <= o (branch-free lower bound)
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const int v = __shfl_sync(0xffffffffu, lincl, src + step - 1);
-                if (v <= o) src += step;
-            }
-            src = min(src, 31);
-            const int f0 = __shfl_sync(0xffffffffu, first[0], src);
-            const int f1 = __shfl_sync(0xffffffffu, first[1], src);
-            const int l0 = __shfl_sync(0xffffffffu, lcs[0], src);
-            const int e_src = __shfl_sync(0xffffffffu, lexcl, src);
+            const unsigned r0 = unsigned(lexcl - base), r1 = unsigned(start1 - base);
+            const unsigned marks = __reduce_or_sync(
+                0xffffffffu, (has0 && r0 < 32u ? 1u << r0 : 0u) | (has1 && r1 < 32u ? 1u << r1 : 0u));
+            const int src = before + __popc(marks & (lt | (1u << lane)));
+            before += __popc(marks);
             float4 ph = make_float4(0.f, 0.f, 0.f, 0.f), pl = ph;
             int j = 0;
             if (o < ltot) {
-                const int off = o - e_src;
-                j = off < l0 ? f0 + off : f1 + (off - l0);
+                j = S.seg[src] + o;
                 ph = A.p4[j];
                 pl = A.plo[j];
             }

@@ -350,7 +350,7 @@ struct WarpSmem {
     float4 ntA[kNodeTile];   // centre of mass, mass
     float4 ntQ[kNodeTile];   // Qxx, Qyy, Qxy, Qxz
     float2 ntYZ[kNodeTile];  // Qyz, T
-    int lanemap[QUAD ? 32 * NPL : 1];  // slot -> node of a round (mixed form)
+    int seg[32];  // opened leaves of a slot row: first particle minus first slot
     int slot_pos[kBatch];
 };
 
@@ -614,43 +614,8 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             // pop up to kRound nodes from the top ranges (kNodesPerLane per lane: their loads
             // are issued together, so one round's memory latency covers them all)
             int nodes[kNodesPerLane];
-            int nnodes;
-            if constexpr (!QUAD) {
-                nnodes = pop_round<kNodesPerLane>(S.stack, sp, nodes);
-            } else {  // the slots' nodes staged in shared memory (shorter round latency)
-                const int k = min(sp, 32);
-                int e = 0, c = 0;
-                if (lane < k) {
-                    e = S.stack[sp - 1 - lane];
-                    c = e & 15;
-                }
-                const int incl = warp_incl_scan(c);
-                const int excl = incl - c;
-                const unsigned fullm = __ballot_sync(0xffffffffu, lane < k && incl <= kRound);
-                const int nfull = __popc(fullm);
-                nnodes = __shfl_sync(0xffffffffu, incl, k - 1);
-                int take = c;
-                if (nfull < k) {  // range `nfull` is split: the rest stays on the stack
-                    nnodes = kRound;
-                    if (lane == nfull) {
-                        take = kRound - excl;
-                        S.stack[sp - 1 - lane] = (((e >> 4) + take) << 4) | (c - take);
-                    }
-                }
-                __syncwarp();
-                if (lane < k && lane <= nfull) {
-                    const int first = e >> 4;
-                    for (int t = 0; t < take && excl + t < kRound; ++t) S.lanemap[excl + t] = first + t;
-                }
-                sp -= nfull;
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < kNodesPerLane; ++i) {
-                    const int slot = lane + 32 * i;
-                    nodes[i] = slot < nnodes ? S.lanemap[slot] : -1;
-                }
-                __syncwarp();
-            }
+            const int nnodes = pop_round<kNodesPerLane>(S.stack, sp, nodes);
+            __syncwarp();
             float4 As[kNodesPerLane], Bs[kNodesPerLane];
             float RQs[kNodesPerLane];
 #pragma unroll
@@ -683,30 +648,27 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             // The loads this slot needs are issued here, ahead of the pushes and appends that
             // do not depend on them: an accepted quadrupole node's moments, and the first 32
             // particles of the round's opened leaves (concatenated in lane order; entry o goes
-            // to lane o, which finds its leaf by a binary search over the inclusive sums).
+            // to lane o, which finds its leaf from the leaves' start marks).
             float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
             float2 yv = make_float2(0.f, 0.f);
             if (QUAD && accept && !mono) {
                 qv = wq[node];
                 yv = wt[node];
             }
-            const bool anyleaf = __any_sync(0xffffffffu, leaf);
-            int lincl = 0, lexcl = 0, ltot = 0;
+            const unsigned leafm = __ballot_sync(0xffffffffu, leaf);
+            const bool anyleaf = leafm != 0u;
+            int lexcl = 0, ltot = 0, nseg = -1;
             float4 lp = make_float4(0.f, 0.f, 0.f, 0.f);
             if (anyleaf) {
                 const int lc = leaf ? -code : 0;
-                lincl = warp_incl_scan(lc);
+                const int lincl = warp_incl_scan(lc);
                 lexcl = lincl - lc;
                 ltot = __shfl_sync(0xffffffffu, lincl, 31);
-                int src = 0;
-#pragma unroll
-                for (int step = 16; step; step >>= 1) {
-                    const int v = __shfl_sync(0xffffffffu, lincl, src + step - 1);
-                    if (v <= lane) src += step;
-                }
-                const int f = __shfl_sync(0xffffffffu, first, src);
-                const int x = __shfl_sync(0xffffffffu, lexcl, src);
-                if (lane < ltot) lp = p4[f + (lane - x)];
+                if (leaf) S.seg[__popc(leafm & lt)] = first - lexcl;
+                const unsigned marks = segment_marks(leaf, lexcl, 0);
+                __syncwarp();
+                if (lane < ltot) lp = p4[S.seg[nseg + __popc(marks & (lt | (1u << lane)))] + lane];
+                nseg += __popc(marks);
             }
 
             // opened internal nodes: push their child ranges
@@ -756,20 +718,16 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             for (int done = n0; done < ltot;) {
                 if (fill == Smem::kTile) GF_WALK_FLUSH();
                 const int chunk = min(Smem::kTile - fill, ltot - done);
-                // warp-cooperative copy: entry o of the concatenated leaves goes to lane o % 32,
-                // which finds its leaf by a binary search over the inclusive sums (32 loads in
-                // flight at once instead of each leaf's particles one after another)
+                // warp-cooperative copy: entry o of the concatenated leaves goes to lane o % 32
+                // (32 loads in flight at once instead of each leaf's particles one after another)
                 for (int base = 0; base < chunk; base += 32) {
                     const int o = done + base + lane;
-                    int src = 0;
-#pragma unroll
-                    for (int step = 16; step; step >>= 1) {
-                        const int v = __shfl_sync(0xffffffffu, lincl, src + step - 1);
-                        if (v <= o) src += step;
-                    }
-                    const int f = __shfl_sync(0xffffffffu, first, src);
-                    const int x = __shfl_sync(0xffffffffu, lexcl, src);
-                    if (base + lane < chunk) S.tile[fill + base + lane] = p4[f + (o - x)];
+                    const unsigned marks = segment_marks(leaf, lexcl, done + base);
+                    const int q = nseg + __popc(marks & (lt | (1u << lane)));
+                    if (base + lane < chunk) S.tile[fill + base + lane] = p4[S.seg[q] + o];
+                    // leaves that start in the entries copied (a chunk may end inside the row)
+                    const int row = min(32, chunk - base);
+                    nseg += __popc(row < 32 ? marks & ((1u << row) - 1u) : marks);
                 }
                 fill += chunk;
                 done += chunk;
