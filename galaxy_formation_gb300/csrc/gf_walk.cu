@@ -30,6 +30,15 @@ namespace gf {
 namespace {
 
 constexpr int kWalkWarps = 4;
+// Reference form: two warps share an item of more than 32 particles when there are at most
+// kSplitItems items per warp that runs. With few items a launch lasts as long as its slowest ones
+// (10k particles: 390 items, the slowest 215k cycles, 143k of them evaluating its list for two
+// particles per lane). Thresholds of 2, 4 and 8 measured the same.
+constexpr int kSplitItems = 4;
+// The kernel that can do so also evaluates in batches and takes four blocks per SM, which costs
+// throughput where there are many items: it runs up to this many particles (Engine.gravity at
+// 10k: 386 -> 351 us, sub-steps at 200k 3493 -> 3150 us; at 4M it would take 7230-7350 us, not 7070).
+constexpr int kSplitParticles = 400000;
 constexpr int kStackCap = 1024;   // child ranges per warp
 constexpr int kTileCap = 256;     // interaction entries per warp
 // Nodes tested per lane and round of the walk (their loads are issued together, so one
@@ -359,15 +368,98 @@ __device__ __forceinline__ float soft_r2(float ex, float ey, float ez, float eps
     return fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2)));
 }
 
+// 1 / sqrt(r2). NORMAL: r2 is a normal number (the softening alone makes it one), so the
+// instruction's flush of subnormal inputs cannot matter and its plain form gives the bits of
+// rsqrtf without the three instructions that scale subnormal inputs up (of 17 per pair: gravity
+// of the 4M cloud 7.57 -> 7.12 ms, mixed form of the 1M disk 12.9 -> 12.4 ms per two evaluations).
+template <bool NORMAL>
+__device__ __forceinline__ float inv_sqrt(float r2) {
+    if constexpr (NORMAL) {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+        return y;
+    } else {
+        return rsqrtf(r2);
+    }
+}
+
+template <bool NORMAL>
 __device__ __forceinline__ void pair_acc(const float4 e, float x, float y, float z, float eps2,
                                          float& ax, float& ay, float& az) {
     const float ex = e.x - x, ey = e.y - y, ez = e.z - z;
     const float r2 = soft_r2(ex, ey, ez, eps2);
-    const float inv = rsqrtf(r2);
+    const float inv = inv_sqrt<NORMAL>(r2);
     const float f = e.w * inv * inv * inv;
     ax += f * ex;
     ay += f * ey;
     az += f * ez;
+}
+
+// B entries for one particle, the entries' chains side by side and the sums in entry
+// order: the operations of pair_acc, staged so that their latencies overlap (a lone warp per
+// scheduler: 33 -> 22 cycles per entry). For walks of few items: with five warps per scheduler the
+// evaluation is bound by issue (13 instructions per entry) and the batches' registers spill.
+constexpr int kBatchOne = 4, kBatchTwo = 4;
+
+template <int B, bool NORMAL>
+__device__ __forceinline__ void pair_batch(const float4* tile, float x, float y, float z, float eps2,
+                                           float& ax, float& ay, float& az) {
+    float4 e[B];
+    float f[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) e[u] = tile[u];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        e[u].x -= x;
+        e[u].y -= y;
+        e[u].z -= z;
+        f[u] = soft_r2(e[u].x, e[u].y, e[u].z, eps2);
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) f[u] = inv_sqrt<NORMAL>(f[u]);
+#pragma unroll
+    for (int u = 0; u < B; ++u) f[u] = e[u].w * f[u] * f[u] * f[u];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        ax += f[u] * e[u].x;
+        ay += f[u] * e[u].y;
+        az += f[u] * e[u].z;
+    }
+}
+
+// the same for two particles (62 -> 51 cycles per entry for a lone warp)
+template <int B, bool NORMAL>
+__device__ __forceinline__ void pair_batch_two(const float4* tile, float x0, float y0, float z0, float x1, float y1,
+                                               float z1, float eps2, float& ax0, float& ay0, float& az0, float& ax1,
+                                               float& ay1, float& az1) {
+    float4 e[B];
+    float f[B], g[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) e[u] = tile[u];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        f[u] = soft_r2(e[u].x - x0, e[u].y - y0, e[u].z - z0, eps2);
+        g[u] = soft_r2(e[u].x - x1, e[u].y - y1, e[u].z - z1, eps2);
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        f[u] = inv_sqrt<NORMAL>(f[u]);
+        g[u] = inv_sqrt<NORMAL>(g[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        f[u] = e[u].w * f[u] * f[u] * f[u];
+        g[u] = e[u].w * g[u] * g[u] * g[u];
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        ax0 += f[u] * (e[u].x - x0);
+        ay0 += f[u] * (e[u].y - y0);
+        az0 += f[u] * (e[u].z - z0);
+        ax1 += g[u] * (e[u].x - x1);
+        ay1 += g[u] * (e[u].y - y1);
+        az1 += g[u] * (e[u].z - z1);
+    }
 }
 
 // the same pair with the softened potential -m / sqrt(|d|^2 + eps^2) (energy diagnostics;
@@ -392,11 +484,12 @@ __device__ __forceinline__ void pair_acc_pot(const float4 e, float x, float y, f
 // (unlike 1/r) does not annihilate; it matters for cells accepted within a few eps.
 // c_t = (5/2) T eps^2 is the node's constant of that term (the caller computes it once per node
 // for all the particles it serves).
+template <bool NORMAL>
 __device__ __forceinline__ void quad_acc(const float4 e, const float4 q, float qyz, float c_t, float x, float y,
                                          float z, float eps2, float& ax, float& ay, float& az) {
     const float dx = e.x - x, dy = e.y - y, dz = e.z - z;
     const float r2 = soft_r2(dx, dy, dz, eps2);
-    const float inv = rsqrtf(r2);
+    const float inv = inv_sqrt<NORMAL>(r2);
     const float inv2 = inv * inv;
     const float inv3 = inv2 * inv;
     const float inv5 = inv3 * inv2;
@@ -413,7 +506,7 @@ __device__ __forceinline__ void quad_acc(const float4 e, const float4 q, float q
 }
 
 // Evaluates the tile entries [0, fill) for the lane's particle(s); POT also sums potentials.
-template <bool POT>
+template <bool POT, bool NORMAL, bool BATCH>
 __device__ __forceinline__ void eval_tile(const float4* tile, int fill, bool two, int r, int sub, float eps2,
                                           float x0, float y0, float z0, float x1, float y1, float z1,
                                           float& ax0, float& ay0, float& az0, float& ax1, float& ay1,
@@ -431,25 +524,33 @@ __device__ __forceinline__ void eval_tile(const float4* tile, int fill, bool two
         return;
     }
     if (two) {
+        int j = 0;
+        if constexpr (BATCH)
+            for (; j + kBatchTwo <= fill; j += kBatchTwo)
+                pair_batch_two<kBatchTwo, NORMAL>(tile + j, x0, y0, z0, x1, y1, z1, eps2, ax0, ay0, az0, ax1, ay1, az1);
 #pragma unroll 2
-        for (int j = 0; j < fill; ++j) {
+        for (; j < fill; ++j) {
             const float4 e = tile[j];
-            pair_acc(e, x0, y0, z0, eps2, ax0, ay0, az0);
-            pair_acc(e, x1, y1, z1, eps2, ax1, ay1, az1);
+            pair_acc<NORMAL>(e, x0, y0, z0, eps2, ax0, ay0, az0);
+            pair_acc<NORMAL>(e, x1, y1, z1, eps2, ax1, ay1, az1);
         }
     } else if (r == 1) {
+        int j = 0;
+        if constexpr (BATCH)
+            for (; j + kBatchOne <= fill; j += kBatchOne)
+                pair_batch<kBatchOne, NORMAL>(tile + j, x0, y0, z0, eps2, ax0, ay0, az0);
 #pragma unroll 4
-        for (int j = 0; j < fill; ++j) pair_acc(tile[j], x0, y0, z0, eps2, ax0, ay0, az0);
+        for (; j < fill; ++j) pair_acc<NORMAL>(tile[j], x0, y0, z0, eps2, ax0, ay0, az0);
     } else {
 #pragma unroll 4
-        for (int j = sub; j < fill; j += r) pair_acc(tile[j], x0, y0, z0, eps2, ax0, ay0, az0);
+        for (int j = sub; j < fill; j += r) pair_acc<NORMAL>(tile[j], x0, y0, z0, eps2, ax0, ay0, az0);
     }
 }
 
 // Mixed form: entries ksub, ksub + m, ... of both tiles for the lane's PPL (4) particles (each
 // entry loaded once from shared memory serves the PPL); the tile's partial sums go to Kahan
 // totals.
-template <int PPL>
+template <int PPL, bool NORMAL>
 __device__ __forceinline__ void eval_quad(const float4* tile, const float4* ntA, const float4* ntQ,
                                           const float2* ntYZ, int fill, int fillN, int ksub, int m, float eps2,
                                           const float (&x)[4], const float (&y)[4], const float (&z)[4],
@@ -460,14 +561,14 @@ __device__ __forceinline__ void eval_quad(const float4* tile, const float4* ntA,
     for (int j = ksub; j < fill; j += m) {
         const float4 e = tile[j];
 #pragma unroll
-        for (int t = 0; t < PPL; ++t) pair_acc(e, x[t], y[t], z[t], eps2, px[t], py[t], pz[t]);
+        for (int t = 0; t < PPL; ++t) pair_acc<NORMAL>(e, x[t], y[t], z[t], eps2, px[t], py[t], pz[t]);
     }
     for (int j = ksub; j < fillN; j += m) {
         const float4 e = ntA[j], q = ntQ[j];
         const float2 yt = ntYZ[j];
         const float c_t = 2.5f * yt.y * eps2;
 #pragma unroll
-        for (int t = 0; t < PPL; ++t) quad_acc(e, q, yt.x, c_t, x[t], y[t], z[t], eps2, px[t], py[t], pz[t]);
+        for (int t = 0; t < PPL; ++t) quad_acc<NORMAL>(e, q, yt.x, c_t, x[t], y[t], z[t], eps2, px[t], py[t], pz[t]);
     }
 #pragma unroll
     for (int t = 0; t < PPL; ++t) {
@@ -482,17 +583,18 @@ __device__ __forceinline__ void eval_quad(const float4* tile, const float4* ntA,
 // 5 keeps the latter free of register spills; the wide-round variant needs more registers.
 // WARPS (block shape) and SMALL (tile size) are the mixed walk's tunable launch shape: the
 // register bound keeps 16 warps per SM whatever the block shape.
-template <bool QUAD, bool POT = false, int NPL = (QUAD ? 2 : 1), int WARPS = kWalkWarps, bool SMALL = false>
-__global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) : 5) k_walk(
+template <bool QUAD, bool POT = false, int NPL = (QUAD ? 2 : 1), int WARPS = kWalkWarps, bool SMALL = false,
+          bool NORMAL = true, bool SPLIT = false>
+__global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) : (SPLIT ? 4 : 5)) k_walk(
     const float4* __restrict__ wa, const float4* __restrict__ wb, const float4* __restrict__ wq,
     const float2* __restrict__ wt, const float* __restrict__ wrq, const float4* __restrict__ p4,
     const int* __restrict__ perm, const uint8_t* __restrict__ active, const int4* __restrict__ work,
     const float4* __restrict__ sphere, const float2* __restrict__ gam, TreeCounts* cnt, int nn, float eps2,
     double* __restrict__ acc, uint32_t* status, int stride, double* __restrict__ pot = nullptr) {
     static_assert(!(QUAD && POT), "potentials come from the monopole walk");
+    static_assert(!SPLIT || (!QUAD && !POT), "only items of the reference form are shared by two warps");
     using Smem = WarpSmem<QUAD, NPL, SMALL>;
     constexpr int kNodesPerLane = NPL;
-    constexpr int kRound = 32 * kNodesPerLane;
     __shared__ Smem smem_all[WARPS];
     Smem& S = smem_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -502,16 +604,24 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
     // regions of a work list in tree order, each taken in order (1: the list's own order).
     const int nwork = cnt->num_work;
     const int per = (nwork + stride - 1) / stride;
-    const int ntick = per * stride;
+    // SPLIT: two warps share an item of more than 32 particles, 32 each. Both walk it, so the
+    // traversal is done twice, but the evaluation, most of a lone warp's time, is halved; every
+    // particle's sum keeps its order. (QUAD: lanes hold four particles and share the entries,
+    // which such a split would change.)
+    const int halves = SPLIT && nwork <= kSplitItems * int(gridDim.x) * WARPS ? 2 : 1;
+    const int ntick = per * stride * halves;
 
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(&cnt->walk_next, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= ntick) break;
+        const int half = SPLIT && halves > 1 ? t & 1 : 0;
+        if (SPLIT && halves > 1) t >>= 1;
         const int g = (t % stride) * per + t / stride;
         if (g >= nwork) continue;
         const int4 w = work[g];
+        if (SPLIT && half && w.z <= 32) continue;
         const float4 sph = sphere[g];
         // relative criterion: accept a node when its distance from the sphere exceeds both
         // open_r (geometric) and rho * gm (rho = B.w: 0 outside quadrupole trees); take an
@@ -523,6 +633,8 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
         // are evaluated in batches, each batch walking the tree again.
         for (int pb = 0; pb < Pall; pb += Smem::kBatch) {
         const int P = min(Smem::kBatch, Pall - pb);
+        const bool split = SPLIT && halves > 1 && P > 32;  // this warp: slots 32 half .. 32 half + 31
+        if (SPLIT && half && !split) continue;
 
         // compact the active particles of this batch into slots
         int nslot = 0;
@@ -559,7 +671,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             for (int t = 0; t < kPpl; ++t) slot[t] = t < ppl ? ppl * q + t : P;  // P: no particle
         } else {
             if (P <= 16) r = P <= 1 ? 32 : P <= 2 ? 16 : P <= 4 ? 8 : P <= 8 ? 4 : 2;
-            slot[0] = lane / r;
+            slot[0] = lane / r + 32 * half;
             slot[1] = slot[0] + 32;
             sub = lane % r;
         }
@@ -567,7 +679,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
         bool has[kPpl];
 #pragma unroll
         for (int t = 0; t < kPpl; ++t) {
-            has[t] = lane_on && slot[t] < P && (QUAD || t == 0 || P > 32);
+            has[t] = lane_on && slot[t] < P && (QUAD || t == 0 || (P > 32 && !split));
             x[t] = y[t] = z[t] = 0.f;
             if (has[t]) {
                 const float4 p = p4[S.slot_pos[slot[t]]];
@@ -580,7 +692,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
         KahanF kx[kPpl], ky[kPpl], kz[kPpl];
 #pragma unroll
         for (int t = 0; t < kPpl; ++t) ax[t] = ay[t] = az[t] = ph[t] = 0.f;
-        const bool two = P > 32;
+        const bool two = P > 32 && !split;
 
         int fill = 0, fillN = 0;
         unsigned long long listlen = 0, nodelen = 0;
@@ -590,10 +702,10 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
         nodelen += fillN;                                                                            \
         __syncwarp();                                                                                \
         if constexpr (QUAD) {                                                                        \
-            if (lane_on) eval_quad<4>(S.tile, S.ntA, S.ntQ, S.ntYZ, fill, fillN, ksub, m, eps2, x, y, z, \
+            if (lane_on) eval_quad<4, NORMAL>(S.tile, S.ntA, S.ntQ, S.ntYZ, fill, fillN, ksub, m, eps2, x, y, z, \
                                       kx, ky, kz);                                                   \
         } else {                                                                                     \
-            eval_tile<POT>(S.tile, fill, two, r, sub, eps2, x[0], y[0], z[0], x[1], y[1], z[1],      \
+            eval_tile<POT, NORMAL, SPLIT>(S.tile, fill, two, r, sub, eps2, x[0], y[0], z[0], x[1], y[1], z[1],      \
                            ax[0], ay[0], az[0], ax[1], ay[1], az[1], ph[0], ph[1]);                  \
         }                                                                                            \
         __syncwarp();                                                                                \
@@ -744,7 +856,8 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
         GF_WALK_FLUSH();
 #undef GF_WALK_FLUSH
         if (lane == 0) {
-            atomicAdd(&cnt->pairs, listlen * (unsigned long long)P);
+            const int mine = split ? (half ? P - 32 : 32) : P;
+            atomicAdd(&cnt->pairs, listlen * (unsigned long long)mine);
             if (QUAD) atomicAdd(&cnt->qpairs, nodelen * (unsigned long long)P);
         }
         if constexpr (QUAD) {
@@ -867,57 +980,67 @@ namespace {
 // Every shape keeps its static shared memory under 48 KB per block (8 warps of the large tiles
 // would not).
 
-template <int WARPS, bool SMALL>
+// NORMAL: the softening alone makes every softened distance a normal float32 (any eps above 1e-15).
+template <int WARPS, bool SMALL, bool NORMAL, int NPL = 2>
 void launch_quad_walk(const Octree& T, const uint8_t* active, float eps2, double* acc, cudaStream_t s) {
     static int bps = 0;
     if (!bps) {
-        GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_walk<true, false, 2, WARPS, SMALL>, WARPS * 32,
-                                                              0));
+        GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &bps, k_walk<true, false, NPL, WARPS, SMALL, NORMAL>, WARPS * 32, 0));
         bps = std::max(1, bps);
     }
-    k_walk<true, false, 2, WARPS, SMALL><<<bps * ctx().sms, WARPS * 32, 0, s>>>(
+    k_walk<true, false, NPL, WARPS, SMALL, NORMAL><<<bps * ctx().sms, WARPS * 32, 0, s>>>(
         T.w_a.as<float4>(), T.w_b.as<float4>(), T.w_q.as<float4>(), T.w_t.as<float2>(), T.w_rq.as<float>(),
         T.p4.as<float4>(), T.perm.as<int>(), active, T.work.as<int4>(), T.sphere.as<float4>(),
         T.item_gam.as<float2>(), T.counts.as<TreeCounts>(), T.node_cap, eps2, acc, ctx().d_status, T.walk_stride);
 }
 
+template <bool POT, bool NORMAL, bool SPLIT>
+void launch_mono_walk(const Octree& T, const uint8_t* active, float eps2, double* acc, cudaStream_t s, double* pot) {
+    static int bps = 0;
+    if (!bps) {
+        GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &bps, k_walk<false, POT, 1, kWalkWarps, false, NORMAL, SPLIT>, kWalkWarps * 32, 0));
+        bps = std::max(1, bps);
+    }
+    k_walk<false, POT, 1, kWalkWarps, false, NORMAL, SPLIT><<<bps * ctx().sms, kWalkWarps * 32, 0, s>>>(
+        T.w_a.as<float4>(), T.w_b.as<float4>(), nullptr, nullptr, nullptr, T.p4.as<float4>(), T.perm.as<int>(), active,
+        T.work.as<int4>(), T.sphere.as<float4>(), nullptr, T.counts.as<TreeCounts>(), T.node_cap, eps2, acc,
+        ctx().d_status, T.walk_stride, pot);
+}
+
+template <bool NORMAL>
+void launch_walk(const Octree& T, const uint8_t* active, float eps2, double* acc, cudaStream_t s, int npl, int shape) {
+    if (!T.quad) {
+        if (T.n <= kSplitParticles)
+            launch_mono_walk<false, NORMAL, true>(T, active, eps2, acc, s, nullptr);
+        else
+            launch_mono_walk<false, NORMAL, false>(T, active, eps2, acc, s, nullptr);
+    } else if (npl > 2) {
+        launch_quad_walk<kWalkWarps, false, NORMAL, 8>(T, active, eps2, acc, s);
+    } else {
+        switch (shape) {
+            case 1: launch_quad_walk<2, false, NORMAL>(T, active, eps2, acc, s); break;
+            case 2: launch_quad_walk<4, true, NORMAL>(T, active, eps2, acc, s); break;
+            case 3: launch_quad_walk<2, true, NORMAL>(T, active, eps2, acc, s); break;
+            default: launch_quad_walk<4, false, NORMAL>(T, active, eps2, acc, s); break;
+        }
+    }
+}
+
 }  // namespace
 
 void Octree::walk(double eps, double* acc, cudaStream_t s, double* pot, int npl, int shape) {
-    Context& C = ctx();
     const float eps2 = float(eps * eps);
-    static int bps_mono = 0, bps_quad = 0;
-    if (!bps_mono) {
-        GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_mono, k_walk<false>, kWalkWarps * 32, 0));
-        GF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps_quad, k_walk<true>, kWalkWarps * 32, 0));
-        bps_mono = std::max(1, bps_mono);
-        bps_quad = std::max(1, bps_quad);
-    }
     ProfScope ps(kStWalk, s);
     last_walked() = this;
     if (pot) {
         if (quad) throw Error(GF_ERR_ARG, "potentials come from the monopole walk");
-        k_walk<false, true><<<bps_mono * C.sms, kWalkWarps * 32, 0, s>>>(
-            w_a.as<float4>(), w_b.as<float4>(), nullptr, nullptr, nullptr, p4.as<float4>(), perm.as<int>(), active_ptr,
-            work.as<int4>(), sphere.as<float4>(), nullptr, counts.as<TreeCounts>(), node_cap, eps2, acc, C.d_status,
-            walk_stride, pot);
-    } else if (quad && npl > 2) {
-        k_walk<true, false, 8><<<bps_quad * C.sms, kWalkWarps * 32, 0, s>>>(
-            w_a.as<float4>(), w_b.as<float4>(), w_q.as<float4>(), w_t.as<float2>(), w_rq.as<float>(), p4.as<float4>(),
-            perm.as<int>(), active_ptr, work.as<int4>(), sphere.as<float4>(), item_gam.as<float2>(),
-            counts.as<TreeCounts>(), node_cap, eps2, acc, C.d_status, walk_stride);
-    } else if (quad) {
-        switch (shape) {
-            case 1: launch_quad_walk<2, false>(*this, active_ptr, eps2, acc, s); break;
-            case 2: launch_quad_walk<4, true>(*this, active_ptr, eps2, acc, s); break;
-            case 3: launch_quad_walk<2, true>(*this, active_ptr, eps2, acc, s); break;
-            default: launch_quad_walk<4, false>(*this, active_ptr, eps2, acc, s); break;
-        }
+        launch_mono_walk<true, false, false>(*this, active_ptr, eps2, acc, s, pot);
+    } else if (eps2 >= 1e-30f) {
+        launch_walk<true>(*this, active_ptr, eps2, acc, s, npl, shape);
     } else {
-        k_walk<false><<<bps_mono * C.sms, kWalkWarps * 32, 0, s>>>(
-            w_a.as<float4>(), w_b.as<float4>(), nullptr, nullptr, nullptr, p4.as<float4>(), perm.as<int>(), active_ptr,
-            work.as<int4>(), sphere.as<float4>(), nullptr, counts.as<TreeCounts>(), node_cap, eps2, acc, C.d_status,
-            walk_stride);
+        launch_walk<false>(*this, active_ptr, eps2, acc, s, npl, shape);
     }
     GF_CHECK_LAUNCH();
 }
