@@ -380,7 +380,7 @@ int gf_sph_forces(int n, int k, const double* pos, const double* vel, const doub
         double* d_acc = g_st.acc.get<double>(3 * size_t(n));
         double* d_dudt = g_st.dudt.get<double>(n);
         double* d_dt = g_st.dt.get<double>(n);
-        sph_forces<int64_t>(g_sph, n, k, k, d_pos, d_vel, d_mass, d_nb, d_h, d_u, gamma, alpha, beta,
+        sph_forces<int64_t>(g_sph, n, k, k, nullptr, d_pos, d_vel, d_mass, d_nb, d_h, d_u, gamma, alpha, beta,
                             d_rho, d_acc, d_dudt, d_dt, s);
         download(rho, d_rho, size_t(n), s);
         download(acc, d_acc, 3 * size_t(n), s);
@@ -426,7 +426,7 @@ int gf_sph_forces_dev(int n, int k, const double* pos, const double* vel, const 
         require(n >= 0 && k >= 0, "negative size");
         if (n == 0) return;
         require(pos && vel && mass && nb && h && u && rho && acc && dudt && dt_i, "null array");
-        sph_forces<int64_t>(g_sph, n, k, k, pos, vel, mass, nb, h, u, gamma, alpha, beta, rho, acc, dudt,
+        sph_forces<int64_t>(g_sph, n, k, k, nullptr, pos, vel, mass, nb, h, u, gamma, alpha, beta, rho, acc, dudt,
                             dt_i, pick(stream));
     });
 }

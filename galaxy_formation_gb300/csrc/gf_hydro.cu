@@ -697,13 +697,13 @@ void ForceEngine::hydro(const ForceArgs& a, cudaStream_t s) {
     double* du = dudt.get<double>(ng);
     double* dti = dt_i.get<double>(ng);
     float* dv = gdivv.get<float>(ng);
+    // visit the gas in the Morton order of the last neighbour-search tree (same gas set)
+    const int* order = order_ng == ng ? knn_tree.perm.as<int>() : nullptr;
     if (sph_float32) {
-        // visit the gas in the Morton order of the last neighbour-search tree (same gas set)
-        const int* order = order_ng == ng ? knn_tree.perm.as<int>() : nullptr;
         sph_forces32<int>(sph32, ng, kNgb, kCand, order, gp, gv, gm, nb, hh, gu, a.gamma, a.alpha, a.beta, r,
                           gacc_, du, dti, s, dv, sub);
     } else {
-        sph_forces<int>(sph, ng, kNgb, kCand, gp, gv, gm, nb, hh, gu, a.gamma, a.alpha, a.beta, r, gacc_, du, dti,
+        sph_forces<int>(sph, ng, kNgb, kCand, order, gp, gv, gm, nb, hh, gu, a.gamma, a.alpha, a.beta, r, gacc_, du, dti,
                         s, dv, sub);
     }
     k_scatter_f<<<ggrid, kThreads, 0, s>>>(ng, gi, dv, divv_prev.as<float>(), sub);

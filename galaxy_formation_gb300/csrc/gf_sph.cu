@@ -1,10 +1,10 @@
 // gf_sph.cu — SPH on the GPU (galaxy_formation/sph.py).
 //
 //   kernel / kernel_grad ..... sph.py:31-54, float64
-//   sph_forces ............... sph.py:57-106: density pass, then an equation-of-state pass
-//                              (P/rho^2 and sound speed per particle), then the force pass
-//                              (pressure, Monaghan-Gingold viscosity on approaching pairs,
-//                              du/dt, Courant step); one thread per particle, float64.
+//   sph_forces ............... sph.py:57-106: density pass with the equation of state of each
+//                              particle (P/rho^2, sound speed), then the force pass (pressure,
+//                              Monaghan-Gingold viscosity on approaching pairs, du/dt, Courant
+//                              step); a few lanes per particle, float64.
 //   knn_from_candidates ...... sph.py:109-135: one warp per particle, float64 distances,
 //                              bitonic sort of the (<= 64) candidates in shared memory.
 //   exact k nearest .......... replaces cKDTree(p).query(p, k) (sph.py:165-166):
@@ -25,6 +25,7 @@
 #include <cstdio>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "gf_mlp.cuh"
 #include "gf_sph.cuh"
@@ -73,122 +74,264 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
     if (dw) dw[i] = dw_m4(r[i], h[i]);
 }
 
+// ---- sph_forces in float64 ---------------------------------------------------------------
+//
+// Bound by the float64 pipe (2 lanes per SM and clock on this GPU), so the pair terms are written
+// for few float64 instructions: about 18 in the density pass and 56 in the force pass, against
+// 30 and 100 with a division and a square root per factor.
+//   * 1/r by a seed and one step of third order, r = r^2 (1/r); 1/x the same way (inv_root,
+//     inverse): the error of the seed cubed is below rounding.
+//   * the kernel's two branches are one polynomial whose coefficients are picked by integer
+//     compares on q's upper word.
+//   * per-particle factors (1/h, the kernel's normalisation, P/rho^2, scaled sound speed) are
+//     computed once per particle, and the two quotients of the viscosity share one inverse.
+// kLanes lanes share a particle's row: without them a lone warp works through 32 neighbours one
+// after another, and small sets leave most of the chip idle.
+
+// Neighbour data of a pair term. PackedSrc: one 128-byte record per particle, a line per
+// neighbour: {x, y, z, m}, {vx, vy, vz, h/2}, {-3/(4 pi h^4), 1/h, P/rho^2, alpha c/2}, {rho, c}.
+struct PairEos {
+    double s4n, inv_h, pr2, ca;
+};
+struct alignas(128) SphRec {
+    double4_32a xm, vh, eos, rc;
+};
+struct PackedSrc {
+    const SphRec* rec;
+    __device__ __forceinline__ double4_32a xm(int64_t j) const { return rec[j].xm; }
+    __device__ __forceinline__ double4_32a vh(int64_t j) const { return rec[j].vh; }
+    __device__ __forceinline__ PairEos eos(int64_t j) const {
+        const double4_32a e = rec[j].eos;
+        return PairEos{e.x, e.y, e.z, e.w};
+    }
+    __device__ __forceinline__ double rho(int64_t j) const { return rec[j].rc.x; }
+    __device__ __forceinline__ double sound(int64_t j) const { return rec[j].rc.y; }
+};
+// PlainSrc: the caller's arrays and two scratch arrays (the entry point that may not allocate);
+// a neighbour's 1/h is then formed per pair.
+struct PlainSrc {
+    const double* pos;
+    const double* vel;
+    const double* mass;
+    const double* h;
+    const double* rho_;
+    const double* pr2;
+    const double* cs;
+    double ha;  // alpha / 2
+    __device__ __forceinline__ double4_32a xm(int64_t j) const {
+        return double4_32a{pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], mass[j]};
+    }
+    __device__ __forceinline__ double4_32a vh(int64_t j) const {
+        return double4_32a{vel[3 * j], vel[3 * j + 1], vel[3 * j + 2], 0.5 * h[j]};
+    }
+    __device__ __forceinline__ PairEos eos(int64_t j) const {
+        const double ih = 1.0 / h[j], ih2 = ih * ih;
+        return PairEos{ih2 * ih2 * (-0.75 / kPi), ih, pr2[j], ha * cs[j]};
+    }
+    __device__ __forceinline__ double rho(int64_t j) const { return rho_[j]; }
+    __device__ __forceinline__ double sound(int64_t j) const { return cs[j]; }
+};
+
+__device__ __forceinline__ unsigned exponent_of(double x) { return unsigned(__double2hiint(x)) >> 20; }
+
+// r and 1/r of r2 >= 0 (1/r capped at 1e30, as sph.py:53's max(r, 1e-30)). y, the hardware's
+// approximation, has e = 1 - r2 y^2 of about 2^-20; y (1 - e)^(-1/2) = y (1 + e/2 + 3/8 e^2 + ...).
+__device__ __forceinline__ void inv_root(double r2, double& r, double& inv_r) {
+    if (exponent_of(r2) - 825u < 1160u) {  // 2^-198 <= r2 < 2^962
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+        const double e = fma(-(r2 * y), y, 1.0);
+        inv_r = fma(y * e, fma(0.375, e, 0.5), y);
+        r = r2 * inv_r;
+    } else {
+        r = sqrt(r2);
+        inv_r = 1.0 / fmax(r, 1e-30);
+    }
+}
+
+// 1/x of a normal x far from the ends of the range: seed y with e = 1 - x y, y (1 + e + e^2 + ...).
+__device__ __forceinline__ double inverse(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// q < 1 and q < 2 on the upper word of a float64 (NaN and negative values are neither)
+__device__ __forceinline__ bool below_1(double q) { return unsigned(__double2hiint(q)) < 0x3ff00000u; }
+__device__ __forceinline__ bool below_2(double q) { return unsigned(__double2hiint(q)) < 0x40000000u; }
+
+// M4 kernel without its 1/(pi h^3) (sph.py:31-40): 1 - 3/2 q^2 + 3/4 q^3, or (2 - q)^3 / 4
+__device__ __forceinline__ double w_shape64(double q) {
+    const bool in = below_1(q);
+    const double x = in ? q : 2.0 - q;
+    const double w = fma(x * x, fma(in ? 0.75 : 0.25, x, in ? -1.5 : 0.0), in ? 1.0 : 0.0);
+    return below_2(q) ? w : 0.0;
+}
+
+// -4/3 dW/dq without its 1/(pi h^4) (sph.py:43-54): q (4 - 3 q), or (2 - q)^2
+__device__ __forceinline__ double dw_shape64(double q) {
+    const bool in = below_1(q);
+    const double l = fma(in ? -3.0 : -1.0, q, in ? 4.0 : 2.0);
+    return (in ? q : below_2(q) ? l : 0.0) * l;
+}
+
+template <int kLanes>
+__device__ __forceinline__ double lanes_sum(double v) {
+#pragma unroll
+    for (int o = kLanes / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ double nan64() { return __longlong_as_double(0x7ff8000000000000ll); }
+
+__global__ void k_sph_pack(int n, const double* __restrict__ pos, const double* __restrict__ vel,
+                           const double* __restrict__ mass, const double* __restrict__ h, SphRec* __restrict__ rec) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    rec[i].xm = double4_32a{pos[3 * size_t(i)], pos[3 * size_t(i) + 1], pos[3 * size_t(i) + 2], mass[i]};
+    rec[i].vh = double4_32a{vel[3 * size_t(i)], vel[3 * size_t(i) + 1], vel[3 * size_t(i) + 2], 0.5 * h[i]};
+}
+
 // A neighbour row from the caller may hold an index outside [0, n): such a particle gets NaN
 // outputs and GF_ERR_ARG is raised (status may be null), instead of a read out of bounds.
-template <class Idx>
-__device__ __forceinline__ bool row_in_range(const Idx* __restrict__ row, int k, int n, uint32_t* status) {
+
+// pass 1 (sph.py:63-71): rho_i = sum_j m_j W(r_ij, h_i), the particle itself included; then the
+// equation of state of the particle (the per-j factors of sph.py:88-89), into its record
+// (PackedSrc) or pr2 / cs.
+template <class Idx, int kLanes, class Src>
+__global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, Src src, const int* __restrict__ order,
+                                                          const Idx* __restrict__ nb, const double* __restrict__ h,
+                                                          const double* __restrict__ u, double gamma, double ha,
+                                                          double* __restrict__ rho, SphRec* rec, double* pr2,
+                                                          double* cs, Subset sub, uint32_t* status) {
+    const int s = threadIdx.x % kLanes;
+    int i = 0;
+    const bool on = subset_item(sub, (blockIdx.x * kThreads + threadIdx.x) / kLanes, n, order, i);
     bool ok = true;
-    for (int jj = 0; jj < k; ++jj) {
-        const int64_t j = row[jj];
-        ok &= j >= 0 && j < n;
+    double sum = 0.0, hi = 1.0;
+    if (on) {
+        const double4_32a p = src.xm(i);
+        hi = h[i];
+        const double inv_h = 1.0 / hi;
+        const Idx* row = nb + size_t(i) * ld;
+#pragma unroll 4
+        for (int jj = s; jj < k; jj += kLanes) {
+            int64_t j = row[jj];
+            if (j < 0 || j >= n) {
+                ok = false;
+                j = i;
+            }
+            const double4_32a q = src.xm(j);
+            const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            double r = 0.0, inv_r;
+            if (j != i) inv_root(r2, r, inv_r);
+            sum = fma(q.w, w_shape64(r * inv_h), sum);
+        }
     }
+    sum = lanes_sum<kLanes>(sum);
+    if (kLanes > 1) ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
+    if (!on || s != 0) return;
     if (!ok) raise_status(status, GF_ERR_ARG);
-    return ok;
-}
-
-// pass 1 (sph.py:63-71): rho_i = sum_j m_j W(r_ij, h_i), the particle itself included
-template <class Idx>
-__global__ void k_sph_density(int n, int k, int ld, const double* __restrict__ pos, const double* __restrict__ mass,
-                              const Idx* __restrict__ nb, const double* __restrict__ h,
-                              double* __restrict__ rho, Subset sub, uint32_t* status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!subset_item(sub, i, n, nullptr, i)) return;
-    if (!row_in_range(nb + size_t(i) * ld, k, n, status)) {
-        rho[i] = __longlong_as_double(0x7ff8000000000000ll);
-        return;
-    }
-    const double xi = pos[3 * size_t(i)], yi = pos[3 * size_t(i) + 1], zi = pos[3 * size_t(i) + 2];
-    const double hi = h[i];
-    double s = 0.0;
-    for (int jj = 0; jj < k; ++jj) {
-        const int64_t j = nb[size_t(i) * ld + jj];
-        const double dx = xi - pos[3 * j], dy = yi - pos[3 * j + 1], dz = zi - pos[3 * j + 2];
-        s += mass[j] * w_m4(sqrt(dx * dx + dy * dy + dz * dz), hi);
-    }
-    rho[i] = s;
-}
-
-// P / rho^2 and the sound speed of every particle (the per-j factors of sph.py:88-89)
-__global__ void k_sph_eos(int n, const double* __restrict__ rho, const double* __restrict__ u,
-                          double gamma, double* __restrict__ pr2, double* __restrict__ cs, Subset sub) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!subset_item(sub, i, n, nullptr, i)) return;
-    const double P = (gamma - 1) * rho[i] * u[i];
-    pr2[i] = P / (rho[i] * rho[i]);
-    cs[i] = sqrt(gamma * (gamma - 1) * u[i]);
-}
-
-// (1/r) dW/dr of sph.py:43-54 with the per-particle factors 1/h and 1/(pi h^4) precomputed
-// and 1/r shared by both smoothing lengths of a pair (one float64 division per pair).
-__device__ __forceinline__ double dw_m4_pre(double r, double inv_r, double inv_h, double s4) {
-    const double q = r * inv_h;
-    double g;
-    if (q < 1.0) {
-        g = s4 * (-3 * q + 2.25 * q * q);
-    } else if (q < 2.0) {
-        const double t = 2 - q;
-        g = -s4 * 0.75 * t * t;
+    const double d = !ok ? nan64() : sum == 0.0 ? 0.0 : sum * (1.0 / (kPi * hi * hi * hi));
+    const double P = (gamma - 1) * d * u[i];
+    const double pr = P / (d * d), c = sqrt(gamma * (gamma - 1) * u[i]);
+    rho[i] = d;
+    if (rec) {
+        const double ih = 1.0 / hi, ih2 = ih * ih;
+        rec[i].eos = double4_32a{ih2 * ih2 * (-0.75 / kPi), ih, pr, ha * c};
+        rec[i].rc = double4_32a{d, c, 0.0, 0.0};
     } else {
-        return 0.0;
+        pr2[i] = pr;
+        cs[i] = c;
     }
-    return g * inv_r;
 }
 
 // pass 2 (sph.py:72-106)
-template <class Idx>
-__global__ void k_sph_force(int n, int k, int ld, const double* __restrict__ pos, const double* __restrict__ vel,
-                            const double* __restrict__ mass, const Idx* __restrict__ nb,
-                            const double* __restrict__ h, const double* __restrict__ rho,
-                            const double* __restrict__ pr2, const double* __restrict__ cs, double alpha,
-                            double beta, double* __restrict__ acc, double* __restrict__ dudt,
-                            double* __restrict__ dt_i, float* __restrict__ divv, Subset sub, uint32_t* status) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!subset_item(sub, i, n, nullptr, i)) return;
-    if (!row_in_range(nb + size_t(i) * ld, k, n, status)) {
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        acc[3 * size_t(i)] = acc[3 * size_t(i) + 1] = acc[3 * size_t(i) + 2] = nan;
-        dudt[i] = dt_i[i] = nan;
-        if (divv) divv[i] = __int_as_float(0x7fc00000);
-        return;
-    }
-    const double xi = pos[3 * size_t(i)], yi = pos[3 * size_t(i) + 1], zi = pos[3 * size_t(i) + 2];
-    const double vxi = vel[3 * size_t(i)], vyi = vel[3 * size_t(i) + 1], vzi = vel[3 * size_t(i) + 2];
-    const double hi = h[i], rhoi = rho[i], pri = pr2[i], ci = cs[i];
-    const double inv_hi = 1.0 / hi, s4i = 1.0 / (kPi * hi * hi * hi * hi);
-    double ax = 0, ay = 0, az = 0, du = 0, mu_max = 0, dv = 0;
-    for (int jj = 0; jj < k; ++jj) {
-        const int64_t j = nb[size_t(i) * ld + jj];
-        if (j == i) continue;
-        const double dx = xi - pos[3 * j], dy = yi - pos[3 * j + 1], dz = zi - pos[3 * j + 2];
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double hj = h[j];
-        const double inv_r = 1.0 / fmax(r, 1e-30);
-        const double gi = dw_m4_pre(r, inv_r, inv_hi, s4i);
-        const double inv_hj = 1.0 / hj, ih2 = inv_hj * inv_hj;
-        const double gj = dw_m4_pre(r, inv_r, inv_hj, ih2 * ih2 * (1.0 / kPi));
-        const double vr = (vxi - vel[3 * j]) * dx + (vyi - vel[3 * j + 1]) * dy + (vzi - vel[3 * j + 2]) * dz;
-        double visc = 0.0;
-        if (vr < 0) {
-            const double hb = 0.5 * (hi + hj);
-            const double mu = hb * vr / (r * r + 0.01 * hb * hb);
-            mu_max = fmax(mu_max, -mu);
-            visc = (-alpha * 0.5 * (ci + cs[j]) * mu + beta * mu * mu) / (0.5 * (rhoi + rho[j]));
+template <class Idx, int kLanes, class Src>
+__global__ void __launch_bounds__(kThreads) k_sph_force(int n, int k, int ld, Src src, const int* __restrict__ order,
+                                                        const Idx* __restrict__ nb, const double* __restrict__ h,
+                                                        double alpha, double beta, double* __restrict__ acc,
+                                                        double* __restrict__ dudt, double* __restrict__ dt_i,
+                                                        float* __restrict__ divv, Subset sub, uint32_t* status) {
+    const int s = threadIdx.x % kLanes;
+    int i = 0;
+    const bool on = subset_item(sub, (blockIdx.x * kThreads + threadIdx.x) / kLanes, n, order, i);
+    bool ok = true;
+    double ax = 0, ay = 0, az = 0, du = 0, dv = 0, mu_min = 0;
+    if (on) {
+        const double4_32a p = src.xm(i), v = src.vh(i);
+        const PairEos ei = src.eos(i);
+        const double rhoi = src.rho(i);
+        const Idx* row = nb + size_t(i) * ld;
+        for (int jj = s; jj < k; jj += kLanes) {
+            const int64_t j = row[jj];
+            if (j == i) continue;
+            if (j < 0 || j >= n) {
+                ok = false;
+                continue;
+            }
+            const double4_32a q = src.xm(j), w = src.vh(j);
+            const PairEos ej = src.eos(j);
+            const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            double r, inv_r;
+            inv_root(r2, r, inv_r);
+            // r times the (1/r) dW/dr of both smoothing lengths
+            const double gi = ei.s4n * dw_shape64(r * ei.inv_h);
+            const double gj = ej.s4n * dw_shape64(r * ej.inv_h);
+            const double vr = (v.x - w.x) * dx + (v.y - w.y) * dy + (v.z - w.z) * dz;
+            const double pgi = ei.pr2 * gi;
+            double f = fma(ej.pr2, gj, pgi), fu = pgi;
+            if (vr < 0) {
+                // mu = hb vr / (r^2 + 0.01 hb^2), visc = (-alpha c mu + beta mu^2) / rho (mean c and rho)
+                const double hb = v.w + w.w, num = hb * vr;
+                const double den = fma(0.01 * hb, hb, r2), rs = rhoi + src.rho(j);
+                const double prod = den * rs;
+                double mu, half_visc;
+                if (exponent_of(prod) - 123u < 1800u) {
+                    const double inv = inverse(prod);
+                    mu = num * (inv * rs);
+                    half_visc = fma(beta, mu, -(ei.ca + ej.ca)) * mu * (inv * den);
+                } else {
+                    mu = num / den;
+                    half_visc = fma(beta, mu, -(ei.ca + ej.ca)) * mu / rs;
+                }
+                mu_min = fmin(mu_min, mu);
+                const double vg = half_visc * (gi + gj);
+                f += vg;
+                fu = fma(0.5, vg, fu);
+            }
+            const double m = q.w * inv_r, mf = m * f, mv = m * vr;
+            ax = fma(-mf, dx, ax);
+            ay = fma(-mf, dy, ay);
+            az = fma(-mf, dz, az);
+            du = fma(mv, fu, du);
+            dv = fma(mv, gi, dv);
         }
-        const double gb = 0.5 * (gi + gj);
-        const double f = pri * gi + pr2[j] * gj + visc * gb;
-        const double mj = mass[j];
-        ax -= mj * f * dx;
-        ay -= mj * f * dy;
-        az -= mj * f * dz;
-        du += mj * (pri * gi + 0.5 * visc * gb) * vr;
-        dv += mj * vr * gi;
+    }
+    ax = lanes_sum<kLanes>(ax);
+    ay = lanes_sum<kLanes>(ay);
+    az = lanes_sum<kLanes>(az);
+    du = lanes_sum<kLanes>(du);
+    if (divv) dv = lanes_sum<kLanes>(dv);
+#pragma unroll
+    for (int o = kLanes / 2; o; o >>= 1) mu_min = fmin(mu_min, __shfl_xor_sync(0xffffffffu, mu_min, o));
+    if (kLanes > 1) ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
+    if (!on || s != 0) return;
+    if (!ok) {
+        raise_status(status, GF_ERR_ARG);
+        ax = ay = az = du = mu_min = dv = nan64();
     }
     acc[3 * size_t(i)] = ax;
     acc[3 * size_t(i) + 1] = ay;
     acc[3 * size_t(i) + 2] = az;
     dudt[i] = du;
-    dt_i[i] = 0.3 * hi / (ci + 1.2 * (alpha * ci + beta * mu_max) + 1e-30);
-    if (divv) divv[i] = float(-dv / rhoi);  // SPH velocity divergence (a feature of the h guess)
+    const double c = src.sound(i);
+    dt_i[i] = ok ? 0.3 * h[i] / (c + 1.2 * (alpha * c - beta * mu_min) + 1e-30) : nan64();
+    if (divv) divv[i] = ok ? float(-dv / src.rho(i)) : __int_as_float(0x7fc00000);  // SPH velocity divergence
+                                                                                  // (a feature of the h guess)
 }
 
 // ------------------------------------------------------------------- warp bitonic sorts
@@ -719,31 +862,57 @@ void sph_kernel_values(int n, const double* r, const double* h, double* w, doubl
     GF_CHECK_LAUNCH();
 }
 
+// The two float64 passes with L lanes per particle, on any neighbour source.
+template <class Idx, int L, class Src>
+void sph_launch(int n, int k, int ld, const Src& src, const int* order, const Idx* nb, const double* h,
+                const double* u, double gamma, double alpha, double beta, double* rho, SphRec* rec, double* pr2,
+                double* cs, double* acc, double* dudt, double* dt_i, cudaStream_t s, float* divv, Subset sub,
+                uint32_t* status) {
+    const int grid = div_up((long long)n * L, kThreads);
+    {
+        ProfScope ps(kStSphDensity, s);
+        k_sph_density<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 0.5 * alpha, rho, rec,
+                                                        pr2, cs, sub, status);
+        GF_CHECK_LAUNCH();
+    }
+    ProfScope ps(kStSphForce, s);
+    k_sph_force<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, alpha, beta, acc, dudt, dt_i, divv,
+                                                  sub, status);
+    GF_CHECK_LAUNCH();
+}
+
+// Lanes per particle by the particles of a launch: one thread each fills the chip (and needs no
+// reduction) from some hundred thousand on; below, and for the few particles due in a subset of
+// unknown size, four shorten the chain of neighbours. Density + force, measured with 1 / 2 / 4 / 8
+// lanes: 5k gas 204 / 124 / 70 / 74 us (329 us with a division and a square root per factor and a
+// thread per particle); 150k 928 / 892 / 939 / 1032 us (1361); 500k 2365 / 3024 / 2671 / 3010 us
+// (4141).
+constexpr int kSphFourLanes = 128 * 1024, kSphTwoLanes = 256 * 1024;
+
 template <class Idx>
-void sph_forces(SphScratch& S, int n, int k, int ld, const double* pos, const double* vel, const double* mass,
-                const Idx* nb, const double* h, const double* u, double gamma, double alpha,
+void sph_forces(SphScratch& S, int n, int k, int ld, const int* order, const double* pos, const double* vel,
+                const double* mass, const Idx* nb, const double* h, const double* u, double gamma, double alpha,
                 double beta, double* rho, double* acc, double* dudt, double* dt_i, cudaStream_t s, float* divv,
                 Subset sub) {
     if (n <= 0) return;
-    const int grid = div_up(n, kThreads);
-    {
-        ProfScope ps(kStSphDensity, s);
-        k_sph_density<Idx><<<grid, kThreads, 0, s>>>(n, k, ld, pos, mass, nb, h, rho, sub, ctx().d_status);
-        GF_CHECK_LAUNCH();
-    }
-    double* pr2 = S.pr2.get<double>(n);
-    double* cs = S.cs.get<double>(n);
-    k_sph_eos<<<grid, kThreads, 0, s>>>(n, rho, u, gamma, pr2, cs, sub);
+    SphRec* rec = S.rec.get<SphRec>(n);
+    k_sph_pack<<<div_up(n, kThreads), kThreads, 0, s>>>(n, pos, vel, mass, h, rec);
     GF_CHECK_LAUNCH();
-    ProfScope ps(kStSphForce, s);
-    k_sph_force<Idx><<<grid, kThreads, 0, s>>>(n, k, ld, pos, vel, mass, nb, h, rho, pr2, cs, alpha, beta,
-                                               acc, dudt, dt_i, divv, sub, ctx().d_status);
-    GF_CHECK_LAUNCH();
+    auto go = [&](auto lanes) {
+        sph_launch<Idx, decltype(lanes)::value>(n, k, ld, PackedSrc{rec}, order, nb, h, u, gamma, alpha, beta, rho,
+                                                rec, nullptr, nullptr, acc, dudt, dt_i, s, divv, sub, ctx().d_status);
+    };
+    if (sub.idx || n <= kSphFourLanes)
+        go(std::integral_constant<int, 4>());
+    else if (n <= kSphTwoLanes)
+        go(std::integral_constant<int, 2>());
+    else
+        go(std::integral_constant<int, 1>());
 }
-template void sph_forces<int64_t>(SphScratch&, int, int, int, const double*, const double*, const double*,
+template void sph_forces<int64_t>(SphScratch&, int, int, int, const int*, const double*, const double*, const double*,
                                   const int64_t*, const double*, const double*, double, double, double,
                                   double*, double*, double*, double*, cudaStream_t, float*, Subset);
-template void sph_forces<int>(SphScratch&, int, int, int, const double*, const double*, const double*,
+template void sph_forces<int>(SphScratch&, int, int, int, const int*, const double*, const double*, const double*,
                               const int*, const double*, const double*, double, double, double,
                               double*, double*, double*, double*, cudaStream_t, float*, Subset);
 
@@ -941,13 +1110,12 @@ extern "C" int gf_sph_forces_noalloc_dev(int n, int k, const double* pos, const 
     double* pr2 = scratch;
     double* cs = scratch + kNoallocMaxN;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int grid = div_up(n, kThreads);
-    k_sph_density<int64_t><<<grid, kThreads, 0, s>>>(n, k, k, pos, mass, nb, h, rho, Subset(), nullptr);
-    k_sph_eos<<<grid, kThreads, 0, s>>>(n, rho, u, gamma, pr2, cs, Subset());
-    k_sph_force<int64_t><<<grid, kThreads, 0, s>>>(n, k, k, pos, vel, mass, nb, h, rho, pr2, cs, alpha,
-                                                   beta, acc, dudt, dt_i, nullptr, Subset(), nullptr);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return noalloc_fail(GF_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-    c.launches += 3;
+    try {
+        sph_launch<int64_t, 4>(n, k, k, PlainSrc{pos, vel, mass, h, rho, pr2, cs, 0.5 * alpha}, nullptr, nb, h, u,
+                               gamma, alpha, beta, rho, nullptr, pr2, cs, acc, dudt, dt_i, s, nullptr, Subset(),
+                               nullptr);
+    } catch (const Error& err) {
+        return noalloc_fail(err.code, err.what());
+    }
     return GF_OK;
 }

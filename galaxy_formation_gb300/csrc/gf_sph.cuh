@@ -6,15 +6,16 @@
 namespace gf {
 
 struct SphScratch {
-    DevBuf pr2, cs;
+    DevBuf rec;  // SphRec per particle (gf_sph.cu)
 };
 
 void sph_kernel_values(int n, const double* r, const double* h, double* w, double* dw, cudaStream_t s);
 
-// nb: (n, ld) neighbour indices, the first k of each row used.
+// nb: (n, ld) neighbour indices, the first k of each row used. order (optional): the visiting order
+// of the particles, so that neighbouring threads share cache lines.
 template <class Idx>
-void sph_forces(SphScratch& S, int n, int k, int ld, const double* pos, const double* vel, const double* mass,
-                const Idx* nb, const double* h, const double* u, double gamma, double alpha,
+void sph_forces(SphScratch& S, int n, int k, int ld, const int* order, const double* pos, const double* vel,
+                const double* mass, const Idx* nb, const double* h, const double* u, double gamma, double alpha,
                 double beta, double* rho, double* acc, double* dudt, double* dt_i, cudaStream_t s,
                 float* divv = nullptr, Subset sub = Subset());
 
