@@ -247,18 +247,20 @@ int gf_tree_export(int32_t* ints, float* floats, int32_t* order, int32_t* groups
         GF_CUDA(cudaMemcpy(&h, T.counts.as<TreeCounts>(), sizeof h, cudaMemcpyDeviceToHost));
         const int nn = h.total_nodes, n = T.n;
         std::vector<int4> i4(nn);
-        std::vector<float4> mom(nn), geo(nn);
-        std::vector<float> open(nn);
+        std::vector<float4> wa(nn), wb(nn), geo(nn);
+        std::vector<int> bfs(nn);
         GF_CUDA(cudaMemcpy(i4.data(), T.n_i4.p, sizeof(int4) * nn, cudaMemcpyDeviceToHost));
-        GF_CUDA(cudaMemcpy(mom.data(), T.n_mom.p, sizeof(float4) * nn, cudaMemcpyDeviceToHost));
+        GF_CUDA(cudaMemcpy(wa.data(), T.w_a.p, sizeof(float4) * nn, cudaMemcpyDeviceToHost));
+        GF_CUDA(cudaMemcpy(wb.data(), T.w_b.p, sizeof(float4) * nn, cudaMemcpyDeviceToHost));
         GF_CUDA(cudaMemcpy(geo.data(), T.n_geo.p, sizeof(float4) * nn, cudaMemcpyDeviceToHost));
-        GF_CUDA(cudaMemcpy(open.data(), T.n_open.p, sizeof(float) * nn, cudaMemcpyDeviceToHost));
+        GF_CUDA(cudaMemcpy(bfs.data(), T.n_bfs.p, sizeof(int) * nn, cudaMemcpyDeviceToHost));
         for (int k = 0; k < nn; ++k) {
             ints[4 * k] = i4[k].x;
             ints[4 * k + 1] = i4[k].y;
             ints[4 * k + 2] = i4[k].z;
             ints[4 * k + 3] = i4[k].w & 1;
-            const float f[9] = {mom[k].x, mom[k].y, mom[k].z, mom[k].w, open[k],
+            const float4 mom = wa[bfs[k]];
+            const float f[9] = {mom.x, mom.y, mom.z, mom.w, wb[bfs[k]].x,
                                 geo[k].x, geo[k].y, geo[k].z, geo[k].w};
             std::memcpy(floats + 9 * size_t(k), f, sizeof f);
         }

@@ -55,7 +55,7 @@ __device__ __forceinline__ bool finite_bits(double v) {
 // reduces the partials and writes the root cube. min / max are exact, so the result does not
 // depend on the order of the reductions.
 __global__ void k_bbox(const double* __restrict__ pos, int n, double* __restrict__ part, RootBox* __restrict__ root,
-                       uint32_t* status, int* __restrict__ done) {
+                       double theta, uint32_t* status, int* __restrict__ done) {
     long long lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
     int bad = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -141,6 +141,7 @@ __global__ void k_bbox(const double* __restrict__ pos, int n, double* __restrict
     }
     // 0.5 * max extent * 1.0001 + 1e-12 (cpp/nbody.cpp:219), unfused
     R.half = __dadd_rn(__dmul_rn(__dmul_rn(0.5, ext), 1.0001), 1e-12);
+    R.open0 = __ddiv_rn(__dmul_rn(2.0, R.half), theta);
     double cmax = 0;
     for (int a = 0; a < 3; ++a) {
         R.lo[a] = __dsub_rn(R.c[a], R.half);
@@ -400,16 +401,15 @@ __device__ __forceinline__ int live_nodes(int span, const int* nn_dev) {
     return nn_dev ? min(span, *nn_dev) : span;
 }
 
-// Child count of every node and its children's ids in octant order (kids[8k .. 8k + nchild)),
-// so that the bottom-up passes load a node's children together.
+// Child count of every node; arrival counters to zero.
 __global__ void k_nchild(int span, const int* __restrict__ nn_dev, const int4* __restrict__ n_i4,
-                         int* __restrict__ nchild, int* __restrict__ counter, int* __restrict__ kids) {
+                         int* __restrict__ nchild, int* __restrict__ counter) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= live_nodes(span, nn_dev)) return;
     const int4 q = n_i4[k];
     int c = 0;
     if (!(q.w & 1)) {
-        for (int ch = k + 1; ch < q.z && c < 8; ch = n_i4[ch].z) kids[8 * size_t(k) + c++] = ch;  // <= 8 children
+        for (int ch = k + 1; ch < q.z && c < 8; ch = n_i4[ch].z) ++c;  // <= 8 children
     }
     nchild[k] = c;
     counter[k] = 0;
@@ -469,149 +469,6 @@ __global__ void k_gather(int n, const int* __restrict__ perm, const double* __re
 }
 
 // ---------------------------------------------------------------------------- moments
-
-struct MomentArgs {
-    int nn;
-    const int* nn_dev;  // when set: node count read on the device
-    bool refit;
-    float theta;
-    const int4* n_i4;
-    const int* parent;
-    const int* nchild;
-    const int* kids;    // children in octant order, 8 slots per node
-    int* counter;
-    const double4* n_cd;  // build: float64 centre + half
-    const float4* n_geo;  // refit: float32 centre + half
-    float4* mom;
-    float* open_r;
-    float* ndisp;
-    // leaf inputs
-    const int* perm;
-    const double* pos;
-    const double* mass;
-    const float4* p4;
-    const float* pdisp;
-};
-
-__device__ __forceinline__ void finalize(const MomentArgs& A, int k, double M, double sx, double sy,
-                                         double sz, float dm) {
-    const double inv = M > 0 ? __ddiv_rn(1.0, M) : 0.0;
-    const double mx = __dmul_rn(sx, inv), my = __dmul_rn(sy, inv), mz = __dmul_rn(sz, inv);
-    A.mom[k] = make_float4(float(mx), float(my), float(mz), float(M));
-    double ox, oy, oz, first;
-    if (!A.refit) {  // cpp/nbody.cpp:104-106
-        const double4 c = A.n_cd[k];
-        ox = __dsub_rn(mx, c.x);
-        oy = __dsub_rn(my, c.y);
-        oz = __dsub_rn(mz, c.z);
-        first = __ddiv_rn(__dmul_rn(2.0, c.w), double(A.theta));
-    } else {  // cpp/nbody.cpp:301-303: the first term is evaluated in float32
-        const float4 g = A.n_geo[k];
-        ox = __dsub_rn(mx, double(g.x));
-        oy = __dsub_rn(my, double(g.y));
-        oz = __dsub_rn(mz, double(g.z));
-        first = double(__fdiv_rn(__fmul_rn(2.0f, __fadd_rn(g.w, dm)), A.theta));
-        A.ndisp[k] = dm;
-    }
-    const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz)));
-    A.open_r[k] = float(__dadd_rn(first, r));
-}
-
-__global__ void k_moments(MomentArgs A) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= live_nodes(A.nn, A.nn_dev)) return;
-    const int4 q = A.n_i4[k];
-    if (!(q.w & 1)) return;
-    double M = 0, sx = 0, sy = 0, sz = 0;
-    float dm = 0.f;
-    if (q.y <= kLeafMax) {  // the leaf's particles loaded together, summed in order
-        double4 pm[kLeafMax];
-        float pd[kLeafMax];
-#pragma unroll
-        for (int t = 0; t < kLeafMax; ++t) {
-            pm[t] = make_double4(0.0, 0.0, 0.0, 0.0);
-            pd[t] = 0.f;
-            if (t < q.y) {
-                const int i = q.x + t;
-                if (!A.refit) {
-                    const int j = A.perm[i];
-                    pm[t] = make_double4(A.pos[3 * size_t(j)], A.pos[3 * size_t(j) + 1], A.pos[3 * size_t(j) + 2],
-                                         A.mass ? A.mass[j] : 1.0);
-                } else {
-                    const float4 p = A.p4[i];
-                    pm[t] = make_double4(double(p.x), double(p.y), double(p.z), double(p.w));
-                    pd[t] = A.pdisp[i];
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < kLeafMax; ++t) {
-            if (t < q.y) {  // cpp/nbody.cpp:124-131 (build), :285-289 (refit: float x float exact)
-                const double m = pm[t].w;
-                M = __dadd_rn(M, m);
-                sx = __dadd_rn(sx, __dmul_rn(m, pm[t].x));
-                sy = __dadd_rn(sy, __dmul_rn(m, pm[t].y));
-                sz = __dadd_rn(sz, __dmul_rn(m, pm[t].z));
-                dm = fmaxf(dm, pd[t]);
-            }
-        }
-    } else
-    for (int i = q.x; i < q.x + q.y; ++i) {
-        if (!A.refit) {  // cpp/nbody.cpp:124-131
-            const int j = A.perm[i];
-            const double m = A.mass ? A.mass[j] : 1.0;
-            M = __dadd_rn(M, m);
-            sx = __dadd_rn(sx, __dmul_rn(m, A.pos[3 * size_t(j)]));
-            sy = __dadd_rn(sy, __dmul_rn(m, A.pos[3 * size_t(j) + 1]));
-            sz = __dadd_rn(sz, __dmul_rn(m, A.pos[3 * size_t(j) + 2]));
-        } else {  // cpp/nbody.cpp:285-289 (float x float products are exact in float64)
-            const float4 p = A.p4[i];
-            const double m = double(p.w);
-            M = __dadd_rn(M, m);
-            sx = __dadd_rn(sx, m * double(p.x));
-            sy = __dadd_rn(sy, m * double(p.y));
-            sz = __dadd_rn(sz, m * double(p.z));
-            dm = fmaxf(dm, A.pdisp[i]);
-        }
-    }
-    finalize(A, k, M, sx, sy, sz, dm);
-    __threadfence();
-    int p = A.parent[k];
-    while (p >= 0) {
-        const int arrived = atomicAdd(&A.counter[p], 1);
-        if (arrived != A.nchild[p] - 1) return;
-        __threadfence();
-        double PM = 0, px = 0, py = 0, pz = 0;
-        float pd = 0.f;
-        const int nc = A.nchild[p];
-        float4 cms[8];
-        float cds[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {  // the children's records in flight together
-            cms[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-            cds[c] = 0.f;
-            if (c < nc) {
-                const int ch = A.kids[8 * size_t(p) + c];
-                cms[c] = __ldcg(&A.mom[ch]);
-                if (A.refit) cds[c] = __ldcg(&A.ndisp[ch]);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {  // octant order
-            if (c < nc) {
-                const double m = double(cms[c].w);
-                PM = __dadd_rn(PM, m);
-                px = __dadd_rn(px, m * double(cms[c].x));
-                py = __dadd_rn(py, m * double(cms[c].y));
-                pz = __dadd_rn(pz, m * double(cms[c].z));
-                pd = fmaxf(pd, cds[c]);
-            }
-        }
-        finalize(A, p, PM, px, py, pz, pd);
-        __threadfence();
-        p = A.parent[p];
-    }
-}
 
 // Relative opening radius of a quadrupole node: the walk accepts the node for a group sphere
 // (centre c, radius R) when |com - c| - R exceeds rho * (alpha * min |a_old|)^(-1/5), i.e. when
@@ -707,12 +564,71 @@ __device__ __forceinline__ float group8_max(float v) {
     return v;
 }
 
-// The arrival of a finished node at its parent p (child range c0, nc: structure fields, loaded
+__device__ __forceinline__ double group8_sum(double v) {
+#pragma unroll
+    for (int off = 4; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+// The arrival of a finished node at its parent (arrival counter, parent's child count nc, loaded
 // before the atomic). The counter is an acquire-release atomic: it publishes this thread's
 // records of the node and, for the last child, makes its siblings' records visible. Returns
-// whether this arrival completed p.
-__device__ __forceinline__ bool arrive(const RefitBfsArgs& A, int p, int nc) {
-    return atom_add_acq_rel(&A.counter[p], 1) == nc - 1;
+// whether this arrival completed the parent; the counter is then back at zero for the next pass.
+__device__ __forceinline__ bool arrive(int* counter, int nc) {
+    if (atom_add_acq_rel(counter, 1) != nc - 1) return false;
+    *counter = 0;
+    return true;
+}
+
+// Child range {first, count} of node b from its walk record (structure fields, constant here).
+__device__ __forceinline__ int2 child_range(const float4* wb, int b) {
+    const int* pbi = reinterpret_cast<const int*>(wb) + 4 * size_t(b);
+    return make_int2(__ldg(pbi + 1), __ldg(pbi + 2));
+}
+
+// The climb of a warp's completed parents (p, child range pc; -1: none). Each round the four
+// groups of 8 lanes take up to four of them (group k the one held by the k-th lane holding one).
+// combine(q, first child, children, c), called by all lanes (q = -1 for a group without a parent),
+// sums the children's records, lane c of a group child c, and its lane 0 writes the parent; then
+// lane 0 arrives at the grandparent, and a completed grandparent goes back to the lane that held
+// the parent. Each round serves at least one parent and a parent precedes its children in the
+// layout, so the loop ends.
+template <class Combine>
+__device__ __forceinline__ void climb_parents(int p, int2 pc, const int* __restrict__ wparent, const float4* wb,
+                                              int* counter, Combine combine) {
+    const int lane = threadIdx.x & 31;
+    const int grp = lane >> 3, c = lane & 7;
+    for (;;) {
+        const unsigned pend = __ballot_sync(0xffffffffu, p >= 0);
+        if (pend == 0u) break;
+        unsigned rest = pend;  // the holders from the grp-th on (lowest lanes first)
+        for (int k = 0; k < grp; ++k) rest &= rest - 1u;
+        const int src = rest ? __ffs(int(rest)) - 1 : 0;
+        int q = __shfl_sync(0xffffffffu, p, src);
+        const int q0 = __shfl_sync(0xffffffffu, pc.x, src);
+        const int qn = __shfl_sync(0xffffffffu, pc.y, src);
+        if (!rest) q = -1;
+        __syncwarp();  // orders the holder's acquiring arrival before its group's loads
+        int gp = -1;
+        int2 gc = make_int2(0, 0);
+        if (q >= 0 && c == 0) {
+            gp = __ldg(&wparent[q]);
+            if (gp >= 0) gc = child_range(wb, gp);
+        }
+        combine(q, q0, qn, c);
+        int np = -1;
+        if (gp >= 0 && arrive(&counter[gp], gc.y)) np = gp;
+        // back to the holders: the k-th holder (k < 4) was served by group k
+        const int rank = __popc(pend & lanemask_lt());
+        const int from = 8 * min(rank, 3);
+        const int np_ = __shfl_sync(0xffffffffu, np, from);
+        const int nc0_ = __shfl_sync(0xffffffffu, gc.x, from);
+        const int nnc_ = __shfl_sync(0xffffffffu, gc.y, from);
+        if (p >= 0 && rank < 4) {
+            p = np_;
+            pc = make_int2(nc0_, nnc_);
+        }
+    }
 }
 
 // Threads take the nodes from the end of the breadth-first layout (the deepest first), so the
@@ -723,20 +639,15 @@ __device__ __forceinline__ bool arrive(const RefitBfsArgs& A, int p, int nc) {
 // the sums are pairwise with compensation. 64 registers: 4 blocks per SM.
 __global__ void __launch_bounds__(kThreads, 4) k_refit_bfs_quad32(RefitBfsArgs A) {
     const int b = live_nodes(A.span, A.nn_dev) - 1 - int(blockIdx.x * blockDim.x + threadIdx.x);
-    const int lane = threadIdx.x & 31;
-    int p = -1, pc0 = 0, pnc = 0;  // a parent that this lane's arrival completed, its child range
+    int p = -1;  // a parent that this lane's arrival completed, its child range
+    int2 pc = make_int2(0, 0);
     const float4 wb = b >= 0 ? A.wb[b] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int first = __float_as_int(wb.y), code = __float_as_int(wb.z);
     if (b >= 0 && code < 0) {  // a leaf (internal nodes are reached by the climb)
         const int cnt = -code;
         const float4 g = __ldg(&A.wgeo[b]);
         const int par = __ldg(&A.wparent[b]);
-        int c0 = 0, nc = 0;
-        if (par >= 0) {
-            const int* pbi = reinterpret_cast<const int*>(A.wb) + 4 * size_t(par);
-            c0 = __ldg(pbi + 1);
-            nc = __ldg(pbi + 2);
-        }
+        const int2 cr = par >= 0 ? child_range(A.wb, par) : make_int2(0, 0);
         QuadSum S;
         if (cnt <= kLeafMax) {  // the leaf's particles loaded once, together (one memory latency)
             float4 pp[kLeafMax];
@@ -783,33 +694,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_refit_bfs_quad32(RefitBfsArgs A
         }
         A.wq[b] = make_float4(S.xx.s, S.yy.s, S.xy.s, S.xz.s);
         A.wt[b] = make_float2(S.yz.s, S.tr.s);
-        if (par >= 0 && arrive(A, par, nc)) {
+        if (par >= 0 && arrive(&A.counter[par], cr.y)) {
             p = par;
-            pc0 = c0;
-            pnc = nc;
+            pc = cr;
         }
     }
-    // Climb. Each round the four groups of 8 lanes take up to four of the warp's completed
-    // parents (group k the one held by the k-th lane holding one); the group's lane 0 writes
-    // the parent and arrives at the grandparent, and a completed grandparent goes back to the
-    // lane that held the parent. Each round serves at least one parent and a parent precedes
-    // its children in the layout, so the loop ends.
-    const int grp = lane >> 3, c = lane & 7;
-    for (;;) {
-        const unsigned pend = __ballot_sync(0xffffffffu, p >= 0);
-        if (pend == 0u) break;
-        unsigned rest = pend;  // the holders from the grp-th on (lowest lanes first)
-        for (int k = 0; k < grp; ++k) rest &= rest - 1u;
-        const int src = rest ? __ffs(int(rest)) - 1 : 0;
-        int q = __shfl_sync(0xffffffffu, p, src);
-        const int q0 = __shfl_sync(0xffffffffu, pc0, src);
-        const int qn = __shfl_sync(0xffffffffu, pnc, src);
-        if (!rest) q = -1;
-        __syncwarp();  // orders the holder's acquiring arrival before its group's loads
+    climb_parents(p, pc, A.wparent, A.wb, A.counter, [&](int q, int q0, int qn, int c) {
         float4 cm = make_float4(0.f, 0.f, 0.f, 0.f), qc = cm, g = cm;
         float2 yt = make_float2(0.f, 0.f);
         float dmc = 0.f;
-        int gp = -1, gc0 = 0, gnc = 0;
         if (q >= 0) {
             if (c < qn) {
                 cm = __ldcg(&A.wa[q0 + c]);
@@ -817,15 +710,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_refit_bfs_quad32(RefitBfsArgs A
                 qc = __ldcg(&A.wq[q0 + c]);
                 yt = __ldcg(&A.wt[q0 + c]);
             }
-            if (c == 0) {
-                g = __ldg(&A.wgeo[q]);
-                gp = __ldg(&A.wparent[q]);
-                if (gp >= 0) {
-                    const int* pbi = reinterpret_cast<const int*>(A.wb) + 4 * size_t(gp);
-                    gc0 = __ldg(pbi + 1);
-                    gnc = __ldg(pbi + 2);
-                }
-            }
+            if (c == 0) g = __ldg(&A.wgeo[q]);
         }
         // children past qn (and groups without a parent) add zeros
         const float M = group8_sum(cm.w);
@@ -841,25 +726,137 @@ __global__ void __launch_bounds__(kThreads, 4) k_refit_bfs_quad32(RefitBfsArgs A
         const float xz = group8_sum(qc.w + 3.f * m * dx * dz);
         const float yz = group8_sum(yt.x + 3.f * m * dy * dz);
         const float tr = group8_sum(yt.y + m * r2);
-        int np = -1;
         if (q >= 0 && c == 0) {
             finalize_bfs(A, q, g, M, cx, cy, cz, dm);
             A.wq[q] = make_float4(xx, yy, xy, xz);
             A.wt[q] = make_float2(yz, tr);
-            if (gp >= 0 && arrive(A, gp, gnc)) np = gp;
         }
-        // back to the holders: the k-th holder (k < 4) was served by group k
-        const int rank = __popc(pend & lanemask_lt());
-        const int from = 8 * min(rank, 3);
-        const int np_ = __shfl_sync(0xffffffffu, np, from);
-        const int nc0_ = __shfl_sync(0xffffffffu, gc0, from);
-        const int nnc_ = __shfl_sync(0xffffffffu, gnc, from);
-        if (p >= 0 && rank < 4) {
-            p = np_;
-            pc0 = nc0_;
-            pnc = nnc_;
+    });
+}
+
+// Plain form (the reference's arithmetic): monopoles in float64 sums, rounded to the float32 node
+// records (cpp/nbody.cpp:98-131; refit :285-303), in the same bottom-up pass over the breadth-first
+// walk layout. Bound by the float64 pipe and, at small counts, by the chain of arrivals: a leaf's
+// thread sums its particles (7 float64 instructions each), a parent is combined by 8 lanes, one
+// child each. (One thread climbing per subtree and summing its children one after another kept 9 of
+// 32 lanes active: build passes of 10k / 150k particles 64 / 123 us, now 43 / 77 us; refits of
+// 200k 126 -> 72 us; gravity of the 4M cloud 7.07 -> 6.60 ms.)
+struct Moments64Args {
+    int span;
+    const int* nn_dev;
+    bool refit;
+    float theta;
+    const RootBox* root;    // open0: the root's 2 half / theta
+    const int* wparent;
+    const float4* wgeo;     // refit: float32 centre + half
+    const int* dfs;         // build: depth-first id of a breadth-first node
+    const double4* cd;      // build: float64 centre + half, depth-first
+    int* counter;
+    float4* wa;             // com, m
+    float4* wb;             // open_r, first, code, 0
+    float* ndisp;           // refit
+    const int* perm;        // build: particles in float64
+    const double* xbuild;
+    const double* mass;
+    const float4* p4;       // refit: the float32 copies
+    const float* pdisp;
+};
+
+__device__ __forceinline__ void finalize64(const Moments64Args& A, int b, const double4& c, double M, double sx,
+                                           double sy, double sz, float dm) {
+    const double inv = exponent_of(M) - 123u < 1800u ? inverse(M) : M > 0 ? __drcp_rn(M) : 0.0;
+    const double mx = __dmul_rn(sx, inv), my = __dmul_rn(sy, inv), mz = __dmul_rn(sz, inv);
+    A.wa[b] = make_float4(float(mx), float(my), float(mz), float(M));
+    const double ox = __dsub_rn(mx, c.x), oy = __dsub_rn(my, c.y), oz = __dsub_rn(mz, c.z);
+    double first;
+    if (!A.refit) {
+        // 2 half / theta (cpp/nbody.cpp:104-106): half is the root's, halved depth times, so the
+        // quotient is the root's scaled by the same power of two (both exponents drop alike)
+        const double open0 = A.root->open0;
+        const int drop = __double2hiint(A.root->half) - __double2hiint(c.w);
+        first = __hiloint2double(__double2hiint(open0) - drop, __double2loint(open0));
+    } else {  // cpp/nbody.cpp:301-303: the first term is evaluated in float32
+        first = double(__fdiv_rn(__fmul_rn(2.0f, __fadd_rn(float(c.w), dm)), A.theta));
+        A.ndisp[b] = dm;
+    }
+    double r, inv_r;
+    inv_root(__dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz)), r, inv_r);
+    A.wb[b].x = float(__dadd_rn(first, r));
+}
+
+// The centre and half of node b's cell, as the pass measures against them.
+__device__ __forceinline__ double4 cell64(const Moments64Args& A, int b) {
+    if (!A.refit) return A.cd[A.dfs[b]];
+    const float4 g = __ldg(&A.wgeo[b]);
+    return make_double4(double(g.x), double(g.y), double(g.z), double(g.w));
+}
+
+__global__ void __launch_bounds__(kThreads) k_moments64(Moments64Args A) {
+    const int b = live_nodes(A.span, A.nn_dev) - 1 - int(blockIdx.x * blockDim.x + threadIdx.x);
+    int p = -1;
+    int2 pc = make_int2(0, 0);
+    const float4 wb = b >= 0 ? A.wb[b] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int first = __float_as_int(wb.y), code = __float_as_int(wb.z);
+    if (b >= 0 && code < 0) {  // a leaf: its particles in order (cpp/nbody.cpp:124-131, refit :285-289)
+        const double4 g = cell64(A, b);
+        const int par = __ldg(&A.wparent[b]);
+        const int2 cr = par >= 0 ? child_range(A.wb, par) : make_int2(0, 0);
+        double M = 0, sx = 0, sy = 0, sz = 0;
+        float dm = 0.f;
+        for (int base = 0; base < -code; base += kLeafMax) {  // once, but for leaves at the depth limit
+            double4 pm[kLeafMax];
+            float pd[kLeafMax];
+#pragma unroll
+            for (int t = 0; t < kLeafMax; ++t) {  // loaded together
+                pm[t] = make_double4(0.0, 0.0, 0.0, 0.0);
+                pd[t] = 0.f;
+                if (base + t < -code) {
+                    const int i = first + base + t;
+                    if (!A.refit) {
+                        pm[t] = make_double4(A.xbuild[3 * size_t(i)], A.xbuild[3 * size_t(i) + 1],
+                                             A.xbuild[3 * size_t(i) + 2], A.mass ? A.mass[A.perm[i]] : 1.0);
+                    } else {
+                        const float4 q = A.p4[i];
+                        pm[t] = make_double4(double(q.x), double(q.y), double(q.z), double(q.w));
+                        pd[t] = A.pdisp[i];
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < kLeafMax; ++t) {
+                if (base + t < -code) {
+                    M = __dadd_rn(M, pm[t].w);
+                    sx = __dadd_rn(sx, __dmul_rn(pm[t].w, pm[t].x));
+                    sy = __dadd_rn(sy, __dmul_rn(pm[t].w, pm[t].y));
+                    sz = __dadd_rn(sz, __dmul_rn(pm[t].w, pm[t].z));
+                    dm = fmaxf(dm, pd[t]);
+                }
+            }
+        }
+        finalize64(A, b, g, M, sx, sy, sz, dm);
+        if (par >= 0 && arrive(&A.counter[par], cr.y)) {
+            p = par;
+            pc = cr;
         }
     }
+    climb_parents(p, pc, A.wparent, A.wb, A.counter, [&](int q, int q0, int qn, int c) {
+        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
+        double4 g = make_double4(0.0, 0.0, 0.0, 0.0);
+        float dmc = 0.f;
+        if (q >= 0) {
+            if (c < qn) {
+                cm = __ldcg(&A.wa[q0 + c]);
+                if (A.refit) dmc = __ldcg(&A.ndisp[q0 + c]);
+            }
+            if (c == 0) g = cell64(A, q);
+        }
+        const double m = double(cm.w);  // (products of float32 values are exact in float64)
+        const double M = group8_sum(m);
+        const double sx = group8_sum(m * double(cm.x)), sy = group8_sum(m * double(cm.y)),
+                     sz = group8_sum(m * double(cm.z));
+        const float dm = A.refit ? group8_max(dmc) : 0.f;
+        if (q >= 0 && c == 0) finalize64(A, q, g, M, sx, sy, sz, dm);
+    });
 }
 
 // ---------------------------------------------------------------------------- groups + layout
@@ -901,10 +898,9 @@ __global__ void k_bfs_index(int span, const int* __restrict__ nn_dev, const int*
     bfs[val[b]] = b;
 }
 
+// The structure of the breadth-first layout (the moments passes write the rest afterwards).
 __global__ void k_walk_fill(int nn, const int4* __restrict__ n_i4, const int* __restrict__ nchild,
-                            const int* __restrict__ bfs, const float4* __restrict__ mom,
-                            const float* __restrict__ open_r, const float4* __restrict__ geo,
-                            float4* __restrict__ wa, float4* __restrict__ wb,
+                            const int* __restrict__ bfs, const float4* __restrict__ geo, float4* __restrict__ wb,
                             float4* __restrict__ wgeo, int* __restrict__ leaf_of,
                             const int* __restrict__ parent, int* __restrict__ wparent, const int* __restrict__ nn_dev) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -921,12 +917,9 @@ __global__ void k_walk_fill(int nn, const int4* __restrict__ n_i4, const int* __
         first = bfs[k + 1];
         code = nchild[k];
     }
-    // mom null (mixed-form build, neighbour-search trees): no moments here (the mixed form
-    // writes them into this layout afterwards)
-    wa[b] = mom ? mom[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    wb[b] = make_float4(mom ? open_r[k] : 0.f, __int_as_float(first), __int_as_float(code), 0.f);
-    if (wgeo) wgeo[b] = geo[k];
-    if (wparent) wparent[b] = parent[k] < 0 ? -1 : bfs[parent[k]];
+    wb[b] = make_float4(0.f, __int_as_float(first), __int_as_float(code), 0.f);
+    wgeo[b] = geo[k];
+    wparent[b] = parent[k] < 0 ? -1 : bfs[parent[k]];
 }
 
 // ---------------------------------------------------------------------------- deep cells
@@ -1076,7 +1069,7 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     const int nparts = std::min(4 * C.sms, std::max(1, grid));
     int* nb = nbase.get<int>(std::max(size_t(n) + 1, size_t(nparts) * 14 + 16));
     double* part = reinterpret_cast<double*>(nb);  // bbox partials, consumed before the scan
-    k_bbox<<<nparts, kThreads, 0, s>>>(pos, n, part, R, C.d_status, &cnt->bbox_done);
+    k_bbox<<<nparts, kThreads, 0, s>>>(pos, n, part, R, double(theta_f), C.d_status, &cnt->bbox_done);
     GF_CHECK_LAUNCH();
 
     uint64_t* k0 = key.get<uint64_t>(n);
@@ -1158,8 +1151,7 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     }
     int* nch = n_nchild.get<int>(cap);
     int* ctr = n_counter.get<int>(cap);
-    int* kid = n_kids.get<int>(8 * size_t(cap));
-    k_nchild<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, nch, ctr, kid);
+    k_nchild<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, nch, ctr);
     GF_CHECK_LAUNCH();
     k_leaf_sort<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, pm);
     GF_CHECK_LAUNCH();
@@ -1169,38 +1161,6 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     k_gather<<<grid, kThreads, 0, s>>>(n, pm, pos, mass, nullptr, pp, nullptr,
                                        want_knn ? plo.get<float4>(n) : nullptr, 0, xb);
     GF_CHECK_LAUNCH();
-
-    float4* mom = n_mom.get<float4>(cap);
-    float* opr = n_open.get<float>(cap);
-    float* ndp = n_disp.get<float>(cap);
-    if (want_knn) {
-        // a neighbour-search tree needs geometry only: no moments (the walk layout's mass and
-        // opening-radius fields stay unused)
-    } else if (quad) {
-        // mixed form: moments in the breadth-first walk layout, after it is laid out (below)
-    } else {
-        MomentArgs A{};
-        A.nn = span;
-        A.nn_dev = nn_dev;
-        A.refit = false;
-        A.theta = theta_f;
-        A.n_i4 = i4;
-        A.parent = par;
-        A.nchild = nch;
-        A.kids = kid;
-        A.counter = ctr;
-        A.n_cd = cd;
-        A.n_geo = geo;
-        A.mom = mom;
-        A.open_r = opr;
-        A.ndisp = ndp;
-        A.perm = pm;
-        A.pos = pos;
-        A.mass = mass;
-        ProfScope psm(kStTreeMoments, s);
-        k_moments<<<ngrid, kThreads, 0, s>>>(A);
-        GF_CHECK_LAUNCH();
-    }
 
     int* gf_ = gflag.get<int>(cap);
     int* gs = gscan.get<int>(cap);
@@ -1218,23 +1178,20 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     int* bfs = n_bfs.get<int>(cap);
     k_bfs_index<<<ngrid, kThreads, 0, s>>>(span, nn_dev, bv, bfs);
     GF_CHECK_LAUNCH();
-    // breadth-first geometry and parents: the neighbour search, and the mixed form's refit
-    const bool bfs_geo = want_knn || quad;
-    const bool bfs_moments = quad && !want_knn;
-    k_walk_fill<<<ngrid, kThreads, 0, s>>>(span, i4, nch, bfs, bfs_moments ? nullptr : mom, opr, geo,
-                                           w_a.get<float4>(cap), w_b.get<float4>(cap),
-                                           bfs_geo ? w_geo.get<float4>(cap) : nullptr,
-                                           want_knn ? leaf_of.get<int>(n) : nullptr, par,
-                                           bfs_geo ? w_parent.get<int>(cap) : nullptr, nn_dev);
+    k_walk_fill<<<ngrid, kThreads, 0, s>>>(span, i4, nch, bfs, geo, w_b.get<float4>(cap), w_geo.get<float4>(cap),
+                                           want_knn ? leaf_of.get<int>(n) : nullptr, par, w_parent.get<int>(cap),
+                                           nn_dev);
     GF_CHECK_LAUNCH();
-    if (bfs_moments) {  // mixed form: float32 monopole + quadrupole moments in one bottom-up pass
-        GF_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * size_t(span), s));
-        RefitBfsArgs A{span, nn_dev, theta_f, w_parent.as<int>(), w_geo.as<float4>(), ctr, w_a.as<float4>(),
-                       w_b.as<float4>(), w_q.get<float4>(cap), w_t.get<float2>(cap), w_rq.get<float>(cap), ndp, pp,
-                       nullptr};
+    if (!want_knn) {  // (a neighbour-search tree needs geometry only)
+        w_a.get<float4>(cap);
+        n_disp.get<float>(cap);
+        if (quad) {
+            w_q.get<float4>(cap);
+            w_t.get<float2>(cap);
+            w_rq.get<float>(cap);
+        }
         ProfScope psm(kStTreeMoments, s);
-        k_refit_bfs_quad32<<<ngrid, kThreads, 0, s>>>(A);
-        GF_CHECK_LAUNCH();
+        moments(mass, false, span, s);
     }
     valid = true;
     if (!g_no_alloc) {  // outside a capture: the live node count, for outgrowing()
@@ -1277,42 +1234,26 @@ void Octree::refit(const double* pos, const double* mass, cudaStream_t s, cudaSt
         GF_CUDA(cudaStreamWaitEvent(s_moments, gathered, 0));
         s = s_moments;
     }
-    int* ctr = n_counter.as<int>();
-    GF_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * size_t(span), s));
-    if (quad) {  // mixed form: straight into the walk layout
-        RefitBfsArgs A{span, nn_dev, theta_f, w_parent.as<int>(), w_geo.as<float4>(), ctr, w_a.as<float4>(),
-                       w_b.as<float4>(), w_q.as<float4>(), w_t.as<float2>(), w_rq.as<float>(), n_disp.as<float>(), pp,
-                       pd};
+    moments(mass, true, span, s);
+}
+
+// The bottom-up moments pass of a build or a refit, straight into the breadth-first walk layout.
+// (The arrival counters are zero: k_nchild clears them in a build, and each pass leaves them so.)
+void Octree::moments(const double* mass, bool refit, int span, cudaStream_t s) {
+    const int* nn_dev = &counts.as<TreeCounts>()->total_nodes;
+    const int ngrid = div_up(span, kThreads);
+    if (quad) {
+        RefitBfsArgs A{span, nn_dev, theta_f, w_parent.as<int>(), w_geo.as<float4>(), n_counter.as<int>(),
+                       w_a.as<float4>(), w_b.as<float4>(), w_q.as<float4>(), w_t.as<float2>(), w_rq.as<float>(),
+                       n_disp.as<float>(), p4.as<float4>(), refit ? pdisp.as<float>() : nullptr};
         k_refit_bfs_quad32<<<ngrid, kThreads, 0, s>>>(A);
-        GF_CHECK_LAUNCH();
-        return;
     } else {
-        MomentArgs A{};
-        A.nn = span;
-        A.nn_dev = nn_dev;
-        A.refit = true;
-        A.theta = theta_f;
-        A.n_i4 = n_i4.as<int4>();
-        A.parent = n_parent.as<int>();
-        A.nchild = n_nchild.as<int>();
-        A.kids = n_kids.as<int>();
-        A.counter = ctr;
-        A.n_cd = n_cd.as<double4>();
-        A.n_geo = n_geo.as<float4>();
-        A.mom = n_mom.as<float4>();
-        A.open_r = n_open.as<float>();
-        A.ndisp = n_disp.as<float>();
-        A.p4 = pp;
-        A.pdisp = pd;
-        k_moments<<<ngrid, kThreads, 0, s>>>(A);
-        GF_CHECK_LAUNCH();
+        Moments64Args A{span, nn_dev, refit, theta_f, root.as<RootBox>(), w_parent.as<int>(), w_geo.as<float4>(),
+                        bfs_val.as<int>(), n_cd.as<double4>(), n_counter.as<int>(), w_a.as<float4>(),
+                        w_b.as<float4>(), n_disp.as<float>(), perm.as<int>(), xbuild.as<double>(), mass,
+                        p4.as<float4>(), refit ? pdisp.as<float>() : nullptr};
+        k_moments64<<<ngrid, kThreads, 0, s>>>(A);
     }
-    k_walk_fill<<<ngrid, kThreads, 0, s>>>(span, n_i4.as<int4>(), n_nchild.as<int>(), n_bfs.as<int>(),
-                                           n_mom.as<float4>(), n_open.as<float>(), n_geo.as<float4>(),
-                                           w_a.as<float4>(), w_b.as<float4>(),
-                                           want_knn ? w_geo.as<float4>() : nullptr,
-                                           want_knn ? leaf_of.as<int>() : nullptr, n_parent.as<int>(),
-                                           want_knn ? w_parent.as<int>() : nullptr, nn_dev);
     GF_CHECK_LAUNCH();
 }
 

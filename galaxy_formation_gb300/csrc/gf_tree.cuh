@@ -19,6 +19,7 @@ constexpr int kNumWalkShapes = 4;
 struct RootBox {
     double c[3];
     double half;
+    double open0;     // 2 half / theta, the geometric part of the root's opening radius
     double lo[3];     // c - half
     double inv_w;     // 2^21 / (2 half): grid units per unit length
     double margin;    // grid units: closer than this to a cell wall -> exact path
@@ -55,12 +56,9 @@ struct Octree {
     DevBuf cpl9, ldepth, dsplit, nstart, nbase, node_owner;
     // nodes, depth-first (preorder) order
     DevBuf n_i4;      // int4 {start, count, next, leaf | depth << 8}
-    DevBuf n_mom;     // float4 {cx, cy, cz, m}
-    DevBuf n_open;    // float open_r
     DevBuf n_geo;     // float4 {gx, gy, gz, half}
     DevBuf n_cd;      // double4 {centre, half} (build only)
     DevBuf n_parent, n_nchild, n_counter, n_disp, n_bfs;
-    DevBuf n_kids;    // children of each node in octant order (8 slots per node)
     // walk layout, breadth-first order: children of a node are contiguous
     DevBuf w_a;       // float4 {cx, cy, cz, m}
     DevBuf w_b;       // float4 {open_r, first (int bits), code (int bits), rho};
@@ -113,6 +111,7 @@ struct Octree {
     // need the positions only, can be prepared on s meanwhile).
     void refit(const double* pos, const double* mass, cudaStream_t s, cudaStream_t s_moments = nullptr,
                cudaEvent_t gathered = nullptr);
+    void moments(const double* mass, bool refit, int span, cudaStream_t s);
     // Work list of groups with at least one active particle (active may be null); chunk in
     // 1..kChunkMax cuts each group's active particles into items of <= chunk with their own
     // spheres; chunk in kChunkMax+1..kChunkCodeMax (active sets) merges runs of sibling groups
