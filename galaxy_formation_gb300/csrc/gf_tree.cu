@@ -28,6 +28,8 @@
 #include <cfloat>
 #include <climits>
 
+#include <cooperative_groups.h>
+
 #include "gf_tree.cuh"
 
 namespace gf {
@@ -48,6 +50,37 @@ __device__ __forceinline__ long long fkey(double v) {
 __device__ __forceinline__ double fkey_inv(long long k) { return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL)); }
 __device__ __forceinline__ bool finite_bits(double v) {
     return ((__double_as_longlong(v) >> 52) & 0x7ff) != 0x7ff;
+}
+
+// Root cube of a bounding box tot = {lo x, y, z, hi x, y, z} (cpp/nbody.cpp:218-219) and the grid of
+// the fast key path.
+__device__ RootBox root_box(const double (&tot)[6], double theta) {
+    RootBox R;
+    double ext = 0;
+    for (int a = 0; a < 3; ++a) {
+        R.c[a] = __dmul_rn(0.5, __dadd_rn(tot[a], tot[3 + a]));
+        ext = fmax(ext, __dsub_rn(tot[3 + a], tot[a]));
+    }
+    // 0.5 * max extent * 1.0001 + 1e-12 (cpp/nbody.cpp:219), unfused
+    R.half = __dadd_rn(__dmul_rn(__dmul_rn(0.5, ext), 1.0001), 1e-12);
+    R.open0 = __ddiv_rn(__dmul_rn(2.0, R.half), theta);
+    double cmax = 0;
+    for (int a = 0; a < 3; ++a) {
+        R.lo[a] = __dsub_rn(R.c[a], R.half);
+        cmax = fmax(cmax, fabs(R.c[a]));
+    }
+    R.inv_w = __ddiv_rn(2097152.0, __dmul_rn(2.0, R.half));
+    // Rounding of the float64 centre chain (<= 21 roundings of <= 1/2 ulp(|c| + half)) plus
+    // that of the fixed-point position stays below 2^-27 (|c|/half + 2) grid units; the
+    // margin keeps a factor 8 on top.
+    R.margin = ldexp(1.0, -24) * (cmax / R.half + 2.0);
+    // the same test in 32.32 fixed point (scaling by 2^32 is exact): the fraction window
+    // [m_lo, m_hi] of the truncated fixed-point position lies inside [margin, 1 - margin]
+    R.inv_w32 = R.inv_w * 4294967296.0;
+    const double ml = fmin(ceil(R.margin * 4294967296.0), 2147483648.0);
+    R.m_lo = uint32_t(ml);
+    R.m_hi = uint32_t(4294967295.0 - ml);
+    return R;
 }
 
 // float64 bounding box -> root cube (cpp/nbody.cpp:210-219) in one launch: every block reduces
@@ -133,32 +166,7 @@ __global__ void k_bbox(const double* __restrict__ pos, int n, double* __restrict
     double tot[6];
     for (int a = 0; a < 6; ++a) tot[a] = fkey_inv(itot[a]);
     if (tot_bad) raise_status(status, GF_ERR_NONFINITE);
-    RootBox R;
-    double ext = 0;
-    for (int a = 0; a < 3; ++a) {
-        R.c[a] = __dmul_rn(0.5, __dadd_rn(tot[a], tot[3 + a]));
-        ext = fmax(ext, __dsub_rn(tot[3 + a], tot[a]));
-    }
-    // 0.5 * max extent * 1.0001 + 1e-12 (cpp/nbody.cpp:219), unfused
-    R.half = __dadd_rn(__dmul_rn(__dmul_rn(0.5, ext), 1.0001), 1e-12);
-    R.open0 = __ddiv_rn(__dmul_rn(2.0, R.half), theta);
-    double cmax = 0;
-    for (int a = 0; a < 3; ++a) {
-        R.lo[a] = __dsub_rn(R.c[a], R.half);
-        cmax = fmax(cmax, fabs(R.c[a]));
-    }
-    R.inv_w = __ddiv_rn(2097152.0, __dmul_rn(2.0, R.half));
-    // Rounding of the float64 centre chain (<= 21 roundings of <= 1/2 ulp(|c| + half)) plus
-    // that of the fixed-point position stays below 2^-27 (|c|/half + 2) grid units; the
-    // margin keeps a factor 8 on top.
-    R.margin = ldexp(1.0, -24) * (cmax / R.half + 2.0);
-    // the same test in 32.32 fixed point (scaling by 2^32 is exact): the fraction window
-    // [m_lo, m_hi] of the truncated fixed-point position lies inside [margin, 1 - margin]
-    R.inv_w32 = R.inv_w * 4294967296.0;
-    const double ml = fmin(ceil(R.margin * 4294967296.0), 2147483648.0);
-    R.m_lo = uint32_t(ml);
-    R.m_hi = uint32_t(4294967295.0 - ml);
-    *root = R;
+    *root = root_box(tot, theta);
 }
 
 // ---------------------------------------------------------------------------- keys
@@ -210,12 +218,8 @@ __device__ __forceinline__ bool grid_coord(double x, int a, const RootBox& R, ui
     return ic < 2097152u && fr >= R.m_lo && fr <= R.m_hi;
 }
 
-__global__ void k_keys(const double* __restrict__ pos, int n, const RootBox* __restrict__ rootp,
-                       uint64_t* __restrict__ key, int* __restrict__ perm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const RootBox R = *rootp;
-    const double x = pos[3 * size_t(i)], y = pos[3 * size_t(i) + 1], z = pos[3 * size_t(i) + 2];
+// The 63-bit Morton key: the octants of levels 1..21.
+__device__ __forceinline__ uint64_t morton_key(double x, double y, double z, const RootBox& R) {
     uint32_t ix, iy, iz;
     uint64_t k;
     if (grid_coord(x, 0, R, ix) && grid_coord(y, 1, R, iy) && grid_coord(z, 2, R, iz)) {
@@ -224,8 +228,219 @@ __global__ void k_keys(const double* __restrict__ pos, int n, const RootBox* __r
         uint64_t k1, k2;
         exact_keys(x, y, z, R, 21, k, k1, k2);
     }
-    key[i] = k;
+    return k;
+}
+
+__global__ void k_keys(const double* __restrict__ pos, int n, const RootBox* __restrict__ rootp,
+                       uint64_t* __restrict__ key, int* __restrict__ perm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const RootBox R = *rootp;
+    key[i] = morton_key(pos[3 * size_t(i)], pos[3 * size_t(i) + 1], pos[3 * size_t(i) + 2], R);
     perm[i] = i;
+}
+
+// ---------------------------------------------------------------------------- small sets
+
+// Bounding box, keys and their radix sort in one launch, for sets that fit the shared memory of one
+// cluster: kSmallCtas blocks hold m consecutive positions each; eight 8-bit passes rank the keys
+// as the one-sweep sort does (match-any per warp, warps in key order), add up the blocks' digit
+// counts through distributed shared memory and scatter keys and indices straight into the block
+// that holds their new position. Two cluster barriers a pass take the place of a launch, a digit
+// histogram and a look-back. A pass costs about 12,000 cycles at 10k keys, half of it barriers and
+// their latencies, and grows with the keys per block (match-any, scattered remote stores), so the
+// chain of 12 launches is as fast from about 28k keys on: Engine.gravity with the chain / with this
+// launch 325 / 267 us at 5k particles, 350 / 302 at 10k, 366 / 354 at 24k, 375 / 381 at 32k.
+static_assert(kKeyLevels == 21, "eight 8-bit passes over a 63-bit key");
+constexpr int kSmallCtas = 8;
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallItems = 4;                             // keys per thread at most
+constexpr int kSmallMaxPer = kSmallThreads * kSmallItems;  // positions per block at most
+constexpr int kSmallMax = 28 * 1024;
+static_assert(kSmallMax <= kSmallCtas * kSmallMaxPer, "a block's positions fit its threads");
+
+constexpr size_t small_sort_smem(int m) {
+    return size_t(m) * 2 * (sizeof(uint64_t) + sizeof(int)) + sizeof(uint16_t) * kSmallWarps * 256;
+}
+
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
+    k_small_sort(const double* __restrict__ pos, int n, int m, unsigned div_m, double theta, RootBox* __restrict__ root,
+                 uint64_t* __restrict__ key, int* __restrict__ perm, uint32_t* status) {
+    extern __shared__ unsigned char smem_small[];
+    uint64_t* kb = reinterpret_cast<uint64_t*>(smem_small);  // two buffers of m keys
+    int* vb = reinterpret_cast<int*>(kb + 2 * m);            // two of m indices
+    uint16_t* cnt = reinterpret_cast<uint16_t*>(vb + 2 * m);  // [warp][digit]
+    __shared__ int s_tot[kSmallCtas][256], s_part[4][256], s_base[256], s_wsum[kSmallWarps];
+    __shared__ long long s_box[7], s_red[kSmallWarps][7];
+    __shared__ RootBox s_root;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = int(cluster.block_rank());
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = lanemask_lt();
+    const int first = rank * m;                   // this block's positions: [first, first + own)
+    const int own = max(0, min(m, n - first));
+
+    // bounding box of the block's share, then of all blocks (exact: min and max of integer images)
+    long long v[7] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0};
+    for (int o = tid; o < own; o += kSmallThreads) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const double x = pos[3 * size_t(first + o) + a];
+            v[6] |= finite_bits(x) ? 0 : 1;
+            const long long k = fkey(x);
+            v[a] = min(v[a], k);
+            v[3 + a] = max(v[3 + a], k);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            v[a] = min(v[a], __shfl_xor_sync(0xffffffffu, v[a], o));
+            v[3 + a] = max(v[3 + a], __shfl_xor_sync(0xffffffffu, v[3 + a], o));
+        }
+        v[6] |= __shfl_xor_sync(0xffffffffu, v[6], o);
+    }
+    if (lane == 0)
+        for (int a = 0; a < 7; ++a) s_red[warp][a] = v[a];
+    __syncthreads();
+    if (tid < 7) {
+        long long x = s_red[0][tid];
+        for (int w = 1; w < kSmallWarps; ++w) {
+            const long long y = s_red[w][tid];
+            x = tid < 3 ? min(x, y) : tid < 6 ? max(x, y) : x | y;
+        }
+        s_box[tid] = x;
+    }
+    cluster.sync();
+    if (tid < 7) {
+        long long x = *cluster.map_shared_rank(&s_box[tid], 0);
+        for (int c = 1; c < kSmallCtas; ++c) {
+            const long long y = *cluster.map_shared_rank(&s_box[tid], c);
+            x = tid < 3 ? min(x, y) : tid < 6 ? max(x, y) : x | y;
+        }
+        s_red[0][tid] = x;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double tot[6];
+        for (int a = 0; a < 6; ++a) tot[a] = fkey_inv(s_red[0][a]);
+        s_root = root_box(tot, theta);
+        if (rank == 0) {
+            *root = s_root;
+            if (s_red[0][6]) raise_status(status, GF_ERR_NONFINITE);
+        }
+    }
+    __syncthreads();
+    {
+        const RootBox R = s_root;
+        for (int o = tid; o < own; o += kSmallThreads) {
+            const double* p = pos + 3 * size_t(first + o);
+            kb[o] = morton_key(p[0], p[1], p[2], R);
+            vb[o] = first + o;
+        }
+    }
+    __syncthreads();
+
+    const int items = (m + kSmallThreads - 1) / kSmallThreads;  // per thread, uniform over the cluster
+    const int wbase = warp * 32 * items;                        // a warp's consecutive positions
+    auto clear_counts = [&] {
+        for (int t = lane; t < 128; t += 32) reinterpret_cast<unsigned*>(cnt + warp * 256)[t] = 0u;
+        __syncwarp();
+    };
+    clear_counts();
+    for (int pass = 0; pass < 8; ++pass) {
+        const uint64_t* ki = kb + (pass & 1) * m;
+        const int* vi = vb + (pass & 1) * m;
+        uint64_t* ko = kb + (1 - (pass & 1)) * m;
+        int* vo = vb + (1 - (pass & 1)) * m;
+        const int shift = 8 * pass;
+        uint64_t k[kSmallItems];
+        int rk[kSmallItems];
+#pragma unroll
+        for (int s = 0; s < kSmallItems; ++s) {
+            if (s >= items) break;
+            const int o = wbase + 32 * s + lane;
+            const bool ok = o < own;
+            k[s] = ok ? ki[o] : 0ull;
+            const unsigned d = ok ? unsigned(k[s] >> shift) & 255u : 256u;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const int before = ok ? cnt[warp * 256 + d] : 0;
+            rk[s] = before + __popc(peers & lt);
+            __syncwarp();
+            if (ok && lane == __ffs(peers) - 1) cnt[warp * 256 + d] = uint16_t(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // four threads per digit: exclusive prefix over the warps; the block's count of every digit
+        // goes to all blocks
+        const int d = tid & 255, part = tid >> 8;
+        constexpr int kPart = kSmallWarps / 4;
+        int sum = 0;
+#pragma unroll
+        for (int w = 0; w < kPart; ++w) sum += cnt[(part * kPart + w) * 256 + d];
+        s_part[part][d] = sum;
+        __syncthreads();
+        int run = 0, own_d = 0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int x = s_part[t][d];
+            if (t < part) run += x;
+            own_d += x;
+        }
+#pragma unroll
+        for (int c = 2 * part; c < 2 * part + 2; ++c) *cluster.map_shared_rank(&s_tot[rank][d], c) = own_d;
+        auto counted = cluster.barrier_arrive();
+#pragma unroll
+        for (int w = 0; w < kPart; ++w) {
+            const int c = cnt[(part * kPart + w) * 256 + d];
+            cnt[(part * kPart + w) * 256 + d] = uint16_t(run);
+            run += c;
+        }
+        cluster.barrier_wait(std::move(counted));
+        // the digit's keys in all blocks, and in the blocks before this one
+        int all = 0, prev = 0;
+        if (tid < 256) {
+#pragma unroll
+            for (int c = 0; c < kSmallCtas; ++c) {
+                const int x = s_tot[c][tid];
+                all += x;
+                if (c < rank) prev += x;
+            }
+        }
+        int scan = warp_incl_scan(all);  // over the 256 digits: the first eight warps
+        if (lane == 31) s_wsum[warp] = scan;
+        __syncthreads();
+        if (tid < 256) {
+            int before = 0;
+            for (int w = 0; w < warp; ++w) before += s_wsum[w];
+            s_base[tid] = before + scan - all + prev;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < kSmallItems; ++s) {
+            if (s >= items) break;
+            const int o = wbase + 32 * s + lane;
+            if (o < own) {
+                const unsigned dg = unsigned(k[s] >> shift) & 255u;
+                const unsigned to = unsigned(s_base[dg] + int(cnt[warp * 256 + dg]) + rk[s]);
+                const unsigned c = __umulhi(to, div_m);  // to / m
+                const unsigned off = to - c * unsigned(m);
+                *cluster.map_shared_rank(ko + off, c) = k[s];
+                *cluster.map_shared_rank(vo + off, c) = vi[o];
+            }
+        }
+        auto scattered = cluster.barrier_arrive();
+        __syncwarp();
+        clear_counts();
+        cluster.barrier_wait(std::move(scattered));
+    }
+    for (int o = tid; o < own; o += kSmallThreads) {
+        key[first + o] = kb[o];
+        perm[first + o] = vb[o];
+    }
 }
 
 // ---------------------------------------------------------------------------- prefixes
@@ -1052,6 +1267,21 @@ void Octree::deep_sort_attr() {
     }
 }
 
+void Octree::small_sort(const double* pos, cudaStream_t s) {
+    static bool attr = false;
+    if (!attr) {
+        GF_CUDA(cudaFuncSetAttribute(k_small_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(small_sort_smem(kSmallMaxPer))));
+        attr = true;
+    }
+    const int m = std::max(2, div_up(n, kSmallCtas));
+    // floor(t / m) = mulhi(t, div_m) for every t below kSmallMax: t m < 2^32
+    const unsigned div_m = m > 1 ? unsigned((0x100000000ull + m - 1) / m) : 0u;
+    k_small_sort<<<kSmallCtas, kSmallThreads, small_sort_smem(m), s>>>(
+        pos, n, m, div_m, double(theta_f), root.as<RootBox>(), key.as<uint64_t>(), perm.as<int>(), ctx().d_status);
+    GF_CHECK_LAUNCH();
+}
+
 void Octree::build(int n_, const double* pos, const double* mass, double theta, cudaStream_t s, bool graph_safe) {
     Context& C = ctx();
     ProfScope ps(want_knn ? kStKnnTree : kStTreeBuild, s);
@@ -1066,19 +1296,23 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     GF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(TreeCounts), s));
 
     const int grid = div_up(n, kThreads);
-    const int nparts = std::min(4 * C.sms, std::max(1, grid));
-    int* nb = nbase.get<int>(std::max(size_t(n) + 1, size_t(nparts) * 14 + 16));
-    double* part = reinterpret_cast<double*>(nb);  // bbox partials, consumed before the scan
-    k_bbox<<<nparts, kThreads, 0, s>>>(pos, n, part, R, double(theta_f), C.d_status, &cnt->bbox_done);
-    GF_CHECK_LAUNCH();
-
     uint64_t* k0 = key.get<uint64_t>(n);
     int* pm = perm.get<int>(n);
-    k_keys<<<grid, kThreads, 0, s>>>(pos, n, R, k0, pm);
-    GF_CHECK_LAUNCH();
-    {
+    key_alt.get<uint64_t>(n);
+    perm_alt.get<int>(n);
+    const int nparts = std::min(4 * C.sms, std::max(1, grid));
+    int* nb = nbase.get<int>(std::max(size_t(n) + 1, size_t(nparts) * 14 + 16));
+    if (n <= kSmallMax) {
         ProfScope pso(want_knn ? kStCount : kStTreeSort, s);
-        radix_sort_pairs(k0, pm, key_alt.get<uint64_t>(n), perm_alt.get<int>(n), n, 0, 63, s, &scratch);
+        small_sort(pos, s);
+    } else {
+        double* part = reinterpret_cast<double*>(nb);  // bbox partials, consumed before the scan
+        k_bbox<<<nparts, kThreads, 0, s>>>(pos, n, part, R, double(theta_f), C.d_status, &cnt->bbox_done);
+        GF_CHECK_LAUNCH();
+        k_keys<<<grid, kThreads, 0, s>>>(pos, n, R, k0, pm);
+        GF_CHECK_LAUNCH();
+        ProfScope pso(want_knn ? kStCount : kStTreeSort, s);
+        radix_sort_pairs(k0, pm, key_alt.as<uint64_t>(), perm_alt.as<int>(), n, 0, 63, s, &scratch);
     }
 
     int8_t* c9 = cpl9.get<int8_t>(n);

@@ -103,6 +103,7 @@ struct Octree {
     // outgrows node_cap raises GF_ERR_CAPACITY and is left empty).
     void build(int n, const double* pos, const double* mass, double theta, cudaStream_t s,
                bool graph_safe = false);
+    void small_sort(const double* pos, cudaStream_t s);
     void reserve_graph_build();
     void deep_sort_attr();
     // Node kernels read the live node count on the device (valid after captured rebuilds).

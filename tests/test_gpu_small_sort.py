@@ -1,0 +1,28 @@
+"""The one-launch bounding box, keys and sort of small sets: the tree equals the oracle's node for
+node (structure, particle order) at the edges of the split over the cluster's blocks (fewer
+particles than blocks, empty last blocks, uneven shares) and of the launch rule (28,672 particles
+and one more), with coincident points, points on cell walls and cells deeper than a key."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 17, 63, 1023, 8191, 8193, 10000, 28671, 28672, 28673])
+@pytest.mark.parametrize("kind", ["normal", "grid", "deep"])
+def test_small_sort_builds_the_same_tree(gpulib, oracle, n, kind):
+    from galaxy_formation_gb300.engine import Engine
+
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(n, 3))
+    if kind == "grid":  # many ties and coordinates on cell walls
+        x = np.round(x * 4) / 4
+    elif kind == "deep":  # groups that only separate below level 21, and coincident ones
+        x = x[rng.integers(0, max(1, n // 12), n)]
+        x[::2] *= 1 + 1e-9 * rng.integers(0, 4, size=(len(x[::2]), 1))
+    x = np.ascontiguousarray(x)
+    m = rng.uniform(0.5, 1.5, n)
+    a, b = Engine().build_tree(x, m, 0.7), oracle.build_tree(x, m, 0.7)
+    for f in ("start", "count", "next", "leaf", "order", "groups"):
+        assert np.array_equal(a[f], b[f]), f
