@@ -1359,7 +1359,8 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     if (!graph_safe) {
         nn = h_counts->total_nodes;
         // headroom: later synchronisation-free rebuilds (captured or not) build inside it
-        if (nn > node_cap) node_cap = nn + nn / 2 + 1024;
+        // (a tree within an eighth of the capacity would keep asking for regular builds: outgrowing)
+        if (nn > node_cap - node_cap / 8) node_cap = nn + nn / 2 + 1024;
     }
     const int cap = node_cap;
     // node kernels cover [0, span) and read the live count on the device
