@@ -584,7 +584,7 @@ static long long walk_counter(bool quad_only) {
         if (!T || !T->valid) return;
         GF_CUDA(cudaDeviceSynchronize());
         TreeCounts* c = T->counts.as<TreeCounts>();
-        GF_CUDA(cudaMemcpy(&p, quad_only ? &c->qpairs : &c->pairs, sizeof p, cudaMemcpyDeviceToHost));
+        GF_CUDA(cudaMemcpy(&p, quad_only ? &c->w.qpairs : &c->w.pairs, sizeof p, cudaMemcpyDeviceToHost));
     });
     return (long long)p;
 }

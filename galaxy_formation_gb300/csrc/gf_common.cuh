@@ -258,6 +258,16 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
     return old;
 }
 
+// Relaxed loads and stores at GPU scope (look-back statuses).
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(unsigned* p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void raise_status(uint32_t* st, uint32_t bit) {
     if (st) atomicOr(st, bit);
 }

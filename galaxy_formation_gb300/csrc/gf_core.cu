@@ -15,7 +15,7 @@
 #include <algorithm>
 #include <cstring>
 
-#include "gf_common.cuh"
+#include "gf_scan.cuh"
 
 namespace gf {
 
@@ -103,45 +103,7 @@ int collect_status(cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------------------
-// exclusive scan (int32): tile sums -> scan of tile sums -> per-tile scan + offset (up to
-// kScanDirectTiles tiles the last two steps are one launch)
-
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-__device__ __forceinline__ int block_excl_scan(int v, int* s_warp, int* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    int incl = warp_incl_scan(v);
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < nw ? s_warp[lane] : 0;
-        int wi = warp_incl_scan(w);
-        if (lane < nw) s_warp[lane] = wi - w;
-        if (lane == nw - 1) s_warp[32] = wi;
-    }
-    __syncthreads();
-    const int r = incl - v + s_warp[warp];
-    if (total) *total = s_warp[32];
-    __syncthreads();
-    return r;
-}
-
-__global__ void k_scan_tile_sums(const int* __restrict__ in, int n, int* __restrict__ sums) {
-    __shared__ int s_warp[33];
-    const int base = blockIdx.x * kScanTile;
-    int acc = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int i = base + k * kScanThreads + threadIdx.x;
-        if (i < n) acc += in[i];
-    }
-    int tot;
-    block_excl_scan(acc, s_warp, &tot);
-    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
+// exclusive scan (int32; the passes are in gf_scan.cuh)
 
 // single block: exclusive scan of `cnt` tile sums in place, total to *total
 __global__ void k_scan_sums(int* sums, int cnt, int* total) {
@@ -172,73 +134,27 @@ __global__ void k_scan_sums(int* sums, int cnt, int* total) {
     if (threadIdx.x == 0 && total) *total = carry;
 }
 
-__global__ void k_scan_tiles(const int* __restrict__ in, int* __restrict__ out, int n,
-                             const int* __restrict__ offs) {
-    __shared__ int s_warp[33];
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems];
-    int acc = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = (base + k < n) ? in[base + k] : 0;
-        acc += v[k];
-    }
-    int ex = block_excl_scan(acc, s_warp, nullptr) + offs[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) out[base + k] = ex;
-        ex += v[k];
-    }
+void scan_sums(int* sums, int cnt, int* total, cudaStream_t s) {
+    k_scan_sums<<<1, 1024, 0, s>>>(sums, cnt, total);
+    GF_CHECK_LAUNCH();
 }
 
-// Second launch of the two-launch scan: each block adds up the tile sums before its own tile
-// (at most kScanDirectTiles of them: a few KB of L2 reads per block) and scans its tile; the
-// last block writes the total.
-constexpr int kScanDirectTiles = 2048;
-
-__global__ void k_scan_tiles_direct(const int* __restrict__ in, int* __restrict__ out, int n,
-                                    const int* __restrict__ sums, int* __restrict__ total) {
-    __shared__ int s_warp[33];
-    int before = 0;
-    for (int t = threadIdx.x; t < int(blockIdx.x); t += kScanThreads) before += sums[t];
-    int prefix;
-    block_excl_scan(before, s_warp, &prefix);
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems];
-    int acc = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = (base + k < n) ? in[base + k] : 0;
-        acc += v[k];
-    }
-    int tile_total;
-    int ex = block_excl_scan(acc, s_warp, &tile_total) + prefix;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) out[base + k] = ex;
-        ex += v[k];
-    }
-    if (total && threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *total = prefix + tile_total;
+int* scan_scratch(int n, ScanScratch* sc) {
+    return (sc ? sc->scan_tmp : g_ctx.scan_tmp).get<int>(size_t(div_up(std::max(n, 1), kScanTile)) + 1);
 }
+
+namespace {
+struct ArrayScan {
+    const int* in;
+    int* out;
+    __device__ int first(int i) const { return in[i]; }
+    __device__ int again(int i) const { return in[i]; }
+    __device__ void put(int i, int, int ex) const { out[i] = ex; }
+};
+}  // namespace
 
 void exclusive_scan(const int* in, int* out, int n, int* total, cudaStream_t s, ScanScratch* sc) {
-    if (n <= 0) {
-        if (total) GF_CUDA(cudaMemsetAsync(total, 0, sizeof(int), s));
-        return;
-    }
-    const int tiles = div_up(n, kScanTile);
-    int* sums = (sc ? sc->scan_tmp : g_ctx.scan_tmp).get<int>(size_t(tiles) + 1);
-    k_scan_tile_sums<<<tiles, kScanThreads, 0, s>>>(in, n, sums);
-    GF_CHECK_LAUNCH();
-    if (tiles <= kScanDirectTiles) {
-        k_scan_tiles_direct<<<tiles, kScanThreads, 0, s>>>(in, out, n, sums, total);
-        GF_CHECK_LAUNCH();
-        return;
-    }
-    k_scan_sums<<<1, 1024, 0, s>>>(sums, tiles, total);
-    GF_CHECK_LAUNCH();
-    k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(in, out, n, sums);
-    GF_CHECK_LAUNCH();
+    scan_with(ArrayScan{in, out}, n, total, s, sc);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -257,15 +173,6 @@ constexpr unsigned kOsInc = 2u << 30;         // or the inclusive prefix up to t
 constexpr unsigned kOsValue = (1u << 30) - 1;
 constexpr long kOsSpinMax = 1l << 20;         // bounded waits (a waited-on tile is always running)
 constexpr int kOsWindow = 16;                 // look-back statuses loaded at a time
-
-__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed(unsigned* p, unsigned v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // Digit counts of every pass: hist[p * 256 + d] (hist zeroed by the caller).
 __global__ void __launch_bounds__(kRsThreads) k_os_hist(const uint64_t* __restrict__ keys, int n, int bit_lo,
@@ -387,9 +294,8 @@ size_t os_scratch_ints(int n) {
 
 void reserve_scan_sort(int n, ScanScratch* sc) {
     DevBuf& sort_tmp = sc ? sc->sort_tmp : g_ctx.sort_tmp;
-    DevBuf& scan_tmp = sc ? sc->scan_tmp : g_ctx.scan_tmp;
     sort_tmp.get<int>(os_scratch_ints(n));
-    scan_tmp.get<int>(size_t(div_up(std::max(n, 1), kScanTile)) + 1);
+    scan_scratch(n, sc);
 }
 
 void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_alt, int n,

@@ -30,6 +30,7 @@
 
 #include <cooperative_groups.h>
 
+#include "gf_scan.cuh"
 #include "gf_tree.cuh"
 
 namespace gf {
@@ -471,29 +472,38 @@ __device__ __forceinline__ int digit(const KeyView& K, int i, int l) {
     return int((K.k2[i] >> (3 * (48 - l))) & 7);
 }
 
-// cpl9[i] = common prefix of positions i and i + L (L = leaf capacity): a cell holding both
-// holds L + 1 particles and must split
-__global__ void k_cpl9(KeyView K, int n, int8_t* __restrict__ cpl9, TreeCounts* cnt, int L) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int c = -1;
-    if (i + L < n) c = cpl(K, i, i + L);
-    if (c == 21 && !K.k1) cnt->deep = 1;
-    cpl9[i] = int8_t(c);
-}
-
-__global__ void k_nstart(KeyView K, int n, const int8_t* __restrict__ cpl9, int8_t* __restrict__ ldepth,
-                         int8_t* __restrict__ dsplit, int* __restrict__ nstart, int L) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int m = -1;
-    for (int j = max(0, i - L); j <= i; ++j) m = max(m, int(cpl9[j]));
-    const int ld = min(kDepthMax, m + 1);
-    const int ds = i == 0 ? 0 : cpl(K, i - 1, i) + 1;
-    ldepth[i] = int8_t(ld);
-    dsplit[i] = int8_t(min(ds, 127));
-    nstart[i] = max(0, ld - ds + 1);
-}
+// The nodes that start at each sorted position, numbered depth-first. A cell holding positions i and
+// i + L (L = leaf capacity) holds more than L particles and must split, so position i's leaf depth
+// is one more than the longest prefix among the pairs (j, j + L) around it, and the nodes of depths
+// dsplit .. ldepth start at i, dsplit one more than the prefix shared with position i - 1.
+struct StartScan {
+    KeyView K;
+    int n, L;
+    int8_t* ldepth;
+    int8_t* dsplit;
+    int* nbase;    // first node id of each position
+    int* owner;    // position of each node id below cap
+    int cap;
+    TreeCounts* cnt;
+    __device__ int first(int i) const {
+        int m = -1;
+        for (int j = max(0, i - L); j <= i; ++j) {
+            if (j + L >= n) break;
+            const int c = cpl(K, j, j + L);
+            m = max(m, c);
+            if (j == i && c == 21 && !K.k1) cnt->deep = 1;
+        }
+        const int ds = i == 0 ? 0 : cpl(K, i - 1, i) + 1;
+        ldepth[i] = int8_t(min(kDepthMax, m + 1));
+        dsplit[i] = int8_t(min(ds, 127));
+        return again(i);
+    }
+    __device__ int again(int i) const { return max(0, int(ldepth[i]) - int(dsplit[i]) + 1); }
+    __device__ void put(int i, int v, int ex) const {
+        nbase[i] = ex;
+        for (int t = 0; t < v && ex + t < cap; ++t) owner[ex + t] = i;
+    }
+};
 
 // first j > i with j == n or cpl(i, j) < d
 __device__ int run_end(const KeyView& K, int n, int i, int d) {
@@ -557,20 +567,54 @@ __device__ int run_begin(const KeyView& K, int i, int lev) {
 // flag and the parent (the previous node of the chain, or the deepest node at depth d - 1 of
 // the run containing i). Threads of consecutive ids take chains of similar depth, so a warp
 // keeps most lanes busy (one thread per starting position left 5 of 32 busy).
-__global__ void k_node_owner(int n, const int* __restrict__ nstart, const int* __restrict__ nbase,
-                             int* __restrict__ owner, int cap) {
+// A leaf's thread also puts its particles in increasing index order (the reference's stable
+// partitions never reorder a leaf), and the nodes of each depth are counted for the breadth-first
+// numbering.
+__global__ void k_node_owner(int n, StartScan S) {  // after the node buffers have grown
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int c = nstart[i], b = nbase[i];
-    for (int t = 0; t < c && b + t < cap; ++t) owner[b + t] = i;
+    if (i < n) S.put(i, S.again(i), S.nbase[i]);
 }
 
-__global__ void k_emit(KeyView K, int n, int span, const RootBox* __restrict__ rootp,
-                       const int8_t* __restrict__ ldepth, const int8_t* __restrict__ dsplit,
-                       const int* __restrict__ nbase, const int* __restrict__ owner,
-                       const TreeCounts* __restrict__ cnt, int4* __restrict__ n_i4,
-                       double4* __restrict__ n_cd, float4* __restrict__ n_geo,
-                       int* __restrict__ n_parent, int cap) {
+// Particle indices of a leaf into increasing order: up to kLeafMax of them by a sorting network in
+// registers (Batcher's odd-even merge, 19 exchanges); leaves of more than 64 hold identical keys
+// and are sorted already.
+__device__ __forceinline__ void sort_leaf(int* p, int count) {
+    if (count <= kLeafMax) {
+        static_assert(kLeafMax == 8, "a network of 8");
+        int v[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) v[t] = t < count ? p[t] : INT_MAX;
+        constexpr int kA[19] = {0, 2, 4, 6, 0, 1, 4, 5, 1, 5, 0, 1, 2, 3, 2, 3, 1, 3, 5};
+        constexpr int kB[19] = {1, 3, 5, 7, 2, 3, 6, 7, 2, 6, 4, 5, 6, 7, 4, 5, 2, 4, 6};
+#pragma unroll
+        for (int c = 0; c < 19; ++c) {
+            const int a = v[kA[c]], b = v[kB[c]];
+            v[kA[c]] = min(a, b);
+            v[kB[c]] = max(a, b);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            if (t < count) p[t] = v[t];
+        return;
+    }
+    if (count > 64) return;
+    for (int a = 1; a < count; ++a) {
+        const int v = p[a];
+        int b = a - 1;
+        while (b >= 0 && p[b] > v) {
+            p[b + 1] = p[b];
+            --b;
+        }
+        p[b + 1] = v;
+    }
+}
+
+__device__ __forceinline__ void emit_node(KeyView K, int n, int span, const RootBox* __restrict__ rootp,
+                                          const int8_t* __restrict__ ldepth, const int8_t* __restrict__ dsplit,
+                                          const int* __restrict__ nbase, const int* __restrict__ owner,
+                                          const TreeCounts* cnt, int4* __restrict__ n_i4, double4* __restrict__ n_cd,
+                                          float4* __restrict__ n_geo, int* __restrict__ n_parent,
+                                          int* __restrict__ perm, int cap, int* s_depth) {
     const int id = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = cnt->total_nodes;
     if (id >= span || id >= total || id >= cap) return;  // past cap: reported by k_node_cap_check
@@ -602,6 +646,22 @@ __global__ void k_emit(KeyView K, int n, int span, const RootBox* __restrict__ r
     n_cd[id] = make_double4(c[0], c[1], c[2], h);
     n_geo[id] = make_float4(float(c[0]), float(c[1]), float(c[2]), float(h));
     n_parent[id] = parent;
+    atomicAdd(&s_depth[d], 1);
+    if (d == ld) sort_leaf(perm + i, end - i);
+}
+
+__global__ void k_emit(KeyView K, int n, int span, const RootBox* __restrict__ rootp,
+                       const int8_t* __restrict__ ldepth, const int8_t* __restrict__ dsplit,
+                       const int* __restrict__ nbase, const int* __restrict__ owner,
+                       TreeCounts* __restrict__ cnt, int4* __restrict__ n_i4,
+                       double4* __restrict__ n_cd, float4* __restrict__ n_geo,
+                       int* __restrict__ n_parent, int* __restrict__ perm, int cap) {
+    __shared__ int s_depth[kDepthMax + 1];
+    if (threadIdx.x <= kDepthMax) s_depth[threadIdx.x] = 0;
+    __syncthreads();
+    emit_node(K, n, span, rootp, ldepth, dsplit, nbase, owner, cnt, n_i4, n_cd, n_geo, n_parent, perm, cap, s_depth);
+    __syncthreads();
+    if (threadIdx.x <= kDepthMax && s_depth[threadIdx.x]) atomicAdd(&cnt->depth_nodes[threadIdx.x], s_depth[threadIdx.x]);
 }
 
 __global__ void k_node_cap_check(TreeCounts* cnt, int cap, uint32_t* status) {
@@ -614,39 +674,6 @@ __global__ void k_node_cap_check(TreeCounts* cnt, int cap, uint32_t* status) {
 // Node kernels: launched over [0, span); the live node count is *nn_dev.
 __device__ __forceinline__ int live_nodes(int span, const int* nn_dev) {
     return nn_dev ? min(span, *nn_dev) : span;
-}
-
-// Child count of every node; arrival counters to zero.
-__global__ void k_nchild(int span, const int* __restrict__ nn_dev, const int4* __restrict__ n_i4,
-                         int* __restrict__ nchild, int* __restrict__ counter) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= live_nodes(span, nn_dev)) return;
-    const int4 q = n_i4[k];
-    int c = 0;
-    if (!(q.w & 1)) {
-        for (int ch = k + 1; ch < q.z && c < 8; ch = n_i4[ch].z) ++c;  // <= 8 children
-    }
-    nchild[k] = c;
-    counter[k] = 0;
-}
-
-// Inside a leaf the reference keeps increasing particle index (stable partitions).
-__global__ void k_leaf_sort(int span, const int* __restrict__ nn_dev, const int4* __restrict__ n_i4,
-                            int* __restrict__ perm) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= live_nodes(span, nn_dev)) return;
-    const int4 q = n_i4[k];
-    if (!(q.w & 1) || q.y > 64) return;  // larger leaves hold identical keys: already sorted
-    int* p = perm + q.x;
-    for (int a = 1; a < q.y; ++a) {
-        const int v = p[a];
-        int b = a - 1;
-        while (b >= 0 && p[b] > v) {
-            p[b + 1] = p[b];
-            --b;
-        }
-        p[b + 1] = v;
-    }
 }
 
 // Positions (and masses) in tree order: p4 = float32 position and mass, plo = the float32
@@ -1076,41 +1103,122 @@ __global__ void __launch_bounds__(kThreads) k_moments64(Moments64Args A) {
 
 // ---------------------------------------------------------------------------- groups + layout
 
-__global__ void k_group_flag(int span, const int* __restrict__ nn_dev, int gmax, const int4* __restrict__ n_i4,
-                             const int* __restrict__ parent, int* __restrict__ flag) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= span) return;
-    if (k >= live_nodes(span, nn_dev)) {  // past the live nodes: no group (the scan covers span)
-        flag[k] = 0;
-        return;
+// Walk groups: the shallowest nodes holding at most gmax particles, in depth-first order. The same
+// pass counts every node's children and clears its arrival counter.
+struct GroupScan {
+    const int* nn_dev;
+    int span, gmax;
+    const int4* n_i4;
+    const int* parent;
+    int* nchild;
+    int* counter;
+    int* groups;
+    __device__ int first(int k) const {
+        if (k >= live_nodes(span, nn_dev)) return 0;  // past the live nodes (the scan covers span)
+        const int4 q = n_i4[k];
+        int c = 0;
+        if (!(q.w & 1)) {
+            for (int ch = k + 1; ch < q.z && c < 8; ch = n_i4[ch].z) ++c;  // <= 8 children
+        }
+        nchild[k] = c;
+        counter[k] = 0;
+        return again(k);
     }
-    const int4 q = n_i4[k];
-    const bool candidate = q.y <= gmax || (q.w & 1);
-    const int p = parent[k];
-    flag[k] = candidate && (p < 0 || n_i4[p].y > gmax) ? 1 : 0;
-}
+    __device__ int again(int k) const {
+        if (k >= live_nodes(span, nn_dev)) return 0;
+        const int4 q = n_i4[k];
+        const bool candidate = q.y <= gmax || (q.w & 1);
+        const int p = parent[k];
+        return candidate && (p < 0 || n_i4[p].y > gmax) ? 1 : 0;
+    }
+    __device__ void put(int k, int v, int ex) const {
+        if (v) groups[ex] = k;
+    }
+};
 
-__global__ void k_group_write(int span, const int* __restrict__ nn_dev, const int* __restrict__ flag,
-                              const int* __restrict__ scan, int* __restrict__ groups) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= live_nodes(span, nn_dev)) return;
-    if (flag[k]) groups[scan[k]] = k;
-}
+// Breadth-first numbering: a stable counting sort by depth (the nodes per depth are counted by the
+// emission). One sweep like a pass of the radix sort, over kDepthBins digits: tiles in ticket
+// order, a thread per depth adds up the tiles before its own by look-back. bfs[k] = rank of node
+// k, dfs[rank] = k.
+constexpr int kBfsThreads = 256, kBfsItems = 4, kBfsTile = kBfsThreads * kBfsItems;
+constexpr int kBfsWarps = kBfsThreads / 32;
+constexpr int kDepthBins = 64;
+constexpr unsigned kBfsOwn = 1u << 30, kBfsAll = 2u << 30, kBfsValue = (1u << 30) - 1;
+constexpr long kBfsSpinMax = 1l << 20;  // bounded waits (a waited-on tile is always running)
 
-// breadth-first order = stable sort by depth; slots past the live nodes sort last
-__global__ void k_bfs_keys(int span, const int* __restrict__ nn_dev, const int4* __restrict__ n_i4,
-                           uint64_t* __restrict__ key, int* __restrict__ val) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= span) return;
-    key[k] = k < live_nodes(span, nn_dev) ? uint64_t(n_i4[k].w >> 8) : 255u;
-    val[k] = k;
-}
-
-__global__ void k_bfs_index(int span, const int* __restrict__ nn_dev, const int* __restrict__ val,
-                            int* __restrict__ bfs) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= live_nodes(span, nn_dev)) return;
-    bfs[val[b]] = b;
+__global__ void __launch_bounds__(kBfsThreads) k_bfs_rank(int span, TreeCounts* cnt, const int4* __restrict__ n_i4,
+                                                          unsigned* __restrict__ status, int* __restrict__ bfs,
+                                                          int* __restrict__ dfs, uint32_t* err) {
+    __shared__ int s_cnt[kBfsWarps][kDepthBins];
+    __shared__ int s_base[kDepthBins];
+    __shared__ int s_tile;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = lanemask_lt();
+    if (tid == 0) s_tile = atomicAdd(&cnt->bfs_ticket, 1);
+    for (int t = tid; t < kBfsWarps * kDepthBins; t += kBfsThreads) (&s_cnt[0][0])[t] = 0;
+    __syncthreads();
+    const int nodes = live_nodes(span, &cnt->total_nodes);
+    const int tile = s_tile;
+    const int base = tile * kBfsTile + warp * 32 * kBfsItems;
+    if (tile * kBfsTile >= nodes) return;  // nothing here, and no later tile waits for it
+    int d[kBfsItems], rk[kBfsItems];
+#pragma unroll
+    for (int s = 0; s < kBfsItems; ++s) {
+        const int k = base + 32 * s + lane;
+        d[s] = k < nodes ? n_i4[k].w >> 8 : kDepthBins;
+    }
+#pragma unroll
+    for (int s = 0; s < kBfsItems; ++s) {
+        const bool ok = d[s] < kDepthBins;
+        const unsigned peers = __match_any_sync(0xffffffffu, d[s]);
+        const int before = ok ? s_cnt[warp][d[s]] : 0;
+        rk[s] = before + __popc(peers & lt);
+        __syncwarp();
+        if (ok && lane == __ffs(peers) - 1) s_cnt[warp][d[s]] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    if (tid < kDepthBins) {
+        int run = 0;
+        for (int w = 0; w < kBfsWarps; ++w) {
+            const int c = s_cnt[w][tid];
+            s_cnt[w][tid] = run;
+            run += c;
+        }
+        int shallower = 0;  // nodes of smaller depths
+        for (int t = 0; t < tid && t <= kDepthMax; ++t) shallower += cnt->depth_nodes[t];
+        unsigned* mine = status + size_t(tile) * kDepthBins + tid;
+        int excl = 0;
+        if (tile == 0) {
+            st_relaxed(mine, kBfsAll | unsigned(run));
+        } else {
+            st_relaxed(mine, kBfsOwn | unsigned(run));
+            long polls = 0;
+            for (int j = tile - 1; j >= 0;) {
+                const unsigned w = ld_relaxed(status + size_t(j) * kDepthBins + tid);
+                if ((w & ~kBfsValue) == 0u) {  // not there yet
+                    if (++polls < kBfsSpinMax) continue;
+                    raise_status(err, GF_ERR_TIMEOUT);
+                    break;
+                }
+                excl += int(w & kBfsValue);
+                if (w & kBfsAll) break;
+                --j;
+            }
+            st_relaxed(mine, kBfsAll | unsigned(excl + run));
+        }
+        s_base[tid] = shallower + excl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kBfsItems; ++s) {
+        const int k = base + 32 * s + lane;
+        if (k < nodes) {
+            const int b = s_base[d[s]] + s_cnt[warp][d[s]] + rk[s];
+            bfs[k] = b;
+            dfs[b] = k;
+        }
+    }
 }
 
 // The structure of the breadth-first layout (the moments passes write the rest afterwards).
@@ -1254,6 +1362,8 @@ void Octree::reserve_graph_build() {
     sphere.get<float4>(std::max(size_t(node_cap), size_t(n)) + 1);
     if (quad) item_gam.get<float2>(std::max(size_t(node_cap), size_t(n)) + 1);
     gweight.get<int>(std::max(node_cap, 1));
+    gflag.get<int>(std::max(node_cap, 1));
+    gscan.get<int>(std::max(node_cap, 1));
     reserve_scan_sort(std::max(n, node_cap), &scratch);
     deep_sort_attr();
 }
@@ -1315,21 +1425,14 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
         radix_sort_pairs(k0, pm, key_alt.as<uint64_t>(), perm_alt.as<int>(), n, 0, 63, s, &scratch);
     }
 
-    int8_t* c9 = cpl9.get<int8_t>(n);
-    int8_t* ld = ldepth.get<int8_t>(n);
-    int8_t* ds = dsplit.get<int8_t>(n);
-    int* ns = nstart.get<int>(n);
-    KeyView K{k0, nullptr, nullptr};
+    StartScan starts{KeyView{k0, nullptr, nullptr}, n, leaf_max, ldepth.get<int8_t>(n), dsplit.get<int8_t>(n), nb,
+                     node_owner.as<int>(), node_owner.p ? node_cap : 0, cnt};
     // Deep cells (> 8 particles in one level-21 cell) need extension keys. A regular build
     // finds out on the host; a captured one always computes them (zero outside deep runs,
     // where they leave every common-prefix length the tree uses unchanged).
     bool deep = graph_safe;
     if (!graph_safe) {
-        k_cpl9<<<grid, kThreads, 0, s>>>(K, n, c9, cnt, leaf_max);
-        GF_CHECK_LAUNCH();
-        k_nstart<<<grid, kThreads, 0, s>>>(K, n, c9, ld, ds, ns, leaf_max);
-        GF_CHECK_LAUNCH();
-        exclusive_scan(ns, nb, n, &cnt->total_nodes, s, &scratch);
+        scan_with(starts, n, &cnt->total_nodes, s, &scratch);
         GF_CUDA(cudaMemcpyAsync(h_counts, cnt, sizeof(TreeCounts), cudaMemcpyDeviceToHost, s));
         GF_CUDA(cudaStreamSynchronize(s));
         deep = h_counts->deep != 0;
@@ -1337,25 +1440,22 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     if (deep) {
         uint64_t* e1 = key1.get<uint64_t>(n);
         uint64_t* e2 = key2.get<uint64_t>(n);
-        int* starts = reinterpret_cast<int*>(key_alt.get<uint64_t>(n));  // scratch
+        int* run_starts = reinterpret_cast<int*>(key_alt.as<uint64_t>());  // scratch
         int* nst = &cnt->deep_runs;
-        k_deep_keys<<<grid, kThreads, 0, s>>>(n, k0, pm, pos, R, e1, e2, starts, nst, leaf_max);
+        k_deep_keys<<<grid, kThreads, 0, s>>>(n, k0, pm, pos, R, e1, e2, run_starts, nst, leaf_max);
         GF_CHECK_LAUNCH();
         deep_sort_attr();
         const size_t sm = size_t(kDeepRunMax) * (2 * sizeof(uint64_t) + sizeof(int));
-        k_deep_sort<<<2 * C.sms, 512, sm, s>>>(n, k0, e1, e2, pm, starts, nst, C.d_status);
+        k_deep_sort<<<2 * C.sms, 512, sm, s>>>(n, k0, e1, e2, pm, run_starts, nst, C.d_status);
         GF_CHECK_LAUNCH();
-        K = KeyView{k0, e1, e2};
-        k_cpl9<<<grid, kThreads, 0, s>>>(K, n, c9, cnt, leaf_max);
-        GF_CHECK_LAUNCH();
-        k_nstart<<<grid, kThreads, 0, s>>>(K, n, c9, ld, ds, ns, leaf_max);
-        GF_CHECK_LAUNCH();
-        exclusive_scan(ns, nb, n, &cnt->total_nodes, s, &scratch);
+        starts.K = KeyView{k0, e1, e2};
+        scan_with(starts, n, &cnt->total_nodes, s, &scratch);
         if (!graph_safe) {
             GF_CUDA(cudaMemcpyAsync(h_counts, cnt, sizeof(TreeCounts), cudaMemcpyDeviceToHost, s));
             GF_CUDA(cudaStreamSynchronize(s));
         }
     }
+    const KeyView K = starts.K;
     if (!graph_safe) {
         nn = h_counts->total_nodes;
         // headroom: later synchronisation-free rebuilds (captured or not) build inside it
@@ -1375,43 +1475,35 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     {
         ProfScope pse(want_knn ? kStCount : kStTreeEmit, s);
         int* own = node_owner.get<int>(cap);
-        k_node_owner<<<grid, kThreads, 0, s>>>(n, ns, nb, own, cap);
-        GF_CHECK_LAUNCH();
-        k_emit<<<ngrid, kThreads, 0, s>>>(K, n, span, R, ld, ds, nb, own, cnt, i4, cd, geo, par, cap);
+        if (cap > starts.cap) {  // the buffers have grown since the scan
+            starts.owner = own;
+            starts.cap = cap;
+            k_node_owner<<<grid, kThreads, 0, s>>>(n, starts);
+            GF_CHECK_LAUNCH();
+        }
+        k_emit<<<ngrid, kThreads, 0, s>>>(K, n, span, R, starts.ldepth, starts.dsplit, nb, own, cnt, i4, cd, geo, par,
+                                          pm, cap);
         GF_CHECK_LAUNCH();
     }
     if (graph_safe) {  // more nodes than the buffers hold: flag, and leave an empty tree
         k_node_cap_check<<<1, 1, 0, s>>>(cnt, cap, C.d_status);
         GF_CHECK_LAUNCH();
     }
-    int* nch = n_nchild.get<int>(cap);
-    int* ctr = n_counter.get<int>(cap);
-    k_nchild<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, nch, ctr);
-    GF_CHECK_LAUNCH();
-    k_leaf_sort<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, pm);
-    GF_CHECK_LAUNCH();
-
     float4* pp = p4.get<float4>(n);
     double* xb = xbuild.get<double>(3 * size_t(n));
     k_gather<<<grid, kThreads, 0, s>>>(n, pm, pos, mass, nullptr, pp, nullptr,
                                        want_knn ? plo.get<float4>(n) : nullptr, 0, xb);
     GF_CHECK_LAUNCH();
 
-    int* gf_ = gflag.get<int>(cap);
-    int* gs = gscan.get<int>(cap);
-    k_group_flag<<<ngrid, kThreads, 0, s>>>(span, nn_dev, group_max, i4, par, gf_);
-    GF_CHECK_LAUNCH();
-    exclusive_scan(gf_, gs, span, &cnt->num_groups, s, &scratch);
-    k_group_write<<<ngrid, kThreads, 0, s>>>(span, nn_dev, gf_, gs, groups.get<int>(cap));
-    GF_CHECK_LAUNCH();
-
-    uint64_t* bk = bfs_key.get<uint64_t>(cap);
-    int* bv = bfs_val.get<int>(cap);
-    k_bfs_keys<<<ngrid, kThreads, 0, s>>>(span, nn_dev, i4, bk, bv);
-    GF_CHECK_LAUNCH();
-    radix_sort_pairs(bk, bv, bfs_key_alt.get<uint64_t>(cap), bfs_val_alt.get<int>(cap), span, 0, 8, s, &scratch);
+    int* nch = n_nchild.get<int>(cap);
+    scan_with(GroupScan{nn_dev, span, group_max, i4, par, nch, n_counter.get<int>(cap), groups.get<int>(cap)}, span,
+              &cnt->num_groups, s, &scratch);
     int* bfs = n_bfs.get<int>(cap);
-    k_bfs_index<<<ngrid, kThreads, 0, s>>>(span, nn_dev, bv, bfs);
+    const int bfs_tiles = div_up(span, kBfsTile);
+    const size_t status_words = size_t(bfs_tiles) * kDepthBins;
+    unsigned* status = bfs_status.get<unsigned>(size_t(div_up(cap, kBfsTile)) * kDepthBins);
+    GF_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned) * status_words, s));
+    k_bfs_rank<<<bfs_tiles, kBfsThreads, 0, s>>>(span, cnt, i4, status, bfs, bfs_val.get<int>(cap), C.d_status);
     GF_CHECK_LAUNCH();
     k_walk_fill<<<ngrid, kThreads, 0, s>>>(span, i4, nch, bfs, geo, w_b.get<float4>(cap), w_geo.get<float4>(cap),
                                            want_knn ? leaf_of.get<int>(n) : nullptr, par, w_parent.get<int>(cap),

@@ -32,13 +32,17 @@ struct TreeCounts {
     int total_nodes;
     int deep;         // some level-21 cell holds more than kLeafMax particles
     int num_groups;
-    int num_work;
-    int walk_next;    // dynamic scheduler of the walk
     int deep_runs;    // level-21 cells holding more than the leaf capacity (their first positions)
-    int reserved;
     int bbox_done;    // blocks of the bounding-box pass that have written their partials
-    unsigned long long pairs;   // list interactions evaluated by the last walk (all kinds)
-    unsigned long long qpairs;  // of which with quadrupole nodes (mixed form)
+    int bfs_ticket;   // tiles of the breadth-first ranking handed out
+    int depth_nodes[kDepthMax + 1];  // nodes per depth
+    // the walk's counters, cleared together by prepare_walk
+    struct Walk {
+        int num_work;
+        int walk_next;    // dynamic scheduler of the walk
+        unsigned long long pairs;   // list interactions evaluated by the last walk (all kinds)
+        unsigned long long qpairs;  // of which with quadrupole nodes (mixed form)
+    } w;
 };
 
 struct Octree {
@@ -53,7 +57,7 @@ struct Octree {
 
     // particles (tree order unless noted)
     DevBuf key, key_alt, perm, perm_alt, key1, key2, p4, xbuild, pdisp;
-    DevBuf cpl9, ldepth, dsplit, nstart, nbase, node_owner;
+    DevBuf ldepth, dsplit, nbase, node_owner;
     // nodes, depth-first (preorder) order
     DevBuf n_i4;      // int4 {start, count, next, leaf | depth << 8}
     DevBuf n_geo;     // float4 {gx, gy, gz, half}
@@ -70,7 +74,8 @@ struct Octree {
     DevBuf w_q;       // float4 {Qxx, Qyy, Qxy, Qxz} (quadrupole trees)
     DevBuf w_t;       // float2 {Qyz, T = sum m |d|^2 about the centre of mass} (quadrupole trees)
     DevBuf w_rq;      // float (M b^2)^(1/4): the quadrupole-order radius (quadrupole trees)
-    DevBuf bfs_key, bfs_key_alt, bfs_val, bfs_val_alt;
+    DevBuf bfs_val;   // depth-first id of each breadth-first node
+    DevBuf bfs_status;  // look-back statuses of the breadth-first ranking
     // neighbour search extras (tree order): float32 remainders x - float(x) and the
     // breadth-first index of each particle's leaf
     DevBuf plo, leaf_of, w_parent;

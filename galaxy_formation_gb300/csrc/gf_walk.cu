@@ -136,7 +136,7 @@ __device__ __forceinline__ void emit_item(int b, int e, const float4* __restrict
     const ItemStats st = item_stats(b, e, p4, perm, active, aold, alpha, alpha_q);
     if (!st.valid) return;
     int slot = 0;
-    if (lane == 0) slot = atomicAdd(&cnt->num_work, 1);
+    if (lane == 0) slot = atomicAdd(&cnt->w.num_work, 1);
     slot = __shfl_sync(0xffffffffu, slot, 0);
     if (lane == 0) {
         work[slot] = make_int4(b, e - b, st.nact, 0);
@@ -327,7 +327,7 @@ __global__ void k_group_prep(const int* __restrict__ groups, const int4* __restr
                 br2 = warp_max(br2);
                 amin = warp_min(amin);
                 int slot = 0;
-                if (lane == 0) slot = atomicAdd(&cnt->num_work, 1);
+                if (lane == 0) slot = atomicAdd(&cnt->w.num_work, 1);
                 slot = __shfl_sync(0xffffffffu, slot, 0);
                 if (lane == 0) {
                     work[slot] = make_int4(b, q.y, P, r0);
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
     // Tickets go to items through a stride permutation: ticket t -> item (t mod stride) *
     // ceil(nwork / stride) + t / stride, so the warps at work at one time spread over `stride`
     // regions of a work list in tree order, each taken in order (1: the list's own order).
-    const int nwork = cnt->num_work;
+    const int nwork = cnt->w.num_work;
     const int per = (nwork + stride - 1) / stride;
     // SPLIT: two warps share an item of more than 32 particles, 32 each. Both walk it, so the
     // traversal is done twice, but the evaluation, most of a lone warp's time, is halved; every
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
 
     for (;;) {
         int t = 0;
-        if (lane == 0) t = atomicAdd(&cnt->walk_next, 1);
+        if (lane == 0) t = atomicAdd(&cnt->w.walk_next, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= ntick) break;
         const int half = SPLIT && halves > 1 ? t & 1 : 0;
@@ -857,8 +857,8 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
 #undef GF_WALK_FLUSH
         if (lane == 0) {
             const int mine = split ? (half ? P - 32 : 32) : P;
-            atomicAdd(&cnt->pairs, listlen * (unsigned long long)mine);
-            if (QUAD) atomicAdd(&cnt->qpairs, nodelen * (unsigned long long)P);
+            atomicAdd(&cnt->w.pairs, listlen * (unsigned long long)mine);
+            if (QUAD) atomicAdd(&cnt->w.qpairs, nodelen * (unsigned long long)P);
         }
         if constexpr (QUAD) {
             // sum the m entry groups of every particle in a fixed order (the tile is free now)
@@ -922,8 +922,7 @@ void Octree::prepare_walk(const uint8_t* active, cudaStream_t s, int chunk, cons
                           float alpha_q) {
     Context& C = ctx();
     TreeCounts* cnt = counts.as<TreeCounts>();
-    GF_CUDA(cudaMemsetAsync(&cnt->num_work, 0, 2 * sizeof(int), s));  // num_work, walk_next
-    GF_CUDA(cudaMemsetAsync(&cnt->pairs, 0, 2 * sizeof(unsigned long long), s));  // pairs, qpairs
+    GF_CUDA(cudaMemsetAsync(&cnt->w, 0, sizeof cnt->w, s));
     ProfScope ps(kStGroupPrep, s);
     // items: one per group (<= nodes), or at most one per active particle with chunks
     const size_t cap = std::max(size_t(node_cap), size_t(n)) + 1;
@@ -947,7 +946,7 @@ void Octree::prepare_walk(const uint8_t* active, cudaStream_t s, int chunk, cons
         k_item_flag<<<blocks, 256, 0, s>>>(groups.as<int>(), n_i4.as<int4>(), n_parent.as<int>(), gw, cnt, cap_w,
                                            span, fl, C.d_status);
         GF_CHECK_LAUNCH();
-        exclusive_scan(fl, sl, span, &cnt->num_work, s, &scratch);
+        exclusive_scan(fl, sl, span, &cnt->w.num_work, s, &scratch);
         k_item_fill<<<blocks, 256, 0, s>>>(groups.as<int>(), n_i4.as<int4>(), n_parent.as<int>(), gw,
                                            active != nullptr, cnt, cap_w, fl,
                                            sl, p4.as<float4>(), perm.as<int>(), active,
