@@ -165,19 +165,34 @@ __device__ __forceinline__ int pop_round(int* stack, int& sp, int (&node)[NPL]) 
 
 __device__ __forceinline__ unsigned exponent_of(double x) { return unsigned(__double2hiint(x)) >> 20; }
 
-// r and 1/r of r2 >= 0 (1/r capped at 1e30). y, the hardware's
-// approximation, has e = 1 - r2 y^2 of about 2^-20; y (1 - e)^(-1/2) = y (1 + e/2 + 3/8 e^2 + ...).
+// r and 1/r of r2 >= 0 (1/r capped at 1e30). y, the hardware's approximation of 1/sqrt(r2), has
+// e = 1 - r2 y^2 of about 2^-20; the roots are r2 y and y times (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 + ...,
+// each rounded once at the end.
 __device__ __forceinline__ void inv_root(double r2, double& r, double& inv_r) {
     if (exponent_of(r2) - 825u < 1160u) {  // 2^-198 <= r2 < 2^962
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
-        const double e = fma(-(r2 * y), y, 1.0);
-        inv_r = fma(y * e, fma(0.375, e, 0.5), y);
-        r = r2 * inv_r;
+        const double r0 = r2 * y;
+        const double e = fma(-r0, y, 1.0);
+        const double c = e * fma(0.375, e, 0.5);
+        r = fma(r0, c, r0);
+        inv_r = fma(y, c, y);
     } else {
         r = sqrt(r2);
         inv_r = 1.0 / fmax(r, 1e-30);
     }
+}
+
+// The root alone.
+__device__ __forceinline__ double root(double r2) {
+    if (exponent_of(r2) - 123u < 1800u) {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+        const double r0 = r2 * y;
+        const double e = fma(-r0, y, 1.0);
+        return fma(r0, e * fma(0.375, e, 0.5), r0);
+    }
+    return sqrt(r2);
 }
 
 // 1/x of a normal x far from the ends of the range: seed y with e = 1 - x y, y (1 + e + e^2 + ...).

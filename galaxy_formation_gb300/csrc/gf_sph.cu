@@ -77,8 +77,8 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
 // ---- sph_forces in float64 ---------------------------------------------------------------
 //
 // Bound by the float64 pipe (2 lanes per SM and clock on this GPU), so the pair terms are written
-// for few float64 instructions: about 18 in the density pass and 56 in the force pass, against
-// 30 and 100 with a division and a square root per factor.
+// for few float64 instructions: about 17 in the density pass and 49 in the force pass, against
+// 30 and 100 with a division and a square root per factor. (At 500k gas the pipe is 85 % busy.)
 //   * 1/r by a seed and one step of third order, r = r^2 (1/r); 1/x the same way (inv_root,
 //     inverse): the error of the seed cubed is below rounding.
 //   * the kernel's two branches are one polynomial whose coefficients are picked by integer
@@ -88,10 +88,14 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
 // kLanes lanes share a particle's row: without them a lone warp works through 32 neighbours one
 // after another, and small sets leave most of the chip idle.
 
+// The kernel gradient's normalisation -3 / (4 pi h^4) (sph.py:43-54).
+__device__ __forceinline__ double grad_norm(double h) { return -0.75 / (kPi * h * h * h * h); }
+
 // Neighbour data of a pair term. PackedSrc: one 128-byte record per particle, a line per
-// neighbour: {x, y, z, m}, {vx, vy, vz, h/2}, {-3/(4 pi h^4), 1/h, P/rho^2, alpha c/2}, {rho, c}.
+// neighbour: {x, y, z, m}, {vx, vy, vz, h/20}, {s, 1/h, s P/rho^2, 5 alpha c}, {rho, c} with s =
+// -3 / (4 pi h^4).
 struct PairEos {
-    double s4n, inv_h, pr2, ca;
+    double s, inv_h, sp, ca;
 };
 struct alignas(128) SphRec {
     double4_32a xm, vh, eos, rc;
@@ -117,16 +121,16 @@ struct PlainSrc {
     const double* rho_;
     const double* pr2;
     const double* cs;
-    double ha;  // alpha / 2
+    double ha;  // 5 alpha
     __device__ __forceinline__ double4_32a xm(int64_t j) const {
         return double4_32a{pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], mass[j]};
     }
     __device__ __forceinline__ double4_32a vh(int64_t j) const {
-        return double4_32a{vel[3 * j], vel[3 * j + 1], vel[3 * j + 2], 0.5 * h[j]};
+        return double4_32a{vel[3 * j], vel[3 * j + 1], vel[3 * j + 2], 0.05 * h[j]};
     }
     __device__ __forceinline__ PairEos eos(int64_t j) const {
-        const double ih = 1.0 / h[j], ih2 = ih * ih;
-        return PairEos{ih2 * ih2 * (-0.75 / kPi), ih, pr2[j], ha * cs[j]};
+        const double s4 = grad_norm(h[j]);
+        return PairEos{s4, 1.0 / h[j], s4 * pr2[j], ha * cs[j]};
     }
     __device__ __forceinline__ double rho(int64_t j) const { return rho_[j]; }
     __device__ __forceinline__ double sound(int64_t j) const { return cs[j]; }
@@ -165,7 +169,7 @@ __global__ void k_sph_pack(int n, const double* __restrict__ pos, const double* 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     rec[i].xm = double4_32a{pos[3 * size_t(i)], pos[3 * size_t(i) + 1], pos[3 * size_t(i) + 2], mass[i]};
-    rec[i].vh = double4_32a{vel[3 * size_t(i)], vel[3 * size_t(i) + 1], vel[3 * size_t(i) + 2], 0.5 * h[i]};
+    rec[i].vh = double4_32a{vel[3 * size_t(i)], vel[3 * size_t(i) + 1], vel[3 * size_t(i) + 2], 0.05 * h[i]};
 }
 
 // A neighbour row from the caller may hold an index outside [0, n): such a particle gets NaN
@@ -200,8 +204,7 @@ __global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, 
             const double4_32a q = src.xm(j);
             const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            double r = 0.0, inv_r;
-            if (j != i) inv_root(r2, r, inv_r);
+            const double r = j != i ? root(r2) : 0.0;
             sum = fma(q.w, w_shape64(r * inv_h), sum);
         }
     }
@@ -214,8 +217,8 @@ __global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, 
     const double pr = P / (d * d), c = sqrt(gamma * (gamma - 1) * u[i]);
     rho[i] = d;
     if (rec) {
-        const double ih = 1.0 / hi, ih2 = ih * ih;
-        rec[i].eos = double4_32a{ih2 * ih2 * (-0.75 / kPi), ih, pr, ha * c};
+        const double s4 = grad_norm(hi);
+        rec[i].eos = double4_32a{s4, 1.0 / hi, s4 * pr, ha * c};
         rec[i].rc = double4_32a{d, c, 0.0, 0.0};
     } else {
         pr2[i] = pr;
@@ -234,11 +237,16 @@ __global__ void __launch_bounds__(kThreads) k_sph_force(int n, int k, int ld, Sr
     int i = 0;
     const bool on = subset_item(sub, (blockIdx.x * kThreads + threadIdx.x) / kLanes, n, order, i);
     bool ok = true;
-    double ax = 0, ay = 0, az = 0, du = 0, dv = 0, mu_min = 0;
+    // Sums over the row: the acceleration; dw = sum m v.d P_i / r and hv = sum m v.d V / r, which
+    // give du/dt (pressure and viscous part) and the velocity divergence; the most negative mu / 10.
+    // With P the kernel gradient's shape (times s), A = s P/rho^2 and half_visc half the pair's
+    // viscosity: V = half_visc (s_i P_i + s_j P_j), and the pair's force is m (A_i P_i + A_j P_j + V) d / r.
+    double ax = 0, ay = 0, az = 0, dw = 0, hv = 0, mu_min = 0;
+    PairEos ei{0, 0, 0, 0};
     if (on) {
         const double4_32a p = src.xm(i), v = src.vh(i);
-        const PairEos ei = src.eos(i);
-        const double rhoi = src.rho(i);
+        ei = src.eos(i);
+        const double rhoi = src.rho(i), beta100 = 100.0 * beta;
         const Idx* row = nb + size_t(i) * ld;
         for (int jj = s; jj < k; jj += kLanes) {
             const int64_t j = row[jj];
@@ -253,51 +261,54 @@ __global__ void __launch_bounds__(kThreads) k_sph_force(int n, int k, int ld, Sr
             const double r2 = dx * dx + dy * dy + dz * dz;
             double r, inv_r;
             inv_root(r2, r, inv_r);
-            // r times the (1/r) dW/dr of both smoothing lengths
-            const double gi = ei.s4n * dw_shape64(r * ei.inv_h);
-            const double gj = ej.s4n * dw_shape64(r * ej.inv_h);
+            const double Pi = dw_shape64(r * ei.inv_h), Pj = dw_shape64(r * ej.inv_h);
             const double vr = (v.x - w.x) * dx + (v.y - w.y) * dy + (v.z - w.z) * dz;
-            const double pgi = ei.pr2 * gi;
-            double f = fma(ej.pr2, gj, pgi), fu = pgi;
+            const double m = q.w * inv_r, mv = m * vr;
+            double f = fma(ej.sp, Pj, ei.sp * Pi);
+            dw = fma(mv, Pi, dw);
             if (vr < 0) {
-                // mu = hb vr / (r^2 + 0.01 hb^2), visc = (-alpha c mu + beta mu^2) / rho (mean c and rho)
-                const double hb = v.w + w.w, num = hb * vr;
-                const double den = fma(0.01 * hb, hb, r2), rs = rhoi + src.rho(j);
+                // mu = hb vr / (r^2 + 0.01 hb^2), visc = (-alpha c mu + beta mu^2) / rho with the means
+                // hb, c and rho of the pair; hs = 0.1 hb and x = mu / 10 save two products
+                const double hs = v.w + w.w, num = hs * vr;
+                const double den = fma(hs, hs, r2), rs = rhoi + src.rho(j);
                 const double prod = den * rs;
-                double mu, half_visc;
+                double x, xr;  // mu / 10, and that over rs
                 if (exponent_of(prod) - 123u < 1800u) {
-                    const double inv = inverse(prod);
-                    mu = num * (inv * rs);
-                    half_visc = fma(beta, mu, -(ei.ca + ej.ca)) * mu * (inv * den);
+                    xr = num * inverse(prod);
+                    x = xr * rs;
                 } else {
-                    mu = num / den;
-                    half_visc = fma(beta, mu, -(ei.ca + ej.ca)) * mu / rs;
+                    x = num / den;
+                    xr = x / rs;
                 }
-                mu_min = fmin(mu_min, mu);
-                const double vg = half_visc * (gi + gj);
-                f += vg;
-                fu = fma(0.5, vg, fu);
+                const double half_visc = fma(beta100, x, -(ei.ca + ej.ca)) * xr;
+                // of negative numbers the smallest has the largest bits (above those of -inf: NaN)
+                const uint64_t xb = uint64_t(__double_as_longlong(x));
+                if (xb > uint64_t(__double_as_longlong(mu_min)) && xb <= 0xfff0000000000000ull) mu_min = x;
+                const double V = half_visc * fma(ej.s, Pj, ei.s * Pi);
+                f += V;
+                hv = fma(mv, V, hv);
             }
-            const double m = q.w * inv_r, mf = m * f, mv = m * vr;
+            const double mf = m * f;
             ax = fma(-mf, dx, ax);
             ay = fma(-mf, dy, ay);
             az = fma(-mf, dz, az);
-            du = fma(mv, fu, du);
-            dv = fma(mv, gi, dv);
         }
     }
     ax = lanes_sum<kLanes>(ax);
     ay = lanes_sum<kLanes>(ay);
     az = lanes_sum<kLanes>(az);
-    du = lanes_sum<kLanes>(du);
-    if (divv) dv = lanes_sum<kLanes>(dv);
+    dw = lanes_sum<kLanes>(dw);
+    hv = lanes_sum<kLanes>(hv);
+    mu_min *= 10.0;
+    double du = fma(0.5, hv, ei.sp * dw);
+    const double dv = ei.s * dw;
 #pragma unroll
     for (int o = kLanes / 2; o; o >>= 1) mu_min = fmin(mu_min, __shfl_xor_sync(0xffffffffu, mu_min, o));
     if (kLanes > 1) ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
     if (!on || s != 0) return;
     if (!ok) {
         raise_status(status, GF_ERR_ARG);
-        ax = ay = az = du = mu_min = dv = nan64();
+        ax = ay = az = du = nan64();
     }
     acc[3 * size_t(i)] = ax;
     acc[3 * size_t(i) + 1] = ay;
@@ -846,7 +857,7 @@ void sph_launch(int n, int k, int ld, const Src& src, const int* order, const Id
     const int grid = div_up((long long)n * L, kThreads);
     {
         ProfScope ps(kStSphDensity, s);
-        k_sph_density<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 0.5 * alpha, rho, rec,
+        k_sph_density<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 5.0 * alpha, rho, rec,
                                                         pr2, cs, sub, status);
         GF_CHECK_LAUNCH();
     }
@@ -1086,7 +1097,7 @@ extern "C" int gf_sph_forces_noalloc_dev(int n, int k, const double* pos, const 
     double* cs = scratch + kNoallocMaxN;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     try {
-        sph_launch<int64_t, 4>(n, k, k, PlainSrc{pos, vel, mass, h, rho, pr2, cs, 0.5 * alpha}, nullptr, nb, h, u,
+        sph_launch<int64_t, 4>(n, k, k, PlainSrc{pos, vel, mass, h, rho, pr2, cs, 5.0 * alpha}, nullptr, nb, h, u,
                                gamma, alpha, beta, rho, nullptr, pr2, cs, acc, dudt, dt_i, s, nullptr, Subset(),
                                nullptr);
     } catch (const Error& err) {
