@@ -806,12 +806,6 @@ __device__ __forceinline__ float group8_max(float v) {
     return v;
 }
 
-__device__ __forceinline__ double group8_sum(double v) {
-#pragma unroll
-    for (int off = 4; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-
 // The arrival of a finished node at its parent (arrival counter, parent's child count nc, loaded
 // before the atomic). The counter is an acquire-release atomic: it publishes this thread's
 // records of the node and, for the last child, makes its siblings' records visible. Returns
@@ -979,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_refit_bfs_quad32(RefitBfsArgs A
 // Plain form (the reference's arithmetic): monopoles in float64 sums, rounded to the float32 node
 // records (cpp/nbody.cpp:98-131; refit :285-303), in the same bottom-up pass over the breadth-first
 // walk layout. Bound by the float64 pipe and, at small counts, by the chain of arrivals: a leaf's
-// thread sums its particles (7 float64 instructions each), a parent is combined by 8 lanes, one
+// thread sums its particles (4 or 7 float64 instructions each), a parent is combined by 8 lanes, one
 // child each. (One thread climbing per subtree and summing its children one after another kept 9 of
 // 32 lanes active: build passes of 10k / 150k particles 64 / 123 us, now 43 / 77 us; refits of
 // 200k 126 -> 72 us; gravity of the 4M cloud 7.07 -> 6.60 ms.)
@@ -1004,26 +998,24 @@ struct Moments64Args {
     const float* pdisp;
 };
 
-__device__ __forceinline__ void finalize64(const Moments64Args& A, int b, const double4& c, double M, double sx,
-                                           double sy, double sz, float dm) {
-    const double inv = exponent_of(M) - 123u < 1800u ? inverse(M) : M > 0 ? __drcp_rn(M) : 0.0;
-    const double mx = __dmul_rn(sx, inv), my = __dmul_rn(sy, inv), mz = __dmul_rn(sz, inv);
-    A.wa[b] = make_float4(float(mx), float(my), float(mz), float(M));
-    const double ox = __dsub_rn(mx, c.x), oy = __dsub_rn(my, c.y), oz = __dsub_rn(mz, c.z);
+// 1/M of a node's mass (0 for a massless node).
+__device__ __forceinline__ double inverse_mass(double M) {
+    return exponent_of(M) - 123u < 1800u ? inverse(M) : M > 0 ? __drcp_rn(M) : 0.0;
+}
+
+// open_r of a node whose centre of mass lies at squared distance o2 from its cell's centre.
+__device__ __forceinline__ float open_radius(const Moments64Args& A, double half, double o2, float dm) {
     double first;
     if (!A.refit) {
         // 2 half / theta (cpp/nbody.cpp:104-106): half is the root's, halved depth times, so the
         // quotient is the root's scaled by the same power of two (both exponents drop alike)
         const double open0 = A.root->open0;
-        const int drop = __double2hiint(A.root->half) - __double2hiint(c.w);
+        const int drop = __double2hiint(A.root->half) - __double2hiint(half);
         first = __hiloint2double(__double2hiint(open0) - drop, __double2loint(open0));
     } else {  // cpp/nbody.cpp:301-303: the first term is evaluated in float32
-        first = double(__fdiv_rn(__fmul_rn(2.0f, __fadd_rn(float(c.w), dm)), A.theta));
-        A.ndisp[b] = dm;
+        first = double(__fdiv_rn(__fmul_rn(2.0f, __fadd_rn(float(half), dm)), A.theta));
     }
-    double r, inv_r;
-    inv_root(__dadd_rn(__dadd_rn(__dmul_rn(ox, ox), __dmul_rn(oy, oy)), __dmul_rn(oz, oz)), r, inv_r);
-    A.wb[b].x = float(__dadd_rn(first, r));
+    return float(first + root(o2));
 }
 
 // The centre and half of node b's cell, as the pass measures against them.
@@ -1067,37 +1059,67 @@ __global__ void __launch_bounds__(kThreads) k_moments64(Moments64Args A) {
 #pragma unroll
             for (int t = 0; t < kLeafMax; ++t) {
                 if (base + t < -code) {
-                    M = __dadd_rn(M, pm[t].w);
-                    sx = __dadd_rn(sx, __dmul_rn(pm[t].w, pm[t].x));
-                    sy = __dadd_rn(sy, __dmul_rn(pm[t].w, pm[t].y));
-                    sz = __dadd_rn(sz, __dmul_rn(pm[t].w, pm[t].z));
+                    M += pm[t].w;
+                    if (A.refit) {  // (exact products: fused or not, the same sums)
+                        sx = fma(pm[t].w, pm[t].x, sx);
+                        sy = fma(pm[t].w, pm[t].y, sy);
+                        sz = fma(pm[t].w, pm[t].z, sz);
+                    } else {
+                        sx = __dadd_rn(sx, __dmul_rn(pm[t].w, pm[t].x));
+                        sy = __dadd_rn(sy, __dmul_rn(pm[t].w, pm[t].y));
+                        sz = __dadd_rn(sz, __dmul_rn(pm[t].w, pm[t].z));
+                    }
                     dm = fmaxf(dm, pd[t]);
                 }
             }
         }
-        finalize64(A, b, g, M, sx, sy, sz, dm);
+        const double inv = inverse_mass(M);
+        const double mx = sx * inv, my = sy * inv, mz = sz * inv;
+        A.wa[b] = make_float4(float(mx), float(my), float(mz), float(M));
+        const double ox = mx - g.x, oy = my - g.y, oz = mz - g.z;
+        A.wb[b].x = open_radius(A, g.w, fma(ox, ox, fma(oy, oy, oz * oz)), dm);
+        if (A.refit) A.ndisp[b] = dm;
         if (par >= 0 && arrive(&A.counter[par], cr.y)) {
             p = par;
             pc = cr;
         }
     }
     climb_parents(p, pc, A.wparent, A.wb, A.counter, [&](int q, int q0, int qn, int c) {
-        float4 cm = make_float4(0.f, 0.f, 0.f, 0.f);
-        double4 g = make_double4(0.0, 0.0, 0.0, 0.0);
-        float dmc = 0.f;
-        if (q >= 0) {
-            if (c < qn) {
-                cm = __ldcg(&A.wa[q0 + c]);
-                if (A.refit) dmc = __ldcg(&A.ndisp[q0 + c]);
+        // Lane c: quantity c & 3 (0 the mass, 1..3 mass times coordinate) of the children 4 (c >> 2)
+        // .. + 3, so that one instruction serves all four sums (the products of float32 values are
+        // exact in float64: a fused multiply-add rounds as the reference's product and sum).
+        const int quantity = c & 3, k0 = c & 4;
+        const float* w = reinterpret_cast<const float*>(A.wa);
+        float cm[4], cx[4], dm = 0.f;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            cm[t] = cx[t] = 0.f;
+            if (q >= 0 && k0 + t < qn) {
+                const size_t r = 4 * size_t(q0 + k0 + t);
+                cm[t] = __ldcg(w + r + 3);
+                cx[t] = quantity ? __ldcg(w + r + (quantity - 1)) : 1.f;
+                if (A.refit) dm = fmaxf(dm, __ldcg(&A.ndisp[q0 + k0 + t]));
             }
-            if (c == 0) g = cell64(A, q);
         }
-        const double m = double(cm.w);  // (products of float32 values are exact in float64)
-        const double M = group8_sum(m);
-        const double sx = group8_sum(m * double(cm.x)), sy = group8_sum(m * double(cm.y)),
-                     sz = group8_sum(m * double(cm.z));
-        const float dm = A.refit ? group8_max(dmc) : 0.f;
-        if (q >= 0 && c == 0) finalize64(A, q, g, M, sx, sy, sz, dm);
+        double4 g = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (q >= 0) g = cell64(A, q);
+        double s = 0.0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) s = fma(double(cm[t]), double(cx[t]), s);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, 4));
+        const double M = __shfl_sync(0xffffffffu, s, 0, 8);
+        const double com = s * inverse_mass(M);  // lanes 1..3
+        const double o = com - (quantity == 1 ? g.x : quantity == 2 ? g.y : g.z);
+        const double oo = o * o;
+        const double o2 = __shfl_sync(0xffffffffu, oo, 1, 8) + __shfl_sync(0xffffffffu, oo, 2, 8) +
+                          __shfl_sync(0xffffffffu, oo, 3, 8);
+        if (q >= 0 && c < 4) reinterpret_cast<float*>(A.wa)[4 * size_t(q) + (c ? c - 1 : 3)] = float(c ? com : M);
+        if (q >= 0 && c == 0) {
+            A.wb[q].x = open_radius(A, g.w, o2, dm);
+            if (A.refit) A.ndisp[q] = dm;
+        }
+        __syncwarp();  // the group's writes before its lane 0 arrives at the grandparent
     });
 }
 
