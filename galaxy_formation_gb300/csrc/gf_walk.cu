@@ -360,6 +360,7 @@ struct WarpSmem {
     float4 ntQ[kNodeTile];   // Qxx, Qyy, Qxy, Qxz
     float2 ntYZ[kNodeTile];  // Qyz, T
     int seg[32];  // opened leaves of a slot row: first particle minus first slot
+    int nodes[NPL > 2 ? 32 * NPL : 1];  // wide rounds: each lane's nodes
     int slot_pos[kBatch];
 };
 
@@ -580,12 +581,12 @@ __device__ __forceinline__ void eval_quad(const float4* tile, const float4* ntA,
 
 // POT (monopole form only): also the softened potential of every walked particle, into pot.
 // Blocks per SM: shared memory allows 4 of the mixed form's and 6 of the reference form's;
-// 5 keeps the latter free of register spills; the wide-round variant needs more registers.
+// 5 keeps the latter free of register spills.
 // WARPS (block shape) and SMALL (tile size) are the mixed walk's tunable launch shape: the
 // register bound keeps 16 warps per SM whatever the block shape.
 template <bool QUAD, bool POT = false, int NPL = (QUAD ? 2 : 1), int WARPS = kWalkWarps, bool SMALL = false,
           bool NORMAL = true, bool SPLIT = false>
-__global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) : (SPLIT ? 4 : 5)) k_walk(
+__global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 4 : 16 / WARPS) : (SPLIT ? 4 : 5)) k_walk(
     const float4* __restrict__ wa, const float4* __restrict__ wb, const float4* __restrict__ wq,
     const float2* __restrict__ wt, const float* __restrict__ wrq, const float4* __restrict__ p4,
     const int* __restrict__ perm, const uint8_t* __restrict__ active, const int4* __restrict__ work,
@@ -728,30 +729,24 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             int nodes[kNodesPerLane];
             const int nnodes = pop_round<kNodesPerLane>(S.stack, sp, nodes);
             __syncwarp();
-            float4 As[kNodesPerLane], Bs[kNodesPerLane];
-            float RQs[kNodesPerLane];
-#pragma unroll
-            for (int i = 0; i < kNodesPerLane; ++i) {
-                As[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                Bs[i] = As[i];
-                RQs[i] = 0.f;
-                if (nodes[i] >= 0) {
-                    As[i] = wa[nodes[i]];
-                    Bs[i] = wb[nodes[i]];
-                    if (QUAD && gq > 0.f) RQs[i] = wrq[nodes[i]];
+            auto load_node = [&](int node, float4& A, float4& B, float& RQ) {
+                A = make_float4(0.f, 0.f, 0.f, 0.f);
+                B = A;
+                RQ = 0.f;
+                if (node >= 0) {
+                    A = wa[node];
+                    B = wb[node];
+                    if (QUAD && gq > 0.f) RQ = wrq[node];
                 }
-            }
-#pragma unroll
-            for (int i = 0; i < kNodesPerLane; ++i) {
-            if (32 * i >= nnodes) break;  // warp-uniform
-            const int node = nodes[i];
+            };
+            // one row of slots: 32 nodes tested, opened nodes pushed, list entries appended
+            auto do_row = [&](int node, const float4& A, const float4& B, float RQ) {
             const bool valid = node >= 0;
-            const float4 A = As[i], B = Bs[i];
             const float dx = A.x - sph.x, dy = A.y - sph.y, dz = A.z - sph.z;
             const float t = (QUAD ? fmaxf(B.x, B.w * gm) : B.x) + sph.w;
             const float dd2 = dx * dx + dy * dy + dz * dz;
             const bool accept = valid && (dd2 > t * t);
-            const float tq = RQs[i] * gq + sph.w;
+            const float tq = RQ * gq + sph.w;
             const bool mono = QUAD && accept && gq > 0.f && dd2 > tq * tq;  // quadrupole below alpha_q a_min
             const int first = __float_as_int(B.y), code = __float_as_int(B.z);
             const bool leaf = valid && !accept && code < 0;
@@ -788,7 +783,7 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             const int npush = __popc(om);
             if (sp + npush > Smem::kStack) {
                 overflow = true;
-                break;
+                return;
             }
             if (open) S.stack[sp + __popc(om & lt)] = (first << 4) | code;
             sp += npush;
@@ -846,7 +841,40 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 1 : 16 / WARPS) 
             }
             }  // any leaf
             __syncwarp();
-            }  // nodes of the lane
+            };
+            if constexpr (NPL > 2) {
+                // a loop of one row's code with the next row's records in flight: unrolled, the
+                // rows' copies of the evaluation overflowed the instruction cache (a warp waited
+                // for instructions 7 to 11 cycles per issue): two blocks of steps at 200k 33.9 -> 21.9 ms
+#pragma unroll
+                for (int i = 0; i < kNodesPerLane; ++i) S.nodes[32 * i + lane] = nodes[i];
+                float4 A, B;
+                float RQ;
+                int node = S.nodes[lane];
+                load_node(node, A, B, RQ);
+#pragma unroll 1
+                for (int i = 0; 32 * i < nnodes && !overflow; ++i) {
+                    float4 An, Bn;
+                    float RQn;
+                    const int next = 32 * (i + 1) < nnodes ? S.nodes[32 * (i + 1) + lane] : -1;
+                    load_node(next, An, Bn, RQn);
+                    do_row(node, A, B, RQ);
+                    node = next;
+                    A = An;
+                    B = Bn;
+                    RQ = RQn;
+                }
+            } else {
+                float4 As[kNodesPerLane], Bs[kNodesPerLane];
+                float RQs[kNodesPerLane];
+#pragma unroll
+                for (int i = 0; i < kNodesPerLane; ++i) load_node(nodes[i], As[i], Bs[i], RQs[i]);
+#pragma unroll
+                for (int i = 0; i < kNodesPerLane; ++i) {
+                    if (32 * i >= nnodes || overflow) break;  // warp-uniform
+                    do_row(nodes[i], As[i], Bs[i], RQs[i]);
+                }
+            }
             if (overflow) break;
         }
         if (overflow) {
