@@ -21,6 +21,7 @@
 //                              in float64 and sorted again, so the result is the exact
 //                              float64 kNN.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -90,6 +91,10 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
 
 // The kernel gradient's normalisation -3 / (4 pi h^4) (sph.py:43-54).
 __device__ __forceinline__ double grad_norm(double h) { return -0.75 / (kPi * h * h * h * h); }
+
+// Threads per block: small blocks even out the last wave of the small launches.
+template <int kLanes>
+constexpr int kSphThreads = kLanes >= 4 ? 64 : 128;
 
 // Neighbour data of a pair term. PackedSrc: one 128-byte record per particle, a line per
 // neighbour: {x, y, z, m}, {vx, vy, vz, h/20}, {s, 1/h, s P/rho^2, 5 alpha c}, {rho, c} with s =
@@ -179,14 +184,14 @@ __global__ void k_sph_pack(int n, const double* __restrict__ pos, const double* 
 // equation of state of the particle (the per-j factors of sph.py:88-89), into its record
 // (PackedSrc) or pr2 / cs.
 template <class Idx, int kLanes, class Src>
-__global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, Src src, const int* __restrict__ order,
+__global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_density(int n, int k, int ld, Src src, const int* __restrict__ order,
                                                           const Idx* __restrict__ nb, const double* __restrict__ h,
                                                           const double* __restrict__ u, double gamma, double ha,
                                                           double* __restrict__ rho, SphRec* rec, double* pr2,
                                                           double* cs, Subset sub, uint32_t* status) {
     const int s = threadIdx.x % kLanes;
     int i = 0;
-    const bool on = subset_item(sub, (blockIdx.x * kThreads + threadIdx.x) / kLanes, n, order, i);
+    const bool on = subset_item(sub, (blockIdx.x * kSphThreads<kLanes> + threadIdx.x) / kLanes, n, order, i);
     bool ok = true;
     double sum = 0.0, hi = 1.0;
     if (on) {
@@ -209,8 +214,27 @@ __global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, 
         }
     }
     sum = lanes_sum<kLanes>(sum);
-    if (kLanes > 1) ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
-    if (!on || s != 0) return;
+    if (kLanes > 1) {
+        ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
+        // the rest is a few divisions per particle: by full warps of one particle per thread (at four
+        // lanes per particle it took a third of the pass)
+        __shared__ double s_sum[kSphThreads<kLanes> / kLanes];
+        __shared__ int s_i[kSphThreads<kLanes> / kLanes];  // INT_MIN: none; ~i: a bad row
+        if (s == 0) {
+            s_sum[threadIdx.x / kLanes] = sum;
+            s_i[threadIdx.x / kLanes] = !on ? INT_MIN : ok ? i : ~i;
+        }
+        __syncthreads();
+        if (threadIdx.x >= kSphThreads<kLanes> / kLanes) return;
+        i = s_i[threadIdx.x];
+        if (i == INT_MIN) return;
+        ok = i >= 0;
+        if (!ok) i = ~i;
+        sum = s_sum[threadIdx.x];
+        hi = h[i];
+    } else if (!on) {
+        return;
+    }
     if (!ok) raise_status(status, GF_ERR_ARG);
     const double d = !ok ? nan64() : sum == 0.0 ? 0.0 : sum * (1.0 / (kPi * hi * hi * hi));
     const double P = (gamma - 1) * d * u[i];
@@ -228,14 +252,14 @@ __global__ void __launch_bounds__(kThreads) k_sph_density(int n, int k, int ld, 
 
 // pass 2 (sph.py:72-106)
 template <class Idx, int kLanes, class Src>
-__global__ void __launch_bounds__(kThreads) k_sph_force(int n, int k, int ld, Src src, const int* __restrict__ order,
+__global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k, int ld, Src src, const int* __restrict__ order,
                                                         const Idx* __restrict__ nb, const double* __restrict__ h,
                                                         double alpha, double beta, double* __restrict__ acc,
                                                         double* __restrict__ dudt, double* __restrict__ dt_i,
                                                         float* __restrict__ divv, Subset sub, uint32_t* status) {
     const int s = threadIdx.x % kLanes;
     int i = 0;
-    const bool on = subset_item(sub, (blockIdx.x * kThreads + threadIdx.x) / kLanes, n, order, i);
+    const bool on = subset_item(sub, (blockIdx.x * kSphThreads<kLanes> + threadIdx.x) / kLanes, n, order, i);
     bool ok = true;
     // Sums over the row: the acceleration; dw = sum m v.d P_i / r and hv = sum m v.d V / r, which
     // give du/dt (pressure and viscous part) and the velocity divergence; the most negative mu / 10.
@@ -854,26 +878,28 @@ void sph_launch(int n, int k, int ld, const Src& src, const int* order, const Id
                 const double* u, double gamma, double alpha, double beta, double* rho, SphRec* rec, double* pr2,
                 double* cs, double* acc, double* dudt, double* dt_i, cudaStream_t s, float* divv, Subset sub,
                 uint32_t* status) {
-    const int grid = div_up((long long)n * L, kThreads);
+    constexpr int threads = kSphThreads<L>;
+    const int grid = div_up((long long)n * L, threads);
     {
         ProfScope ps(kStSphDensity, s);
-        k_sph_density<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 5.0 * alpha, rho, rec,
+        k_sph_density<Idx, L><<<grid, threads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 5.0 * alpha, rho, rec,
                                                         pr2, cs, sub, status);
         GF_CHECK_LAUNCH();
     }
     ProfScope ps(kStSphForce, s);
-    k_sph_force<Idx, L><<<grid, kThreads, 0, s>>>(n, k, ld, src, order, nb, h, alpha, beta, acc, dudt, dt_i, divv,
+    k_sph_force<Idx, L><<<grid, threads, 0, s>>>(n, k, ld, src, order, nb, h, alpha, beta, acc, dudt, dt_i, divv,
                                                   sub, status);
     GF_CHECK_LAUNCH();
 }
 
 // Lanes per particle by the particles of a launch: one thread each fills the chip (and needs no
-// reduction) from some hundred thousand on; below, and for the few particles due in a subset of
-// unknown size, four shorten the chain of neighbours. Density + force, measured with 1 / 2 / 4 / 8
-// lanes: 5k gas 204 / 124 / 70 / 74 us (329 us with a division and a square root per factor and a
-// thread per particle); 150k 928 / 892 / 939 / 1032 us (1361); 500k 2365 / 3024 / 2671 / 3010 us
-// (4141).
-constexpr int kSphFourLanes = 128 * 1024, kSphTwoLanes = 256 * 1024;
+// reduction) from some hundred thousand on; below, more lanes shorten the chain of neighbours, and a
+// subset of unknown size takes four. Density + force in us with 1 / 2 / 4 / 8 lanes (before: a thread
+// per particle with a division and a square root per factor):
+//     5k gas   118 /   70 /   47 /   45   (329)        150k    718 /  673 /  698 /  785   (1361)
+//    20k       171 /  135 /  115 /  123                250k   1140 / 1134 / 1199 / 1356
+//   100k       534 /  476 /  472 /  534                500k   2048 / 2135 / 2262 / 2573   (4141)
+constexpr int kSphEightLanes = 8 * 1024, kSphFourLanes = 128 * 1024, kSphTwoLanes = 256 * 1024;
 
 template <class Idx>
 void sph_forces(SphScratch& S, int n, int k, int ld, const int* order, const double* pos, const double* vel,
@@ -888,7 +914,9 @@ void sph_forces(SphScratch& S, int n, int k, int ld, const int* order, const dou
         sph_launch<Idx, decltype(lanes)::value>(n, k, ld, PackedSrc{rec}, order, nb, h, u, gamma, alpha, beta, rho,
                                                 rec, nullptr, nullptr, acc, dudt, dt_i, s, divv, sub, ctx().d_status);
     };
-    if (sub.idx || n <= kSphFourLanes)
+    if (!sub.idx && n <= kSphEightLanes)
+        go(std::integral_constant<int, 8>());
+    else if (sub.idx || n <= kSphFourLanes)
         go(std::integral_constant<int, 4>());
     else if (n <= kSphTwoLanes)
         go(std::integral_constant<int, 2>());

@@ -1,6 +1,6 @@
 """The float64 SPH passes at the edges of their launch rule and of their pair arithmetic.
 
-Particle counts on both sides of the switches between four, two and one lanes per particle, rows
+Particle counts on both sides of the switches between eight, four, two and one lanes per particle, rows
 of 1 to 33 neighbours (not a multiple of the lanes), coincident particles, pairs outside both
 supports, and sets scaled so far that the squared distances leave the range of the fast inverse
 root. Against NumPy's float64 restatement of sph.py:57-106. A pair term takes fewer than 60
@@ -61,7 +61,8 @@ def _reference(x, v, m, nb, h, u, gamma=5.0 / 3.0, alpha=1.0, beta=2.0):
 
 
 @pytest.mark.parametrize("n,k,scale", [(3, 1, 1.0), (257, 5, 1.0), (4001, 33, 1.0), (4001, 32, 1e-38),
-                                       (4001, 32, 1e30), (128 * 1024, 8, 1.0), (128 * 1024 + 1, 7, 1.0),
+                                       (4001, 32, 1e30), (8 * 1024, 19, 1.0),
+                                       (8 * 1024 + 1, 21, 1.0), (128 * 1024, 8, 1.0), (128 * 1024 + 1, 7, 1.0),
                                        (256 * 1024, 6, 1.0), (256 * 1024 + 1, 5, 1.0)])
 def test_sph_forces_lanes(gpulib, n, k, scale):
     from galaxy_formation_gb300 import sph
