@@ -4,12 +4,12 @@
 // per digit (the single-pass scheme of Adinets & Merrill, "Onesweep", 2022):
 //   histogram  one launch reads the keys once and counts the digits of every pass,
 //   pass       one launch per digit: each block takes the next tile by ticket, ranks its keys
-//              stably (__match_any_sync per warp, warps in key order), publishes its digit
+//              stably (ballots of the digit per warp, warps in key order), publishes its digit
 //              counts, adds up the counts of the tiles before it by decoupled look-back (a
 //              tile's flag says whether its value is its own count or the inclusive prefix;
 //              waits are bounded, GF_ERR_TIMEOUT past the bound) and scatters each key to
 //              (keys of smaller digits) + (its digit in earlier tiles) + its rank.
-// Tiles are 2048 keys (256 threads x 8). Traffic per pass: 12 B read + 12 B write per pair,
+// Tiles are 1024 or 2048 keys (256 threads x 4 or 8). Traffic per pass: 12 B read + 12 B write per pair,
 // plus 8 B per pair once for the histogram.
 #include <cstdarg>
 #include <algorithm>
@@ -164,9 +164,11 @@ constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
 // --- one sweep per digit --------------------------------------------------------------------
 
-constexpr int kOsItems = 8;                   // keys per thread
-constexpr int kOsWarpItems = 32 * kOsItems;   // consecutive keys per warp
-constexpr int kOsTile = kRsThreads * kOsItems;
+// Keys per thread: 8, or 4 up to kOsFewKeys keys, where a tile's own latency counts and tiles of
+// 2048 would leave SMs idle. Eight passes with 4 / 8 / 16 per thread: 60k keys 76 / 88 / 115 us, 100k
+// 76 / 93 / 122, 200k 104 / 92 / 125, 1M 252 / 208 / 199, 4M 742 / 572 / 613.
+constexpr int kOsMinItems = 4;
+constexpr int kOsFewKeys = 144 * 1024;
 constexpr int kOsMaxPasses = 8;
 constexpr unsigned kOsAgg = 1u << 30;         // look-back flags: the tile's own count,
 constexpr unsigned kOsInc = 2u << 30;         // or the inclusive prefix up to the tile
@@ -189,7 +191,20 @@ __global__ void __launch_bounds__(kRsThreads) k_os_hist(const uint64_t* __restri
         if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
+// Lanes whose digit d (0..255) equals this lane's, among the lanes with ok: by the ballots of its
+// eight bits (match.any instead: 8 % slower sorts at 1M keys, its latency is the longer one).
+__device__ __forceinline__ unsigned digit_peers(unsigned d, bool ok) {
+    unsigned peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const unsigned ones = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? ones : ~ones;
+    }
+    return peers;
+}
+
 // One pass: tiles in ticket order; status[tile * 256 + d] holds the flag and value of digit d.
+template <int kOsItems>
 __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     const uint64_t* __restrict__ kin, const int* __restrict__ vin, uint64_t* __restrict__ kout,
     int* __restrict__ vout, int n, int shift, const int* __restrict__ tot, unsigned* __restrict__ status,
@@ -198,6 +213,8 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     __shared__ int s_base[256];
     __shared__ int s_warp[33];
     __shared__ int s_tile;
+    constexpr int kOsWarpItems = 32 * kOsItems;  // consecutive keys per warp
+    constexpr int kOsTile = kRsThreads * kOsItems;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
     for (int w = 0; w < kRsWarps; ++w) s_cnt[w][threadIdx.x] = 0;
@@ -221,7 +238,7 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
         const int i = base + s * 32 + lane;
         const bool ok = i < n;
         const unsigned d = ok ? unsigned((k[s] >> shift) & 255u) : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned peers = digit_peers(d, ok);
         const int before = ok ? s_cnt[warp][d] : 0;
         rank[s] = before + __popc(peers & lt);
         __syncwarp();
@@ -288,7 +305,7 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
 // Scratch of a one-sweep sort of n pairs: digit totals [8][256], tickets [8], tile status
 // [8][tiles][256].
 size_t os_scratch_ints(int n) {
-    const size_t tiles = size_t(div_up(std::max(n, 1), kOsTile));
+    const size_t tiles = size_t(div_up(std::max(n, 1), kRsThreads * kOsMinItems));
     return size_t(kOsMaxPasses) * 256 + 64 + size_t(kOsMaxPasses) * tiles * 256;
 }
 
@@ -304,7 +321,8 @@ void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_a
     if (n > int(kOsValue)) throw Error(GF_ERR_CAPACITY, "radix sort of more than 2^30 - 1 keys");
     const int npass = div_up(bit_hi - bit_lo, 8);
     if (npass < 1 || npass > kOsMaxPasses) throw Error(GF_ERR_ARG, "radix sort bit range");
-    const int tiles = div_up(n, kOsTile);
+    const int items = n <= kOsFewKeys ? kOsMinItems : 8;
+    const int tiles = div_up(n, kRsThreads * items);
     int* hist = (sc ? sc->sort_tmp : g_ctx.sort_tmp).get<int>(os_scratch_ints(n));
     int* tickets = hist + kOsMaxPasses * 256;
     unsigned* status = reinterpret_cast<unsigned*>(tickets + 64);
@@ -316,8 +334,14 @@ void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_a
     uint64_t *ka = keys, *kb = keys_alt;
     int *va = vals, *vb = vals_alt;
     for (int p = 0; p < npass; ++p) {
-        k_os_pass<<<tiles, kRsThreads, 0, s>>>(ka, va, kb, vb, n, bit_lo + 8 * p, hist + 256 * p,
-                                               status + size_t(p) * tiles * 256, tickets + p, g_ctx.d_status);
+        auto pass = [&](auto kernel) {
+            kernel<<<tiles, kRsThreads, 0, s>>>(ka, va, kb, vb, n, bit_lo + 8 * p, hist + 256 * p,
+                                                status + size_t(p) * tiles * 256, tickets + p, g_ctx.d_status);
+        };
+        if (items == kOsMinItems)
+            pass(k_os_pass<kOsMinItems>);
+        else
+            pass(k_os_pass<8>);
         GF_CHECK_LAUNCH();
         std::swap(ka, kb);
         std::swap(va, vb);

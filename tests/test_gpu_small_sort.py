@@ -1,8 +1,8 @@
 """The one-launch bounding box, keys and sort of small sets: the tree equals the oracle's node for
 node (structure, particle order) at the edges of the split over the cluster's blocks (fewer
 particles than blocks, empty last blocks, uneven shares) and of the launch rules (28,672 particles
-and one more; 32,768 and one more for the scans that number nodes and groups), with coincident
-points, points on cell walls and cells deeper than a key."""
+and one more; 32,768 and one more for the scans that number nodes and groups; 147,456 and one more
+for the keys per thread of the larger sorts), with coincident points, points on cell walls and cells deeper than a key."""
 
 import numpy as np
 import pytest
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 17, 63, 1023, 8191, 8193, 10000, 28671, 28672, 28673,
-                               32768, 32769])
+                               32768, 32769, 144 * 1024, 144 * 1024 + 1])
 @pytest.mark.parametrize("kind", ["normal", "grid", "deep"])
 def test_small_sort_builds_the_same_tree(gpulib, oracle, n, kind):
     from galaxy_formation_gb300.engine import Engine
