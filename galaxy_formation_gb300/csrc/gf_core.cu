@@ -191,18 +191,6 @@ __global__ void __launch_bounds__(kRsThreads) k_os_hist(const uint64_t* __restri
         if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-// Lanes whose digit d (0..255) equals this lane's, among the lanes with ok: by the ballots of its
-// eight bits (match.any instead: 8 % slower sorts at 1M keys, its latency is the longer one).
-__device__ __forceinline__ unsigned digit_peers(unsigned d, bool ok) {
-    unsigned peers = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-        const unsigned ones = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-        peers &= (d >> b) & 1u ? ones : ~ones;
-    }
-    return peers;
-}
-
 // One pass: tiles in ticket order; status[tile * 256 + d] holds the flag and value of digit d.
 template <int kOsItems>
 __global__ void __launch_bounds__(kRsThreads) k_os_pass(

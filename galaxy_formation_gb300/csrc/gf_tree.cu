@@ -366,8 +366,8 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
             const int o = wbase + 32 * s + lane;
             const bool ok = o < own;
             k[s] = ok ? ki[o] : 0ull;
-            const unsigned d = ok ? unsigned(k[s] >> shift) & 255u : 256u;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const unsigned d = unsigned(k[s] >> shift) & 255u;
+            const unsigned peers = digit_peers(d, ok);
             const int before = ok ? cnt[warp * 256 + d] : 0;
             rk[s] = before + __popc(peers & lt);
             __syncwarp();
