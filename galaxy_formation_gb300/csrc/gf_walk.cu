@@ -744,9 +744,12 @@ __global__ void __launch_bounds__(WARPS * 32, QUAD ? (NPL > 2 ? 4 : 16 / WARPS) 
             const bool valid = node >= 0;
             const float dx = A.x - sph.x, dy = A.y - sph.y, dz = A.z - sph.z;
             const float t = (QUAD ? fmaxf(B.x, B.w * gm) : B.x) + sph.w;
-            const float dd2 = dx * dx + dy * dy + dz * dz;
+            // |d|^2 with its multiply-adds spelled out, for each form the ones it has always used: left
+            // to the compiler, an instantiation could contract the sum the other way and take a node
+            // whose distance lies within a rounding of its opening radius differently
+            const float dd2 = QUAD ? fmaf(dz, dz, fmaf(dx, dx, dy * dy)) : fmaf(dz, dz, fmaf(dy, dy, dx * dx));
             const bool accept = valid && (dd2 > t * t);
-            const float tq = RQ * gq + sph.w;
+            const float tq = fmaf(RQ, gq, sph.w);
             const bool mono = QUAD && accept && gq > 0.f && dd2 > tq * tq;  // quadrupole below alpha_q a_min
             const int first = __float_as_int(B.y), code = __float_as_int(B.z);
             const bool leaf = valid && !accept && code < 0;

@@ -48,3 +48,28 @@ def test_shared_items(gpulib, oracle, eps, active, sizes, coincident):
         assert np.array_equal(acc[act == 0], ref[act == 0])  # other rows untouched
     if np.any(on):
         assert np.percentile(rel_err(acc[on], ref[on]), 99) < 1e-4
+
+
+def test_every_launch_shape_walks_the_same_lists(gpulib):
+    """The mixed walk's launch shapes test each node with the same arithmetic: the number of list
+    interactions, quadrupole nodes among them, is the same to the last one."""
+    from galaxy_formation_gb300 import _lib, params, synthetic
+
+    lib = gpulib
+    d = synthetic.make_config(1, scale=0.3)
+    n = len(d["mass"])
+    acc, dt = np.empty((n, 3)), np.empty(n)
+    lib.gf_set_option(_lib.OPT_GRAVITY_QUAD, 1)
+    lib.gf_set_option(_lib.OPT_GRAVITY_REL, 0)
+    lib.gf_set_option(_lib.OPT_WALK_MERGE, 40)
+    pairs = []
+    try:
+        for shape in range(4):
+            lib.gf_set_option(_lib.OPT_WALK_SHAPE, shape)
+            _lib.check(lib.gf_accelerations(n, d["pos"], d["vel"], d["mass"], d["kind"], d["u"], 0.55, params.EPS,
+                                            params.GAMMA, 1.0, 2.0, None, 1, 0, 0, acc, dt))
+            pairs.append((lib.gf_walk_pairs(), lib.gf_walk_quad_pairs()))
+    finally:
+        for key in (_lib.OPT_GRAVITY_QUAD, _lib.OPT_WALK_MERGE, _lib.OPT_WALK_SHAPE):
+            lib.gf_set_option(key, 0)
+    assert pairs[0][0] > 0 and len(set(pairs)) == 1, pairs
