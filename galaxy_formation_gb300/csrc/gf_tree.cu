@@ -251,15 +251,15 @@ __global__ void k_keys(const double* __restrict__ pos, int n, const RootBox* __r
 // histogram and a look-back. A pass costs about 12,000 cycles at 10k keys, half of it barriers and
 // their latencies, and grows with the keys per block (match-any, scattered remote stores), so the
 // chain of 12 launches is as fast from about 28k keys on: Engine.gravity with the chain / with this
-// launch 325 / 267 us at 5k particles, 350 / 302 at 10k, 366 / 354 at 24k, 375 / 381 at 32k.
+// launch 325 / 267 us at 5k particles, 350 / 302 at 10k, 366 / 354 at 24k, 375 / 381 at 32k (blocks of
+// 512 threads instead of 1024, whose barriers are longer: 2 % faster builds).
 static_assert(kKeyLevels == 21, "eight 8-bit passes over a 63-bit key");
 constexpr int kSmallCtas = 8;
-constexpr int kSmallThreads = 1024;
+constexpr int kSmallThreads = 512;
 constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr int kSmallItems = 4;                             // keys per thread at most
+constexpr int kSmallItems = 7;                             // keys per thread at most
 constexpr int kSmallMaxPer = kSmallThreads * kSmallItems;  // positions per block at most
-constexpr int kSmallMax = 28 * 1024;
-static_assert(kSmallMax <= kSmallCtas * kSmallMaxPer, "a block's positions fit its threads");
+constexpr int kSmallMax = kSmallCtas * kSmallMaxPer;        // 28,672 particles
 
 constexpr size_t small_sort_smem(int m) {
     return size_t(m) * 2 * (sizeof(uint64_t) + sizeof(int)) + sizeof(uint16_t) * kSmallWarps * 256;
@@ -267,12 +267,12 @@ constexpr size_t small_sort_smem(int m) {
 
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
     k_small_sort(const double* __restrict__ pos, int n, int m, unsigned div_m, double theta, RootBox* __restrict__ root,
-                 uint64_t* __restrict__ key, int* __restrict__ perm, uint32_t* status) {
+                 uint64_t* __restrict__ key, int* __restrict__ perm, TreeCounts* __restrict__ counts, uint32_t* status) {
     extern __shared__ unsigned char smem_small[];
     uint64_t* kb = reinterpret_cast<uint64_t*>(smem_small);  // two buffers of m keys
     int* vb = reinterpret_cast<int*>(kb + 2 * m);            // two of m indices
     uint16_t* cnt = reinterpret_cast<uint16_t*>(vb + 2 * m);  // [warp][digit]
-    __shared__ int s_tot[kSmallCtas][256], s_part[4][256], s_base[256], s_wsum[kSmallWarps];
+    __shared__ int s_tot[kSmallCtas][256], s_part[kSmallThreads / 256][256], s_base[256], s_wsum[kSmallWarps];
     __shared__ long long s_box[7], s_red[kSmallWarps][7];
     __shared__ RootBox s_root;
     namespace cg = cooperative_groups;
@@ -282,6 +282,8 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     const unsigned lt = lanemask_lt();
     const int first = rank * m;                   // this block's positions: [first, first + own)
     const int own = max(0, min(m, n - first));
+    if (rank == 0)  // the build's counters start at zero (nothing uses them before the next launch)
+        for (int t = tid; t < int(sizeof(TreeCounts) / sizeof(int)); t += kSmallThreads) reinterpret_cast<int*>(counts)[t] = 0;
 
     // bounding box of the block's share, then of all blocks (exact: min and max of integer images)
     long long v[7] = {LLONG_MAX, LLONG_MAX, LLONG_MAX, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0};
@@ -378,7 +380,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         // four threads per digit: exclusive prefix over the warps; the block's count of every digit
         // goes to all blocks
         const int d = tid & 255, part = tid >> 8;
-        constexpr int kPart = kSmallWarps / 4;
+        constexpr int kParts = kSmallThreads / 256, kPart = kSmallWarps / kParts;
         int sum = 0;
 #pragma unroll
         for (int w = 0; w < kPart; ++w) sum += cnt[(part * kPart + w) * 256 + d];
@@ -386,13 +388,13 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         __syncthreads();
         int run = 0, own_d = 0;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < kParts; ++t) {
             const int x = s_part[t][d];
             if (t < part) run += x;
             own_d += x;
         }
 #pragma unroll
-        for (int c = 2 * part; c < 2 * part + 2; ++c) *cluster.map_shared_rank(&s_tot[rank][d], c) = own_d;
+        for (int c = part; c < kSmallCtas; c += kParts) *cluster.map_shared_rank(&s_tot[rank][d], c) = own_d;
         auto counted = cluster.barrier_arrive();
 #pragma unroll
         for (int w = 0; w < kPart; ++w) {
@@ -568,8 +570,8 @@ __device__ int run_begin(const KeyView& K, int i, int lev) {
 // the run containing i). Threads of consecutive ids take chains of similar depth, so a warp
 // keeps most lanes busy (one thread per starting position left 5 of 32 busy).
 // A leaf's thread also puts its particles in increasing index order (the reference's stable
-// partitions never reorder a leaf), and the nodes of each depth are counted for the breadth-first
-// numbering.
+// partitions never reorder a leaf), the nodes of each depth are counted for the breadth-first
+// numbering, and that pass's look-back statuses are cleared.
 __global__ void k_node_owner(int n, StartScan S) {  // after the node buffers have grown
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) S.put(i, S.again(i), S.nbase[i]);
@@ -655,8 +657,10 @@ __global__ void k_emit(KeyView K, int n, int span, const RootBox* __restrict__ r
                        const int* __restrict__ nbase, const int* __restrict__ owner,
                        TreeCounts* __restrict__ cnt, int4* __restrict__ n_i4,
                        double4* __restrict__ n_cd, float4* __restrict__ n_geo,
-                       int* __restrict__ n_parent, int* __restrict__ perm, int cap) {
+                       int* __restrict__ n_parent, int* __restrict__ perm, int cap,
+                       unsigned* __restrict__ bfs_status, int status_words) {
     __shared__ int s_depth[kDepthMax + 1];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < status_words; t += gridDim.x * blockDim.x) bfs_status[t] = 0u;
     if (threadIdx.x <= kDepthMax) s_depth[threadIdx.x] = 0;
     __syncthreads();
     emit_node(K, n, span, rootp, ldepth, dsplit, nbase, owner, cnt, n_i4, n_cd, n_geo, n_parent, perm, cap, s_depth);
@@ -1410,7 +1414,8 @@ void Octree::small_sort(const double* pos, cudaStream_t s) {
     // floor(t / m) = mulhi(t, div_m) for every t below kSmallMax: t m < 2^32
     const unsigned div_m = m > 1 ? unsigned((0x100000000ull + m - 1) / m) : 0u;
     k_small_sort<<<kSmallCtas, kSmallThreads, small_sort_smem(m), s>>>(
-        pos, n, m, div_m, double(theta_f), root.as<RootBox>(), key.as<uint64_t>(), perm.as<int>(), ctx().d_status);
+        pos, n, m, div_m, double(theta_f), root.as<RootBox>(), key.as<uint64_t>(), perm.as<int>(),
+        counts.as<TreeCounts>(), ctx().d_status);
     GF_CHECK_LAUNCH();
 }
 
@@ -1425,8 +1430,6 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     if (!h_counts) GF_CUDA(cudaMallocHost(&h_counts, sizeof(TreeCounts)));
     TreeCounts* cnt = counts.get<TreeCounts>(1);
     RootBox* R = root.get<RootBox>(1);
-    GF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(TreeCounts), s));
-
     const int grid = div_up(n, kThreads);
     uint64_t* k0 = key.get<uint64_t>(n);
     int* pm = perm.get<int>(n);
@@ -1438,6 +1441,7 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
         ProfScope pso(want_knn ? kStCount : kStTreeSort, s);
         small_sort(pos, s);
     } else {
+        GF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(TreeCounts), s));
         double* part = reinterpret_cast<double*>(nb);  // bbox partials, consumed before the scan
         k_bbox<<<nparts, kThreads, 0, s>>>(pos, n, part, R, double(theta_f), C.d_status, &cnt->bbox_done);
         GF_CHECK_LAUNCH();
@@ -1489,6 +1493,7 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     const int span = graph_safe ? cap : nn;
     const int* nn_dev = &cnt->total_nodes;
     const int ngrid = div_up(span, kThreads);
+    const int bfs_tiles = div_up(span, kBfsTile);
 
     int4* i4 = n_i4.get<int4>(cap);
     double4* cd = n_cd.get<double4>(cap);
@@ -1504,7 +1509,8 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
             GF_CHECK_LAUNCH();
         }
         k_emit<<<ngrid, kThreads, 0, s>>>(K, n, span, R, starts.ldepth, starts.dsplit, nb, own, cnt, i4, cd, geo, par,
-                                          pm, cap);
+                                          pm, cap, bfs_status.get<unsigned>(size_t(div_up(cap, kBfsTile)) * kDepthBins),
+                                          bfs_tiles * kDepthBins);
         GF_CHECK_LAUNCH();
     }
     if (graph_safe) {  // more nodes than the buffers hold: flag, and leave an empty tree
@@ -1521,11 +1527,8 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
     scan_with(GroupScan{nn_dev, span, group_max, i4, par, nch, n_counter.get<int>(cap), groups.get<int>(cap)}, span,
               &cnt->num_groups, s, &scratch);
     int* bfs = n_bfs.get<int>(cap);
-    const int bfs_tiles = div_up(span, kBfsTile);
-    const size_t status_words = size_t(bfs_tiles) * kDepthBins;
-    unsigned* status = bfs_status.get<unsigned>(size_t(div_up(cap, kBfsTile)) * kDepthBins);
-    GF_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned) * status_words, s));
-    k_bfs_rank<<<bfs_tiles, kBfsThreads, 0, s>>>(span, cnt, i4, status, bfs, bfs_val.get<int>(cap), C.d_status);
+    k_bfs_rank<<<bfs_tiles, kBfsThreads, 0, s>>>(span, cnt, i4, bfs_status.as<unsigned>(), bfs, bfs_val.get<int>(cap),
+                                                 C.d_status);
     GF_CHECK_LAUNCH();
     k_walk_fill<<<ngrid, kThreads, 0, s>>>(span, i4, nch, bfs, geo, w_b.get<float4>(cap), w_geo.get<float4>(cap),
                                            want_knn ? leaf_of.get<int>(n) : nullptr, par, w_parent.get<int>(cap),
@@ -1543,7 +1546,9 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
         moments(mass, false, span, s);
     }
     valid = true;
-    if (!g_no_alloc) {  // outside a capture: the live node count, for outgrowing()
+    if (!graph_safe) {
+        live_pending = false;  // the host knows the node count, and the buffers have room for it
+    } else if (!g_no_alloc) {  // outside a capture: the live node count, for outgrowing()
         if (!h_live) GF_CUDA(cudaMallocHost(&h_live, sizeof(int)));
         if (!live_ev) GF_CUDA(cudaEventCreateWithFlags(&live_ev, cudaEventDisableTiming));
         GF_CUDA(cudaMemcpyAsync(h_live, &cnt->total_nodes, sizeof(int), cudaMemcpyDeviceToHost, s));
