@@ -265,6 +265,35 @@ __device__ inline void warp_sort_u64(unsigned long long* key, int P) {
     }
 }
 
+// Sorting a warp's distances by buckets. The number of points within r grows like r^3, so
+// f (0.4 + 0.6 f) ~ f^(3/2) of f = d^2 / (largest d^2) spreads them evenly over the buckets. The map is
+// weakly monotone in float32 (a product of non-decreasing factors), so the buckets follow the order of
+// the distances; a NaN (0 times infinity) counts as 0.
+constexpr int kSortBuckets = 128;  // four per lane
+
+__device__ __forceinline__ int distance_bucket(float f) {
+    return max(0, min(kSortBuckets - 1, int(f * fmaf(0.6f, f, 0.4f) * float(kSortBuckets))));
+}
+
+// first[kSortBuckets + 1] (16-byte aligned) in shared memory: counters, then the buckets' first places.
+__device__ __forceinline__ void clear_buckets(int* first) {
+    reinterpret_cast<int4*>(first)[threadIdx.x & 31] = make_int4(0, 0, 0, 0);
+}
+
+// Counts (cnt in all) to first places, in place; returns the largest count. Synchronises the warp
+// after its writes; the caller does before.
+__device__ __forceinline__ int bucket_starts(int* first, int cnt) {
+    const int lane = threadIdx.x & 31;
+    const int4 c = reinterpret_cast<const int4*>(first)[lane];
+    const int sum = c.x + c.y + c.z + c.w;
+    const int e = warp_incl_scan(sum) - sum;
+    reinterpret_cast<int4*>(first)[lane] = make_int4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z);
+    if (lane == 0) first[kSortBuckets] = cnt;
+    const int most = __reduce_max_sync(0xffffffffu, max(max(c.x, c.y), max(c.z, c.w)));
+    __syncwarp();
+    return most;
+}
+
 // atomicAdd with acquire-release semantics at GPU scope (bottom-up tree passes: the last
 // arriving child sees its siblings' records without separate fences)
 __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {

@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kCandWarps * 32) k_knn_cand(
 
 // ------------------------------------------------------------------------ exact kNN
 
-constexpr int kKnnWarps = 8;
+constexpr int kKnnOneQuery = 8 * 1024, kKnnTwoQueries = 64 * 1024;  // most queries with one / two per warp
 // Leaf capacity of the neighbour-search tree. The search is exact for any tree; 16 walks
 // fewer levels per query (7 % faster on the 1M disk) but its coarser leaf counts make the
 // learned guess's features less informative, so the reference's 8 is kept.
@@ -408,20 +408,30 @@ __device__ __forceinline__ unsigned long long knn_key(float d2, int j) {
 __device__ __forceinline__ float key_d2(unsigned long long k) { return __uint_as_float(unsigned(k >> 32)); }
 __device__ __forceinline__ int key_idx(unsigned long long k) { return int(unsigned(k)); }
 
-struct KnnSmem {
-    int stack[kKnnStack];
-    unsigned long long key[2][kKnnCap];  // the collected points of the warp's two queries
-    unsigned long long dd[64];  // float64 squared distances as bit patterns
-    int di[64];
-    int seg[64];                // opened leaves of a round: first particle minus first slot
+// A query of a neighbour walk: position (hi / lo) with the radius and its square, in shared memory
+// (registers for two to four of them spilled at four blocks per SM).
+struct KnnQuery {
+    float4 h;  // x y z of the position's high parts, radius
+    float4 l;  // low parts, squared radius
+    float lo, hi;  // bracket of the radius iteration
 };
 
-// A query of a neighbour walk: position (hi/lo), radius; `on` (warp-uniform) false for a slot
-// without a query or one already settled.
-struct KnnQuery {
-    float4 xh, xl;
-    float R, R2;
-    bool on;
+// Shared memory of a warp that serves kQ queries. The sort's counters and the float64 near-ties
+// reuse the walk's stack: a query is finished after its walk.
+template <int kQ>
+struct KnnSmem {
+    union {
+        int stack[kKnnStack];
+        struct {
+            unsigned long long dd[64];  // float64 squared distances as bit patterns
+            int di[64];
+            int first[kSortBuckets + 4];  // of the sort: a bucket's count, then its first key
+        };
+    };
+    unsigned long long key[kQ][kKnnCap];  // the collected points of the warp's queries
+    int seg[32];                // opened leaves of a round: first particle minus first slot
+    KnnQuery q[kQ];
+    int cnt[kQ];                // points of the last walk
 };
 
 struct KnnArgs {
@@ -452,130 +462,182 @@ struct KnnArgs {
                             //    only to settle the neighbour at dsel_col (the h boundary)
 };
 
-// Collects, for each of the warp's (up to) two queries that is on, the points within its radius
-// into S.key[i] (the first kKnnCap of them) and their number into cnt[i]; one walk serves both:
-// a node is opened when it meets either sphere, and each point of an opened leaf is tested
-// against both. A query with more than kKnnCap points is done with this radius: its sphere opens
-// no further nodes (cnt[i] then is only known to exceed kKnnCap). Returns false on stack overflow. The two queries of a warp are neighbours in
-// the tree's order (usually in one leaf), so their walks share most nodes.
-__device__ bool knn_collect(const KnnArgs& A, KnnSmem& S, const KnnQuery (&Q)[2], int leaf, int (&cnt)[2]) {
+// Collects, for each of the warp's (up to) kQ queries that is on, the points within its radius
+// into S.key[i] (the first kKnnCap of them) and their number into S.cnt[i]. One walk serves all: a
+// node is opened when it meets any of the spheres (a test against the queries' bounding box and
+// largest radius opens far too much where consecutive queries lie in cells apart: 10 ms instead of
+// 2 for the 1M disk's gas), and each point of an opened leaf is tested against every query. A query
+// with more than kKnnCap points is done with this radius: its sphere opens no further nodes
+// (S.cnt[i] then is only known to exceed kKnnCap). Returns false on stack overflow. The queries of a
+// warp are neighbours in the tree's order (often in one leaf), so their walks share most nodes.
+template <int kQ>
+__device__ bool knn_collect(const KnnArgs& A, KnnSmem<kQ>& S, unsigned live, int leaf) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
+    int cnt[kQ] = {};
     // start at the smallest ancestor of the leaf whose cube contains every sphere that is on
     // (every point within a radius then lies in that subtree)
     int start = leaf;
     for (int up = 0; start > 0 && up < 64; ++up) {
         const float4 g = A.wgeo[start];
+        const int parent = A.wparent[start];
         const float pad = 2e-6f * (fabsf(g.x) + fabsf(g.y) + fabsf(g.z) + g.w) + 1e-30f;
         bool inside = true;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (!Q[i].on) continue;
-            const float lim = g.w - Q[i].R - pad;
-            inside = inside && fabsf((Q[i].xh.x - g.x) + Q[i].xl.x) <= lim &&
-                     fabsf((Q[i].xh.y - g.y) + Q[i].xl.y) <= lim && fabsf((Q[i].xh.z - g.z) + Q[i].xl.z) <= lim;
+        for (int i = 0; i < kQ; ++i) {
+            if (!(live >> i & 1u)) continue;
+            const float4 qh = S.q[i].h, ql = S.q[i].l;
+            const float lim = g.w - qh.w - pad;
+            inside = inside && fabsf((qh.x - g.x) + ql.x) <= lim && fabsf((qh.y - g.y) + ql.y) <= lim &&
+                     fabsf((qh.z - g.z) + ql.z) <= lim;
         }
         if (inside) break;
-        start = A.wparent[start];
+        start = parent;
     }
     if (start < 0) start = 0;
-    cnt[0] = cnt[1] = 0;
-    bool live[2] = {Q[0].on, Q[1].on};  // still collecting (warp-uniform)
     int sp = 1;
     if (lane == 0) S.stack[0] = (start << 4) | 1;
     __syncwarp();
-    for (int rounds = 0; sp > 0 && (live[0] || live[1]); ++rounds) {
+    for (int rounds = 0; sp > 0; ++rounds) {
         if (rounds > A.nn) return false;  // each node is popped at most once
-        // pop up to 64 nodes (two per lane: their loads overlap)
-        int node[2];
-        const int nnodes = pop_round<2>(S.stack, sp, node);
-        float4 G[2], B[2];
+        int node[1];
+        pop_round<1>(S.stack, sp, node);
+        bool open = false;
+        int first = 0, code = 0;
+        if (node[0] >= 0) {
+            const float4 g = A.wgeo[node[0]], b = A.wb[node[0]];
+            first = __float_as_int(b.y);
+            code = __float_as_int(b.z);
+            // distance from each query to the cell cube, padded for float32 rounding
+            const float lim = g.w + 2e-6f * (fabsf(g.x) + fabsf(g.y) + fabsf(g.z) + g.w) + 1e-30f;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (node[j] >= 0) {
-                G[j] = A.wgeo[node[j]];
-                B[j] = A.wb[node[j]];
+            for (int i = 0; i < kQ; ++i) {
+                if (!(live >> i & 1u)) continue;
+                const float4 qh = S.q[i].h, ql = S.q[i].l;
+                const float ex = fmaxf(fabsf((g.x - qh.x) - ql.x) - lim, 0.f);
+                const float ey = fmaxf(fabsf((g.y - qh.y) - ql.y) - lim, 0.f);
+                const float ez = fmaxf(fabsf((g.z - qh.z) - ql.z) - lim, 0.f);
+                open = open || ex * ex + ey * ey + ez * ez <= ql.w;
             }
         }
-        int first[2] = {0, 0}, lcs[2] = {0, 0};
+        const bool inner = open && code > 0;
+        const unsigned om = __ballot_sync(0xffffffffu, inner);
+        const int npush = __popc(om);
+        if (sp + npush > kKnnStack) return false;
+        if (inner) S.stack[sp + __popc(om & lt)] = (first << 4) | code;
+        sp += npush;
+        // particles of the opened leaves, concatenated in lane order and tested 32 at a time: lane l
+        // takes offset o = base + l
+        const bool leaf_open = open && code < 0;
+        const unsigned lm = __ballot_sync(0xffffffffu, leaf_open);
+        if (lm) {
+            const int lc = leaf_open ? -code : 0;
+            const int lincl = warp_incl_scan(lc);
+            const int lexcl = lincl - lc;
+            const int ltot = __shfl_sync(0xffffffffu, lincl, 31);
+            if (leaf_open) S.seg[__popc(lm & lt)] = first - lexcl;
+            __syncwarp();
+            int before = -1;
+            for (int base = 0; base < ltot; base += 32) {
+                const int o = base + lane;
+                const unsigned marks = segment_marks(leaf_open, lexcl, base);
+                const int src = before + __popc(marks & (lt | (1u << lane)));
+                before += __popc(marks);
+                float4 ph = make_float4(0.f, 0.f, 0.f, 0.f), pl = ph;
+                int j = 0;
+                if (o < ltot) {
+                    j = S.seg[src] + o;
+                    ph = A.p4[j];
+                    pl = A.plo[j];
+                }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (32 * j >= nnodes) break;  // warp-uniform
-            bool open = false;
-            int code = 0;
-            if (node[j] >= 0) {
-                const float4 g = G[j];
-                first[j] = __float_as_int(B[j].y);
-                code = __float_as_int(B[j].z);
-                // distance from each query to the cell cube, padded for float32 rounding
-                const float lim = g.w + 2e-6f * (fabsf(g.x) + fabsf(g.y) + fabsf(g.z) + g.w) + 1e-30f;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    if (!live[i]) continue;
-                    const float ex = fmaxf(fabsf((g.x - Q[i].xh.x) - Q[i].xl.x) - lim, 0.f);
-                    const float ey = fmaxf(fabsf((g.y - Q[i].xh.y) - Q[i].xl.y) - lim, 0.f);
-                    const float ez = fmaxf(fabsf((g.z - Q[i].xh.z) - Q[i].xl.z) - lim, 0.f);
-                    open = open || ex * ex + ey * ey + ez * ez <= Q[i].R2;
+                for (int i = 0; i < kQ; ++i) {
+                    if (!(live >> i & 1u)) continue;
+                    const float4 qh = S.q[i].h, ql = S.q[i].l;
+                    const float dx = (ph.x - qh.x) + (pl.x - ql.x);
+                    const float dy = (ph.y - qh.y) + (pl.y - ql.y);
+                    const float dz = (ph.z - qh.z) + (pl.z - ql.z);
+                    const float d2 = dx * dx + dy * dy + dz * dz;
+                    const bool hit = o < ltot && d2 <= ql.w;
+                    const unsigned hm = __ballot_sync(0xffffffffu, hit);
+                    if (hit) {
+                        const int slot = cnt[i] + __popc(hm & lt);
+                        if (slot < kKnnCap) S.key[i][slot] = knn_key(d2, j);
+                    }
+                    cnt[i] += __popc(hm);
                 }
             }
-            const bool inner = open && code > 0;
-            const unsigned om = __ballot_sync(0xffffffffu, inner);
-            const int npush = __popc(om);
-            if (sp + npush > kKnnStack) return false;
-            if (inner) S.stack[sp + __popc(om & lt)] = (first[j] << 4) | code;
-            sp += npush;
-            lcs[j] = open && code < 0 ? -code : 0;
-        }
-        // particles of the opened leaves, concatenated in lane order (a lane's two leaves in
-        // turn) and tested 32 at a time: lane l takes offset o = base + l
-        const int lc = lcs[0] + lcs[1];
-        if (__any_sync(0xffffffffu, lc > 0)) {  // some leaf opened in this round
-        const int lincl = warp_incl_scan(lc);
-        const int lexcl = lincl - lc;
-        const int ltot = __shfl_sync(0xffffffffu, lincl, 31);
-        const bool has0 = lcs[0] > 0, has1 = lcs[1] > 0;
-        const int start1 = lexcl + lcs[0];
-        const int rank0 = __popc(__ballot_sync(0xffffffffu, has0) & lt) + __popc(__ballot_sync(0xffffffffu, has1) & lt);
-        if (has0) S.seg[rank0] = first[0] - lexcl;
-        if (has1) S.seg[rank0 + (has0 ? 1 : 0)] = first[1] - start1;
-        __syncwarp();
-        int before = -1;
-        for (int base = 0; base < ltot; base += 32) {
-            const int o = base + lane;
-            const unsigned r0 = unsigned(lexcl - base), r1 = unsigned(start1 - base);
-            const unsigned marks = __reduce_or_sync(
-                0xffffffffu, (has0 && r0 < 32u ? 1u << r0 : 0u) | (has1 && r1 < 32u ? 1u << r1 : 0u));
-            const int src = before + __popc(marks & (lt | (1u << lane)));
-            before += __popc(marks);
-            float4 ph = make_float4(0.f, 0.f, 0.f, 0.f), pl = ph;
-            int j = 0;
-            if (o < ltot) {
-                j = S.seg[src] + o;
-                ph = A.p4[j];
-                pl = A.plo[j];
-            }
+            unsigned full = 0;
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (!live[i]) continue;
-                const float dx = (ph.x - Q[i].xh.x) + (pl.x - Q[i].xl.x);
-                const float dy = (ph.y - Q[i].xh.y) + (pl.y - Q[i].xl.y);
-                const float dz = (ph.z - Q[i].xh.z) + (pl.z - Q[i].xl.z);
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                const bool hit = o < ltot && d2 <= Q[i].R2;
-                const unsigned hm = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const int slot = cnt[i] + __popc(hm & lt);
-                    if (slot < kKnnCap) S.key[i][slot] = knn_key(d2, j);
-                }
-                cnt[i] += __popc(hm);
-            }
+            for (int i = 0; i < kQ; ++i) full |= cnt[i] > kKnnCap ? 1u << i : 0u;
+            live &= ~full;
+            if (!live) break;
         }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) live[i] = live[i] && cnt[i] <= kKnnCap;
-        }  // any leaf
         __syncwarp();
     }
+#pragma unroll
+    for (int i = 0; i < kQ; ++i)
+        if (lane == i) S.cnt[i] = cnt[i];
+    __syncwarp();
     return true;
+}
+
+// Sorts the cnt (<= kKnnCap) keys of a query within the squared radius 1 / inv_R2, ascending, by
+// buckets of their distance (distance_bucket): a key's place is its bucket's first one plus the
+// smaller keys of that bucket (two or three). About 130 warp instructions for 64 keys and 210 for 128, where the bitonic
+// network takes 300 and 780. Distances piled up in one bucket take the network.
+__device__ __forceinline__ void knn_sort(unsigned long long* key, int* first, int cnt, float inv_R2) {
+    constexpr int kPer = kKnnCap / 32;
+    const int lane = threadIdx.x & 31;
+    clear_buckets(first);
+    __syncwarp();
+    unsigned long long K[kPer];
+    int at[kPer];  // bucket << 8 | place in it
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        at[t] = -1;
+        if (32 * t >= cnt) break;  // warp-uniform
+        if (32 * t + lane < cnt) {
+            K[t] = key[32 * t + lane];
+            const int b = distance_bucket(key_d2(K[t]) * inv_R2);
+            at[t] = b << 8 | atomicAdd(first + b, 1);
+        }
+    }
+    __syncwarp();
+    if (bucket_starts(first, cnt) > 12) {
+        int P = 64;
+        while (P < cnt) P <<= 1;
+        for (int t = cnt + lane; t < P; t += 32) key[t] = ~0ull;
+        __syncwarp();
+        warp_sort_u64(key, P);
+        return;
+    }
+    int b0[kPer], b1[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        b0[t] = b1[t] = 0;
+        if (32 * t >= cnt) break;
+        if (at[t] >= 0) {
+            b0[t] = first[at[t] >> 8];
+            b1[t] = first[(at[t] >> 8) + 1];
+            key[b0[t] + (at[t] & 255)] = K[t];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        if (32 * t >= cnt) break;
+        int r = b0[t];
+        for (int m = b0[t]; m < b1[t]; ++m) r += key[m] < K[t] ? 1 : 0;
+        at[t] = at[t] >= 0 ? r : -1;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+        if (32 * t >= cnt) break;
+        if (at[t] >= 0) key[at[t]] = K[t];
+    }
+    __syncwarp();
 }
 
 // Sorts the cnt (<= kKnnCap) collected points of query q (tree position), re-measures the
@@ -588,16 +650,14 @@ __device__ __forceinline__ double d2_f64(const KnnArgs& A, int pi, int pj) {
     return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
-__device__ void knn_finish(const KnnArgs& A, unsigned long long* key, unsigned long long* dd, int* di, int cnt,
-                           int q) {
+template <int kQ>
+__device__ void knn_finish(const KnnArgs& A, KnnSmem<kQ>& S, unsigned long long* key, int cnt, float R2, int q) {
+    unsigned long long* dd = S.dd;
+    int* di = S.di;
     const int lane = threadIdx.x & 31;
     const int k = A.k;
     const int oq = A.perm[q];
-    int P = 64;
-    while (P < cnt) P <<= 1;
-    for (int t = cnt + lane; t < P; t += 32) key[t] = ~0ull;
-    __syncwarp();
-    warp_sort_u64(key, P);
+    knn_sort(key, S.first, cnt, 1.0f / R2);
     const int pi = oq;
     if (!A.exact_order) {
         // Float32 order: the k nearest as a set (only pairs tied to float32 rounding can
@@ -612,8 +672,8 @@ __device__ void knn_finish(const KnnArgs& A, unsigned long long* key, unsigned l
             below += v < lo;
             inband += v >= lo && v <= hi;
         }
-        below = warp_sum(below);
-        inband = warp_sum(inband);
+        below = __reduce_add_sync(0xffffffffu, below);
+        inband = __reduce_add_sync(0xffffffffu, inband);
         double best = 0.0;
         int selc = -1;  // caller index of the entry that fixes h
         if (inband == 1) {  // no float32 near-tie: entry c itself, measured in float64
@@ -663,7 +723,7 @@ __device__ void knn_finish(const KnnArgs& A, unsigned long long* key, unsigned l
     const float thr = key_d2(key[k - 1]) * (1.0f + 2e-5f);
     int m = 0;
     for (int t = lane; t < cnt; t += 32) m += key_d2(key[t]) <= thr;
-    m = min(64, warp_sum(m));
+    m = min(64, __reduce_add_sync(0xffffffffu, m));
     for (int t = lane; t < 64; t += 32) {
         double v = INFINITY;
         int tag = 0x7fffffff;
@@ -733,39 +793,32 @@ __device__ __forceinline__ float knn_rank_radius(const unsigned (&b)[kPer], int 
     return sqrtf(__uint_as_float((lo + 1) << kKnnRankShift)) * 1.0001f;
 }
 
-// Starting radii of a warp's two queries without a previous h: the kKnnWindow points around them
+// Starting radius of a query without a previous h: the kKnnWindow points around its warp's queries
 // in tree order hold most of the nearest ones, so the radius that encloses window_rank of them
 // encloses about k of all points. The first search of the 1M disk's 500k gas is bound by the
 // points its spheres collect: from the leaf's cell density, whose one to eight points say little,
 // spheres held hundreds to thousands of them (8.70 ms); from here, with collections that stop at the
-// cap, 3.22 ms (2.10 ms with a previous h).
+// cap, 2.64 ms (1.51 ms with a previous h).
 constexpr int kKnnWindow = 128;
 
-__device__ __forceinline__ void knn_window_radii(const KnnArgs& A, int q0, KnnQuery (&Q)[2]) {
+__device__ __forceinline__ float knn_window_radius(const KnnArgs& A, int q0, const KnnQuery& Q) {
     constexpr int kPer = kKnnWindow / 32;
     const int lane = threadIdx.x & 31;
     const int w0 = max(0, min(q0 - kKnnWindow / 2 + 1, A.n - kKnnWindow));
-    unsigned b[2][kPer];
+    unsigned b[kPer];
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
         const int j = w0 + 32 * t + lane;
-        b[0][t] = b[1][t] = 0xffffffffu;
+        b[t] = 0xffffffffu;
         if (j < A.n) {
             const float4 ph = A.p4[j], pl = A.plo[j];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (!Q[i].on) continue;
-                const float dx = (ph.x - Q[i].xh.x) + (pl.x - Q[i].xl.x);
-                const float dy = (ph.y - Q[i].xh.y) + (pl.y - Q[i].xl.y);
-                const float dz = (ph.z - Q[i].xh.z) + (pl.z - Q[i].xl.z);
-                b[i][t] = __float_as_uint(dx * dx + dy * dy + dz * dz) >> kKnnRankShift;
-            }
+            const float dx = (ph.x - Q.h.x) + (pl.x - Q.l.x);
+            const float dy = (ph.y - Q.h.y) + (pl.y - Q.l.y);
+            const float dz = (ph.z - Q.h.z) + (pl.z - Q.l.z);
+            b[t] = __float_as_uint(dx * dx + dy * dy + dz * dz) >> kKnnRankShift;
         }
     }
-    const int rank = min(A.window_rank, min(A.n, kKnnWindow));
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-        if (Q[i].on) Q[i].R = knn_rank_radius<kPer>(b[i], rank);
+    return knn_rank_radius<kPer>(b, min(A.window_rank, min(A.n, kKnnWindow)));
 }
 
 // Next radius of a query whose sphere holds more than kKnnCap points (key: kKnnCap of them): the
@@ -794,71 +847,80 @@ __device__ __forceinline__ float knn_next_radius(float R, int cnt, int k, const 
     return knn_shrunk_radius(key, k, R);
 }
 
-// One warp per pair of consecutive queries (tree order): walk from the smallest ancestor cell
-// containing both search spheres, collecting for both at once; each query iterates its radius
-// on its own, and a query still searching after the other has settled walks alone. Four blocks
-// of 8 warps per SM (64 registers): 15 % faster than with the 80 registers the compiler takes
-// unbounded (3 blocks), and 15 % faster than one query per warp.
-__global__ void __launch_bounds__(kKnnWarps * 32, 4) k_knn(KnnArgs A) {
-    __shared__ KnnSmem smem_all[kKnnWarps];
-    KnnSmem& S = smem_all[threadIdx.x >> 5];
+// One warp per kQ consecutive queries (tree order): one walk from the smallest ancestor cell that
+// contains all their spheres collects for all of them; each iterates its radius on its own, and
+// those still searching walk again together. Bound by instruction issue (about 70 % of the slots).
+// 32 warps per SM at 64 registers (24 at 80: 15 % slower; 40 at 48, spilling: 12 %). Of the time of a
+// pair of queries 30 % went to node rounds of 28 nodes, 32 % to finishing (the sort), 20 % to points,
+// 8 % to the ascent; with three queries to a walk, rounds of one node per lane instead of two and
+// the sort by buckets the search of 500k gas takes 1.51 ms with a previous h (2.07 before) and 2.64
+// ms without one (3.20).
+template <int kQ, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 32 / kWarps) k_knn(KnnArgs A) {
+    __shared__ __align__(16) KnnSmem<kQ> smem_all[kWarps];
+    KnnSmem<kQ>& S = smem_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int k = A.k;
     const int cap = kKnnCap;  // count window [k, cap]
-    const int nwarps = gridDim.x * kKnnWarps;
-    for (int q0 = 2 * (blockIdx.x * kKnnWarps + (threadIdx.x >> 5)); q0 < A.n; q0 += 2 * nwarps) {
-        KnnQuery Q[2];
-        float lo[2], hi[2];
-        int it[2] = {0, 0}, total = 0;
+    const int nwarps = gridDim.x * kWarps;
+    auto set_radius = [&](int i, float R) {
+        if (!(R > 0.f) || !isfinite(R)) R = 1e-3f;
+        if (lane == 0) S.q[i].h.w = R, S.q[i].l.w = R * R;
+    };
+    for (int q0 = kQ * (blockIdx.x * kWarps + (threadIdx.x >> 5)); q0 < A.n; q0 += kQ * nwarps) {
+        const int nq = min(kQ, A.n - q0);
         const bool window = !A.r_guess && A.window_rank > 0;
-        bool from_window[2] = {window, window};
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int q = q0 + i;
-            Q[i].on = q < A.n;
-            lo[i] = 0.f;
-            hi[i] = INFINITY;
-            if (!Q[i].on) continue;
-            Q[i].xh = A.p4[q];
-            Q[i].xl = A.plo[q];
-            if (!window) Q[i].R = A.r_guess ? A.r_guess[A.perm[q]] : knn_cell_radius(A, q);
+        unsigned on = (1u << nq) - 1u, windowed = window ? on : 0u;  // bits of the queries
+        int total = 0, walks = 0;
+        if (lane < nq) {
+            S.q[lane].h = A.p4[q0 + lane];
+            S.q[lane].l = A.plo[q0 + lane];
+            S.q[lane].lo = 0.f;
+            S.q[lane].hi = INFINITY;
         }
-        if (window) knn_window_radii(A, q0, Q);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            if (!(Q[i].R > 0.f) || !isfinite(Q[i].R)) Q[i].R = 1e-3f;
-            Q[i].R2 = Q[i].R * Q[i].R;
-        }
-        while (Q[0].on || Q[1].on) {
-            int cnt[2];
-            const int leaf = A.leaf_of[Q[0].on ? q0 : q0 + 1];
-            const bool ok_walk = knn_collect(A, S, Q, leaf, cnt);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (!Q[i].on) continue;
-                ++it[i];
-                ++total;
-                if (ok_walk && cnt[i] >= k && cnt[i] <= cap) {
-                    knn_finish(A, S.key[i], S.dd, S.di, cnt[i], q0 + i);
-                    Q[i].on = false;
-                } else if (ok_walk && it[i] < 48) {
-                    Q[i].R = knn_next_radius(Q[i].R, cnt[i], k, S.key[i], lo[i], hi[i]);
-                    Q[i].R2 = Q[i].R * Q[i].R;
-                } else if (from_window[i]) {  // once more, from the cell density
-                    from_window[i] = false;
-                    it[i] = 0;
-                    lo[i] = 0.f;
-                    hi[i] = INFINITY;
-                    Q[i].R = knn_cell_radius(A, q0 + i);
-                    if (!(Q[i].R > 0.f) || !isfinite(Q[i].R)) Q[i].R = 1e-3f;
-                    Q[i].R2 = Q[i].R * Q[i].R;
+        __syncwarp();
+        for (int i = 0; i < nq; ++i)
+            set_radius(i, window      ? knn_window_radius(A, q0, S.q[i])
+                          : A.r_guess ? A.r_guess[A.perm[q0 + i]]
+                                      : knn_cell_radius(A, q0 + i));
+        __syncwarp();
+        while (on) {
+            const bool ok_walk = knn_collect<kQ>(A, S, on, A.leaf_of[q0 + __ffs(on) - 1]);
+            total += __popc(on);
+            ++walks;
+            for (int i = 0; i < nq; ++i) {
+                if (!(on >> i & 1u)) continue;
+                const int cnt = S.cnt[i];
+                const float R = S.q[i].h.w;
+                if (ok_walk && cnt >= k && cnt <= cap) {
+                    knn_finish<kQ>(A, S, S.key[i], cnt, S.q[i].l.w, q0 + i);
+                    on &= ~(1u << i);
+                } else if (ok_walk && walks < 48) {
+                    float lo = S.q[i].lo, hi = S.q[i].hi;
+                    const float next = knn_next_radius(R, cnt, k, S.key[i], lo, hi);
+                    __syncwarp();
+                    if (lane == 0) {
+                        S.q[i].lo = lo;
+                        S.q[i].hi = hi;
+                        S.q[i].h.w = next;
+                        S.q[i].l.w = next * next;
+                    }
+                } else if (windowed >> i & 1u) {  // once more, from the cell density
+                    if (lane == 0) {
+                        S.q[i].lo = 0.f;
+                        S.q[i].hi = INFINITY;
+                    }
+                    set_radius(i, knn_cell_radius(A, q0 + i));
                 } else {
                     knn_fail_output(A, q0 + i, !ok_walk);
-                    Q[i].on = false;
+                    on &= ~(1u << i);
                 }
             }
+            if (walks == 48 || !ok_walk) windowed = 0, walks = 0;
+            __syncwarp();
         }
         if (lane == 0 && A.iters) atomicAdd(A.iters, (unsigned long long)total);
+        __syncwarp();
     }
 }
 
@@ -1031,8 +1093,24 @@ void knn_exact(Octree& T, int n, const double* pos, int k, const float* r_guess,
     A.wparent = T.w_parent.as<int>();
     A.window_rank = cell_start ? 0 : knn_window_rank(k);
     ProfScope ps(kStKnn, s);
-    const int blocks = std::min(div_up(n, 2 * kKnnWarps), 16 * ctx().sms);  // two queries per warp
-    k_knn<<<blocks, kKnnWarps * 32, 0, s>>>(A);
+    // Queries per warp: more of them share a walk, as long as their warps still fill the chip. First /
+    // later search in us with 1, 2, 3, 4 per warp (a Plummer-like cloud):
+    //     5k   83 /  54    124 /   66    148 /   81    193 /  100
+    //    10k  128 /  76    153 /   68    192 /   76    221 /   95
+    //    40k  313 / 189    299 /  165    354 /  151    505 /  162
+    //    80k  581 / 349    551 /  286    487 /  254    499 /  257
+    //   320k 2040 / 1288  1775 / 1193   1662 / 1082   1716 /  941
+    // (1M disk, 500k gas: 2 2854 / 1716, 3 2638 / 1509, 4 2853 / 1622).
+    auto go = [&](auto queries) {
+        constexpr int kQ = decltype(queries)::value, kWarps = kQ <= 2 ? 8 : 4;  // 48 KB of shared memory a block
+        k_knn<kQ, kWarps><<<std::min(div_up(n, kQ * kWarps), 16 * 8 / kWarps * ctx().sms), kWarps * 32, 0, s>>>(A);
+    };
+    if (n <= kKnnOneQuery)
+        go(std::integral_constant<int, 1>{});
+    else if (n <= kKnnTwoQueries)
+        go(std::integral_constant<int, 2>{});
+    else
+        go(std::integral_constant<int, 3>{});
     GF_CHECK_LAUNCH();
 }
 
