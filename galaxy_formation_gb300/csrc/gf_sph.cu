@@ -9,15 +9,15 @@
 //                              bitonic sort of the (<= 64) candidates in shared memory.
 //   exact k nearest .......... replaces cKDTree(p).query(p, k) (sph.py:165-166):
 //                              octree of the points (same builder as gravity); one warp per
-//                              two consecutive queries walks it with a radius per query,
+//                              one to three consecutive queries walks it with a radius each,
 //                              collecting the points within each radius (float32 distances
 //                              from hi/lo split coordinates) until the count lies in
 //                              [k, 128] — the radius iteration, Newton steps on
 //                              count ~ R^3 from a guess (2.5 x the previous h, 1.06 x the
 //                              learned guess of the k-th-neighbour distance, a rank of the
 //                              distances to the points next to the query in the tree's
-//                              order, or the leaf's cell density). The collected points are sorted,
-//                              the k nearest plus near-ties at the boundary are re-measured
+//                              order, or the leaf's cell density). The collected points are
+//                              sorted, the k nearest plus near-ties at the boundary are re-measured
 //                              in float64 and sorted again, so the result is the exact
 //                              float64 kNN.
 #include <algorithm>

@@ -1653,7 +1653,7 @@ void Octree::refit(const double* pos, const double* mass, cudaStream_t s, cudaSt
 }
 
 // The bottom-up moments pass of a build or a refit, straight into the breadth-first walk layout.
-// (The arrival counters are zero: k_nchild clears them in a build, and each pass leaves them so.)
+// (The arrival counters are zero: the group scan clears them in a build, and each pass leaves them so.)
 void Octree::moments(const double* mass, bool refit, int span, cudaStream_t s) {
     const int* nn_dev = &counts.as<TreeCounts>()->total_nodes;
     const int ngrid = div_up(span, kThreads);
