@@ -140,7 +140,8 @@ void scan_sums(int* sums, int cnt, int* total, cudaStream_t s) {
 }
 
 int* scan_scratch(int n, ScanScratch* sc) {
-    return (sc ? sc->scan_tmp : g_ctx.scan_tmp).get<int>(size_t(div_up(std::max(n, 1), kScanTile)) + 1);
+    // (for the smaller tiles: a buffer reserved for n also serves every smaller scan)
+    return (sc ? sc->scan_tmp : g_ctx.scan_tmp).get<int>(size_t(div_up(std::max(n, 1), kScanSmallTile)) + 1);
 }
 
 namespace {

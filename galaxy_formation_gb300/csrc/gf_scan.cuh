@@ -18,20 +18,24 @@
 
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "gf_common.cuh"
 
 namespace gf {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanItems = 8;       // entries per thread of a tile
+constexpr int kScanSmallItems = 1;  // while that makes at most kScanDirectTiles tiles (524,288 entries)
+constexpr int kScanSmallTile = kScanThreads * kScanSmallItems;
 // Tiles up to which each block of the second launch adds up the sums before its own (a few KB of L2
 // reads per block).
 constexpr int kScanDirectTiles = 2048;
-// One cluster launch up to this many entries: 1024 threads x kScanRows entries in each of 8 blocks.
+// One cluster launch up to this many entries: 1024 threads x kScanRows entries in each of 8 blocks
+// (with two rows, 16,384: gravity of 31k particles 292 us, with four 305; up to 24k no difference).
 constexpr int kScanCtas = 8;
 constexpr int kScanClusterThreads = 1024;
-constexpr int kScanRows = 4;
+constexpr int kScanRows = 2;
 constexpr int kScanClusterMax = kScanCtas * kScanClusterThreads * kScanRows;
 
 __device__ __forceinline__ int block_excl_scan(int v, int* s_warp, int* total) {
@@ -90,13 +94,13 @@ __global__ void __cluster_dims__(kScanCtas, 1, 1) __launch_bounds__(kScanCluster
     if (total && rank == 0 && threadIdx.x == 0) *total = all;
 }
 
-template <class F>
+template <class F, int kItems>
 __global__ void k_scan_tile_sums(F f, int n, int* __restrict__ sums) {
     __shared__ int s_warp[33];
-    const int base = blockIdx.x * kScanTile;
+    const int base = blockIdx.x * kScanThreads * kItems;
     int acc = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         const int i = base + k * kScanThreads + threadIdx.x;
         if (i < n) acc += f.first(i);
     }
@@ -107,7 +111,7 @@ __global__ void k_scan_tile_sums(F f, int n, int* __restrict__ sums) {
 
 // offs: the tile sums, or (SCANNED) their exclusive scan; the last block writes the total of the
 // former.
-template <class F, bool SCANNED>
+template <class F, int kItems, bool SCANNED>
 __global__ void k_scan_tiles(F f, int n, const int* __restrict__ offs, int* __restrict__ total) {
     __shared__ int s_warp[33];
     int prefix;
@@ -118,18 +122,18 @@ __global__ void k_scan_tiles(F f, int n, const int* __restrict__ offs, int* __re
         for (int t = threadIdx.x; t < int(blockIdx.x); t += kScanThreads) before += offs[t];
         block_excl_scan(before, s_warp, &prefix);
     }
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems];
+    const int base = (blockIdx.x * kScanThreads + threadIdx.x) * kItems;
+    int v[kItems];
     int acc = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         v[k] = (base + k < n) ? f.again(base + k) : 0;
         acc += v[k];
     }
     int tile_total;
     int ex = block_excl_scan(acc, s_warp, &tile_total) + prefix;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < kItems; ++k) {
         if (base + k < n) f.put(base + k, v[k], ex);
         ex += v[k];
     }
@@ -151,17 +155,28 @@ void scan_with(const F& f, int n, int* total, cudaStream_t s, ScanScratch* sc) {
         GF_CHECK_LAUNCH();
         return;
     }
-    const int tiles = div_up(n, kScanTile);
+    // The values of a tree build's scans are chains of loads (nine key pairs, up to eight children), so
+    // threads with fewer entries finish sooner: the tile sums of the node starts / groups of 200k
+    // particles 17.2 / 19.6 us with eight entries per thread, 5.5 / 6.6 with one; gravity of 100k
+    // particles 438 -> 414 us (four 426, two 416).
     int* sums = scan_scratch(n, sc);
-    k_scan_tile_sums<F><<<tiles, kScanThreads, 0, s>>>(f, n, sums);
-    GF_CHECK_LAUNCH();
-    if (tiles <= kScanDirectTiles) {
-        k_scan_tiles<F, false><<<tiles, kScanThreads, 0, s>>>(f, n, sums, total);
-    } else {
-        scan_sums(sums, tiles, total, s);
-        k_scan_tiles<F, true><<<tiles, kScanThreads, 0, s>>>(f, n, sums, nullptr);
-    }
-    GF_CHECK_LAUNCH();
+    auto go = [&](auto items) {
+        constexpr int kItems = decltype(items)::value;
+        const int tiles = div_up(n, kScanThreads * kItems);
+        k_scan_tile_sums<F, kItems><<<tiles, kScanThreads, 0, s>>>(f, n, sums);
+        GF_CHECK_LAUNCH();
+        if (tiles <= kScanDirectTiles) {
+            k_scan_tiles<F, kItems, false><<<tiles, kScanThreads, 0, s>>>(f, n, sums, total);
+        } else {
+            scan_sums(sums, tiles, total, s);
+            k_scan_tiles<F, kItems, true><<<tiles, kScanThreads, 0, s>>>(f, n, sums, nullptr);
+        }
+        GF_CHECK_LAUNCH();
+    };
+    if (div_up(n, kScanSmallTile) <= kScanDirectTiles)
+        go(std::integral_constant<int, kScanSmallItems>{});
+    else
+        go(std::integral_constant<int, kScanItems>{});
 }
 
 }  // namespace gf

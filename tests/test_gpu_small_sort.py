@@ -1,9 +1,8 @@
 """The one-launch bounding box, keys and sort of small sets: the tree equals the oracle's node for
 node (structure, particle order) at the edges of the split over the cluster's blocks (fewer
 particles than blocks, empty last blocks, uneven shares) and of the launch rules (28,672 particles
-and one more; 32,768 and one more for the scans that number nodes and groups; 147,456 and one more
-for the keys per thread of the larger sorts), with coincident points, points on cell walls and
-cells deeper than a key; and sets whose keys share their top 40 bits in runs just short enough for
+and one more; 147,456 and one more for the keys per thread of the larger sorts), with coincident
+points, points on cell walls and cells deeper than a key; and sets whose keys share their top 40 bits in runs just short enough for
 the insertion sort of the one launch, one longer, and in one run over several blocks."""
 
 import numpy as np
@@ -30,6 +29,12 @@ def test_small_sort_builds_the_same_tree(gpulib, oracle, n, kind):
     a, b = Engine().build_tree(x, m, 0.7), oracle.build_tree(x, m, 0.7)
     for f in ("start", "count", "next", "leaf", "order", "groups"):
         assert np.array_equal(a[f], b[f]), f
+
+
+@pytest.mark.parametrize("n", [16384, 16385, 524288, 524289])
+def test_scan_tiles_build_the_same_tree(gpulib, oracle, n):
+    """The most entries that the scans take in one launch and one per thread, and one more."""
+    test_small_sort_builds_the_same_tree(gpulib, oracle, n, "normal")
 
 
 @pytest.mark.parametrize("n", [31, 4097, 28672])
