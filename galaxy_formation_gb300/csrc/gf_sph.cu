@@ -328,7 +328,10 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
     const double dv = ei.s * dw;
 #pragma unroll
     for (int o = kLanes / 2; o; o >>= 1) mu_min = fmin(mu_min, __shfl_xor_sync(0xffffffffu, mu_min, o));
-    if (kLanes > 1) ok = (__ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1)) & ((1u << kLanes) - 1u)) == 0u;
+    if (kLanes > 1) {
+        const unsigned bad = __ballot_sync(0xffffffffu, !ok) >> (threadIdx.x & 31 & ~(kLanes - 1));
+        ok = (bad & ((1u << kLanes) - 1u)) == 0u;
+    }
     if (!on || s != 0) return;
     if (!ok) {
         raise_status(status, GF_ERR_ARG);

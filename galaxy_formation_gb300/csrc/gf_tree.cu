@@ -292,7 +292,8 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     const int first = rank * m;                   // this block's positions: [first, first + own)
     const int own = max(0, min(m, n - first));
     if (rank == 0)  // the build's counters start at zero (nothing uses them before the next launch)
-        for (int t = tid; t < int(sizeof(TreeCounts) / sizeof(int)); t += kSmallThreads) reinterpret_cast<int*>(counts)[t] = 0;
+        for (int t = tid; t < int(sizeof(TreeCounts) / sizeof(int)); t += kSmallThreads)
+            reinterpret_cast<int*>(counts)[t] = 0;
 
     if (tid == 0) s_found = 0;
     // bounding box of the block's share, then of all blocks (exact: min and max of integer images)

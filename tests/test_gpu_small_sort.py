@@ -2,8 +2,9 @@
 node (structure, particle order) at the edges of the split over the cluster's blocks (fewer
 particles than blocks, empty last blocks, uneven shares) and of the launch rules (28,672 particles
 and one more; 147,456 and one more for the keys per thread of the larger sorts), with coincident
-points, points on cell walls and cells deeper than a key; and sets whose keys share their top 40 bits in runs just short enough for
-the insertion sort of the one launch, one longer, and in one run over several blocks."""
+points, points on cell walls and cells deeper than a key; and sets whose keys share their top
+40 bits in runs just short enough for the insertion sort of the one launch, one longer, and in one
+run over several blocks."""
 
 import numpy as np
 import pytest
