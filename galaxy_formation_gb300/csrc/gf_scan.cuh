@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "gf_common.cuh"
 
@@ -62,6 +63,9 @@ __global__ void __cluster_dims__(kScanCtas, 1, 1) __launch_bounds__(kScanCluster
     k_scan_cluster(F f, int n, int m, int* __restrict__ total) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    // Another block's shared memory may be written only once that block runs: every block says so here
+    // and waits for the others before its first remote store, with its own values read in between.
+    auto running = cluster.barrier_arrive();
     __shared__ int s_warp[33], s_sums[kScanCtas];
     const int rank = int(cluster.block_rank());
     const int lo = rank * m, hi = min(n, lo + m);
@@ -78,6 +82,7 @@ __global__ void __cluster_dims__(kScanCtas, 1, 1) __launch_bounds__(kScanCluster
         ex[r] = sum + block_excl_scan(v[r], s_warp, &row);
         sum += row;
     }
+    cluster.barrier_wait(std::move(running));
     if (threadIdx.x < kScanCtas) *cluster.map_shared_rank(&s_sums[rank], int(threadIdx.x)) = sum;
     cluster.sync();
     int before = 0, all = 0;
