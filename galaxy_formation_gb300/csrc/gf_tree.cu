@@ -464,8 +464,12 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
             const unsigned c = __umulhi(unsigned(p), div_m);
             return cluster.map_shared_rank(vb + cur * m + (p - int(c) * m), c);
         };
-        unsigned starts = 0;  // bit s: a run of two or more starts at this thread's key s
-        int found = 0;        // 1: runs, 2: one too long
+        // four bits for each of this thread's keys: the length minus one of the run that starts there.
+        // (The insertion goes by it: the key after a run belongs to the next run's thread, which may
+        // be moving it.)
+        static_assert(kSmallRun == 16 && kSmallItems <= 8, "four bits per key");
+        unsigned lens = 0;
+        int found = 0;  // 1: runs, 2: one too long
         for (int s = 0; s < items; ++s) {
             const int p = first + tid + kSmallThreads * s;
             if (p >= first + own) break;
@@ -473,7 +477,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
             if (p > 0 && *key_at(p - 1) >> kSmallTopShift == top) continue;
             int len = 1;
             while (p + len < n && len <= kSmallRun && *key_at(p + len) >> kSmallTopShift == top) ++len;
-            if (len > 1) starts |= 1u << s;
+            lens |= unsigned(min(len, kSmallRun) - 1) << (4 * s);
             found |= len > kSmallRun ? 2 : len > 1 ? 1 : 0;
         }
         found = __reduce_or_sync(0xffffffffu, unsigned(found));
@@ -483,13 +487,10 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
         found = s_found;
         if (found & 2) continue;  // all eight digits after all
         if (!found) break;
-        for (int s = 0; starts >> s; ++s) {
-            if (!(starts >> s & 1u)) continue;
+        for (int s = 0; lens; ++s, lens >>= 4) {
             const int p = first + tid + kSmallThreads * s;
-            const uint64_t top = *key_at(p) >> kSmallTopShift;
-            for (int e = p + 1; e < n; ++e) {  // insertion, stable
+            for (int e = p + 1; e <= p + int(lens & 15u); ++e) {  // insertion, stable
                 const uint64_t k = *key_at(e);
-                if (k >> kSmallTopShift != top) break;
                 const int v = *val_at(e);
                 int q = e;
                 for (; q > p && *key_at(q - 1) > k; --q) {
