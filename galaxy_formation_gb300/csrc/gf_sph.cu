@@ -470,11 +470,11 @@ struct KnnArgs {
 // node is opened when it meets any of the spheres (a test against the queries' bounding box and
 // largest radius opens far too much where consecutive queries lie in cells apart: 10 ms instead of
 // 2 for the 1M disk's gas), and each point of an opened leaf is tested against every query. A query
-// with more than kKnnCap points is done with this radius: its sphere opens no further nodes
-// (S.cnt[i] then is only known to exceed kKnnCap). Returns false on stack overflow. The queries of a
+// with more than `enough` (>= kKnnCap) points is done with this radius: its sphere opens no further
+// nodes (S.cnt[i] then is only known to exceed that). Returns false on stack overflow. The queries of a
 // warp are neighbours in the tree's order (often in one leaf), so their walks share most nodes.
 template <int kQ>
-__device__ bool knn_collect(const KnnArgs& A, KnnSmem<kQ>& S, unsigned live, int leaf) {
+__device__ bool knn_collect(const KnnArgs& A, KnnSmem<kQ>& S, unsigned live, int leaf, int enough) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
     int cnt[kQ] = {};
@@ -572,7 +572,7 @@ __device__ bool knn_collect(const KnnArgs& A, KnnSmem<kQ>& S, unsigned live, int
             }
             unsigned full = 0;
 #pragma unroll
-            for (int i = 0; i < kQ; ++i) full |= cnt[i] > kKnnCap ? 1u << i : 0u;
+            for (int i = 0; i < kQ; ++i) full |= cnt[i] > enough ? 1u << i : 0u;
             live &= ~full;
             if (!live) break;
         }
@@ -837,16 +837,23 @@ __device__ __forceinline__ float knn_shrunk_radius(const unsigned long long* key
     return fminf(knn_rank_radius<kPer>(b, k + kKnnShrink), 0.9f * R);
 }
 
-// Radius step of the count-to-k iteration: Newton on count ~ R^3 below k, a rank of the
-// collected distances above the cap, until the count is bracketed; bisection afterwards.
-__device__ __forceinline__ float knn_next_radius(float R, int cnt, int k, const unsigned long long* key, float& lo,
-                                                 float& hi) {
+// Walks of a search that stop at kKnnCap points. A radius from the points of such a walk may be as
+// little as a tenth smaller (the first points met can all lie at the rim), so a start far too large, the
+// previous h of a set that has collapsed since, could use up all the walks: from then on a walk counts
+// every point in the sphere, and the count itself gives the step.
+constexpr int kKnnStopWalks = 12;
+
+// Radius step of the count-to-k iteration: Newton on count ~ R^3 below k and, with the whole count
+// (counted), above the cap; else a rank of the collected distances; bisection once it is bracketed.
+__device__ __forceinline__ float knn_next_radius(float R, int cnt, bool counted, int k, const unsigned long long* key,
+                                                 float& lo, float& hi) {
     if (cnt < k)
         lo = R;
     else
         hi = R;
     if (lo > 0.f && hi < INFINITY) return 0.5f * (lo + hi);
     if (cnt < k) return R * (cnt >= 4 ? cbrtf(1.3f * float(k) / float(cnt)) : 2.0f);
+    if (counted) return R * cbrtf(0.75f * float(kKnnCap) / float(cnt));
     return knn_shrunk_radius(key, k, R);
 }
 
@@ -888,7 +895,9 @@ __global__ void __launch_bounds__(kWarps * 32, 32 / kWarps) k_knn(KnnArgs A) {
                                       : knn_cell_radius(A, q0 + i));
         __syncwarp();
         while (on) {
-            const bool ok_walk = knn_collect<kQ>(A, S, on, A.leaf_of[q0 + __ffs(on) - 1]);
+            const bool counted = walks >= kKnnStopWalks;
+            const bool ok_walk =
+                knn_collect<kQ>(A, S, on, A.leaf_of[q0 + __ffs(on) - 1], counted ? INT_MAX : kKnnCap);
             total += __popc(on);
             ++walks;
             for (int i = 0; i < nq; ++i) {
@@ -900,7 +909,7 @@ __global__ void __launch_bounds__(kWarps * 32, 32 / kWarps) k_knn(KnnArgs A) {
                     on &= ~(1u << i);
                 } else if (ok_walk && walks < 48) {
                     float lo = S.q[i].lo, hi = S.q[i].hi;
-                    const float next = knn_next_radius(R, cnt, k, S.key[i], lo, hi);
+                    const float next = knn_next_radius(R, cnt, counted, k, S.key[i], lo, hi);
                     __syncwarp();
                     if (lane == 0) {
                         S.q[i].lo = lo;
