@@ -153,11 +153,13 @@ __device__ __forceinline__ double w_shape64(double q) {
     return below_2(q) ? w : 0.0;
 }
 
-// -4/3 dW/dq without its 1/(pi h^4) (sph.py:43-54): q (4 - 3 q), or (2 - q)^2
+// -4/3 dW/dq without its 1/(pi h^4) (sph.py:43-54): q (4 - 3 q), or (2 - q)^2 (0 outside the support,
+// also where q is infinite)
 __device__ __forceinline__ double dw_shape64(double q) {
     const bool in = below_1(q);
     const double l = fma(in ? -3.0 : -1.0, q, in ? 4.0 : 2.0);
-    return (in ? q : below_2(q) ? l : 0.0) * l;
+    const double p = (in ? q : l) * l;
+    return below_2(q) ? p : 0.0;
 }
 
 template <int kLanes>

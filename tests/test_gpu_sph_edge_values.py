@@ -1,0 +1,47 @@
+"""The float64 SPH passes on values outside the ordinary range, with each number of lanes per particle
+(eight, four, two, one by the particle count): what one such particle does to the others' results.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = (600, 20000, 200000, 300000)
+ODD = 100  # the particle that is out of the ordinary
+
+
+def _set(n, k=7):
+    rng = np.random.default_rng(n)
+    nb = np.ascontiguousarray((np.arange(n)[:, None] + np.arange(k)[None, :]) % n, np.int64)
+    return {"pos": rng.normal(size=(n, 3)), "vel": rng.normal(size=(n, 3)), "mass": rng.uniform(0.5, 1.5, n) / n,
+            "nb": nb, "h": rng.uniform(0.3, 3.0, n), "u": rng.uniform(0.1, 10.0, n)}
+
+
+def _forces(d):
+    from galaxy_formation_gb300 import sph
+
+    n = len(d["mass"])
+    rho, acc, dudt, dt = np.empty(n), np.empty((n, 3)), np.empty(n), np.empty(n)
+    sph.sph_forces(d["pos"], d["vel"], d["mass"], d["nb"], d["h"], d["u"], 5.0 / 3.0, 1.0, 2.0, rho, acc, dudt, dt)
+    return {"rho": rho, "acc": acc, "dudt": dudt, "dt": dt}
+
+
+def _with(d, **changes):
+    out = {key: val.copy() for key, val in d.items()}
+    for key, val in changes.items():
+        out[key][ODD] = val
+    return out
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("distance", [1e150, 1e160, 1e200])
+def test_a_neighbour_whose_squared_distance_overflows(gpulib, n, distance):
+    """Outside both supports and receding, it adds zero to every sum, like one far enough for that at an
+    ordinary distance: the same bits."""
+    d = _set(n)
+    near = _forces(_with(d, pos=[1e6, 0, 0], vel=[1e3, 0, 0]))
+    far = _forces(_with(d, pos=[distance, 0, 0], vel=[1e3, 0, 0]))
+    for key in near:
+        assert np.isfinite(near[key]).all()
+        assert np.array_equal(far[key], near[key]), key
