@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
     // give du/dt (pressure and viscous part) and the velocity divergence; the most negative mu / 10.
     // With P the kernel gradient's shape (times s), A = s P/rho^2 and half_visc half the pair's
     // viscosity: V = half_visc (s_i P_i + s_j P_j), and the pair's force is m (A_i P_i + A_j P_j + V) d / r.
-    double ax = 0, ay = 0, az = 0, dw = 0, hv = 0, mu_min = 0;
+    double ax = 0, ay = 0, az = 0, dw = 0, hv = 0, mu_min = -0.0;
     PairEos ei{0, 0, 0, 0};
     if (on) {
         const double4_32a p = src.xm(i), v = src.vh(i);
@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
                     xr = x / rs;
                 }
                 const double half_visc = fma(beta100, x, -(ei.ca + ej.ca)) * xr;
-                // of negative numbers the smallest has the largest bits (above those of -inf: NaN)
+                // Of negative numbers the smallest has the largest bits: from those of -0 on, up to those of
+                // -inf. Positive values (a negative hb) and NaN of either sign lie outside.
                 const uint64_t xb = uint64_t(__double_as_longlong(x));
                 if (xb > uint64_t(__double_as_longlong(mu_min)) && xb <= 0xfff0000000000000ull) mu_min = x;
                 const double V = half_visc * fma(ej.s, Pj, ei.s * Pi);

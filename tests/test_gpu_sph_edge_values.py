@@ -45,3 +45,20 @@ def test_a_neighbour_whose_squared_distance_overflows(gpulib, n, distance):
     for key in near:
         assert np.isfinite(near[key]).all()
         assert np.array_equal(far[key], near[key]), key
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("h", [-2.9, -40.0])
+def test_the_courant_step_ignores_receding_and_odd_pairs(gpulib, n, h):
+    """Only a negative mu counts: with a negative smoothing length the approaching pairs have a positive
+    one, whatever the number of lanes. Each rounding of the step is within 2^-53, fewer than 50 of them."""
+    d = _with(_set(n), h=h)
+    dt = _forces(d)["dt"][ODD]
+    gamma, j = 5.0 / 3.0, d["nb"][ODD, 1:]
+    dx = d["pos"][ODD] - d["pos"][j]
+    vr = ((d["vel"][ODD] - d["vel"][j]) * dx).sum(1)
+    hb = 0.5 * (h + d["h"][j])
+    mu = np.where(vr < 0, hb * vr / ((dx * dx).sum(1) + 0.01 * hb * hb), 0.0)
+    c = np.sqrt(gamma * (gamma - 1) * d["u"][ODD])
+    want = 0.3 * h / (2.2 * c + 1.2 * 2.0 * max(0.0, (-mu).max()))
+    assert abs(dt - want) <= 1e-14 * abs(want)
