@@ -141,9 +141,14 @@ struct PlainSrc {
     __device__ __forceinline__ double sound(int64_t j) const { return cs[j]; }
 };
 
-// q < 1 and q < 2 on the upper word of a float64 (NaN and negative values are neither)
-__device__ __forceinline__ bool below_1(double q) { return unsigned(__double2hiint(q)) < 0x3ff00000u; }
-__device__ __forceinline__ bool below_2(double q) { return unsigned(__double2hiint(q)) < 0x40000000u; }
+// q < 1 and q < 2 on the upper word of a float64. Negative values (a negative h) are below both, as for
+// the comparison of the values; a NaN of either sign and -infinity are below neither.
+__device__ __forceinline__ bool below_word(double q, int word) {
+    const int w = __double2hiint(q);
+    return w < word && unsigned(w) < 0xfff00000u;
+}
+__device__ __forceinline__ bool below_1(double q) { return below_word(q, 0x3ff00000); }
+__device__ __forceinline__ bool below_2(double q) { return below_word(q, 0x40000000); }
 
 // M4 kernel without its 1/(pi h^3) (sph.py:31-40): 1 - 3/2 q^2 + 3/4 q^3, or (2 - q)^3 / 4
 __device__ __forceinline__ double w_shape64(double q) {

@@ -62,3 +62,38 @@ def test_the_courant_step_ignores_receding_and_odd_pairs(gpulib, n, h):
     c = np.sqrt(gamma * (gamma - 1) * d["u"][ODD])
     want = 0.3 * h / (2.2 * c + 1.2 * 2.0 * max(0.0, (-mu).max()))
     assert abs(dt - want) <= 1e-14 * abs(want)
+
+
+def _rows_of(d):
+    """The rows that hold ODD, and no other particle's: those whose results it can change."""
+    return np.flatnonzero((d["nb"] == ODD).any(axis=1))
+
+
+def _close_to_numpy(d, got, rows):
+    """Within 1e-13 of the terms' scales of NumPy's restatement (test_gpu_sph_lanes derives both)."""
+    from test_gpu_sph_lanes import _reference
+
+    with np.errstate(all="ignore"):
+        rho, acc, s_acc, dudt, s_dudt, dt = _reference(*(d[key] for key in ("pos", "vel", "mass", "nb", "h", "u")))
+    for key, want, size in (("rho", rho, np.abs(rho)), ("acc", acc, np.abs(s_acc)), ("dudt", dudt, np.abs(s_dudt)),
+                            ("dt", dt, np.abs(dt))):
+        assert np.all(np.abs(got[key] - want)[rows] <= 1e-13 * size[rows]), key
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("h", [-0.7, -2.9, -40.0])
+def test_a_negative_smoothing_length(gpulib, n, h):
+    """The kernels of sph.py:31-54 take the branch of q < 1 for it; so do the passes here."""
+    d = _with(_set(n), h=h)
+    _close_to_numpy(d, _forces(d), _rows_of(d))
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("nan", [np.nan, -np.nan])
+def test_a_smoothing_length_that_is_no_number(gpulib, n, nan):
+    """Its own density is 0 (no pair is inside its support); the others' densities stay."""
+    d = _set(n)
+    got, plain = _forces(_with(d, h=nan)), _forces(d)
+    assert got["rho"][ODD] == 0.0
+    others = np.arange(n) != ODD
+    assert np.array_equal(got["rho"][others], plain["rho"][others])
