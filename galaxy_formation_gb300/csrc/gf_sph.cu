@@ -89,8 +89,9 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
 // kLanes lanes share a particle's row: without them a lone warp works through 32 neighbours one
 // after another, and small sets leave most of the chip idle.
 
-// The kernel gradient's normalisation -3 / (4 pi h^4) (sph.py:43-54).
-__device__ __forceinline__ double grad_norm(double h) { return -0.75 / (kPi * h * h * h * h); }
+// The kernel gradient's normalisation -3 / (4 pi h^4) (sph.py:43-54). It stays finite where h^4
+// underflows (h below 2e-77): it is multiplied by shapes that are zero outside the support.
+__device__ __forceinline__ double grad_norm(double h) { return -0.75 / fmax(kPi * h * h * h * h, 4.2e-309); }
 
 // Threads per block: small blocks even out the last wave of the small launches.
 template <int kLanes>

@@ -97,3 +97,20 @@ def test_a_smoothing_length_that_is_no_number(gpulib, n, nan):
     assert got["rho"][ODD] == 0.0
     others = np.arange(n) != ODD
     assert np.array_equal(got["rho"][others], plain["rho"][others])
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("h", [1e-70, 1e-76, 1e-77, 1e-80])
+def test_a_smoothing_length_whose_fourth_power_underflows(gpulib, n, h):
+    """The normalisation of its gradient is beyond float64; its neighbours lie outside its support."""
+    d = _with(_set(n), h=h)
+    _close_to_numpy(d, _forces(d), _rows_of(d))
+
+
+@pytest.mark.parametrize("n", COUNTS)
+def test_a_smoothing_length_of_zero(gpulib, n):
+    """Its density is zero; the heating of the others does not see its pressure and stays a number."""
+    d = _with(_set(n), h=0.0)
+    got = _forces(d)
+    assert got["rho"][ODD] == 0.0
+    assert np.isfinite(got["dudt"][np.arange(n) != ODD]).all()
