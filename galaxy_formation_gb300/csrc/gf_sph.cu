@@ -21,6 +21,7 @@
 //                              in float64 and sorted again, so the result is the exact
 //                              float64 kNN.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -92,6 +93,12 @@ __global__ void k_sph_kernel(int n, const double* __restrict__ r, const double* 
 // The kernel gradient's normalisation -3 / (4 pi h^4) (sph.py:43-54). It stays finite where h^4
 // underflows (h below 2e-77): it is multiplied by shapes that are zero outside the support.
 __device__ __forceinline__ double grad_norm(double h) { return -0.75 / fmax(kPi * h * h * h * h, 4.2e-309); }
+
+// 1/h for q = r (1/h), finite for any h but 0: a particle's own q is 0 also where h is subnormal.
+__device__ __forceinline__ double inv_length(double h) {
+    const double y = 1.0 / h;
+    return h != 0.0 && fabs(y) > DBL_MAX ? copysign(DBL_MAX, y) : y;
+}
 
 // Threads per block: small blocks even out the last wave of the small launches.
 template <int kLanes>
@@ -205,7 +212,7 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_density(int n, int 
     if (on) {
         const double4_32a p = src.xm(i);
         hi = h[i];
-        const double inv_h = 1.0 / hi;
+        const double inv_h = inv_length(hi);
         const Idx* row = nb + size_t(i) * ld;
 #pragma unroll 4
         for (int jj = s; jj < k; jj += kLanes) {

@@ -114,3 +114,14 @@ def test_a_smoothing_length_of_zero(gpulib, n):
     got = _forces(d)
     assert got["rho"][ODD] == 0.0
     assert np.isfinite(got["dudt"][np.arange(n) != ODD]).all()
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("h", [1e-309, 1e-310, 5e-324])
+def test_a_subnormal_smoothing_length(gpulib, n, h):
+    """W(0, h) of sph.py:31-40 is then infinite, and with it the particle's own density."""
+    d = _set(n)
+    got, plain = _forces(_with(d, h=h)), _forces(d)
+    assert got["rho"][ODD] == np.inf
+    others = np.arange(n) != ODD
+    assert np.array_equal(got["rho"][others], plain["rho"][others])
