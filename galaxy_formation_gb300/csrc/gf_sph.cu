@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_density(int n, int 
             const double4_32a q = src.xm(j);
             const double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const double r = j != i ? root(r2) : 0.0;
+            const double r = j != i ? root(r2) : r2;  // r2 of itself: 0, or NaN of such a position
             sum = fma(q.w, w_shape64(r * inv_h), sum);
         }
     }

@@ -125,3 +125,15 @@ def test_a_subnormal_smoothing_length(gpulib, n, h):
     assert got["rho"][ODD] == np.inf
     others = np.arange(n) != ODD
     assert np.array_equal(got["rho"][others], plain["rho"][others])
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("x", [np.nan, -np.nan, np.inf, -np.inf])
+def test_a_position_that_is_no_number(gpulib, n, x):
+    """Its distances are no numbers either, that to itself included: density zero. The others' densities
+    are as if it were far away."""
+    d = _set(n)
+    got, far = _forces(_with(d, pos=[x, 0, 0])), _forces(_with(d, pos=[1e6, 0, 0]))
+    assert got["rho"][ODD] == 0.0
+    others = np.arange(n) != ODD
+    assert np.array_equal(got["rho"][others], far["rho"][others])
