@@ -65,6 +65,8 @@ __device__ RootBox root_box(const double (&tot)[6], double theta) {
     // 0.5 * max extent * 1.0001 + 1e-12 (cpp/nbody.cpp:219), unfused
     R.half = __dadd_rn(__dmul_rn(__dmul_rn(0.5, ext), 1.0001), 1e-12);
     R.open0 = __ddiv_rn(__dmul_rn(2.0, R.half), theta);
+    // (theta infinite: a node's first term is scaled down from this one by its exponent, which 0 lacks)
+    if (R.open0 == 0.0) R.open0 = ldexp(1.0, -900);
     double cmax = 0;
     for (int a = 0; a < 3; ++a) {
         R.lo[a] = __dsub_rn(R.c[a], R.half);
