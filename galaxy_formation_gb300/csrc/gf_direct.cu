@@ -23,14 +23,15 @@ constexpr int kDirThreads = 64;
 constexpr int kDirParts = 8;  // blocks per cluster: source parts
 
 // m r2^(-3/2). The seed y of 1/sqrt(r2) has e = 1 - r2 y^2 of about 2^-20, and (1 - e)^(-3/2) =
-// 1 + 3/2 e + 15/8 e^2 + ...: the next term is below rounding.
+// 1 + 3/2 e + 15/8 e^2 + ...: the next term is below rounding. (The mass comes last: with an infinite one
+// the series' corrections would cancel.)
 __device__ __forceinline__ double pair_factor(double r2, double m) {
     if (exponent_of(r2) - 423u < 1200u) {  // 2^-600 <= r2 < 2^600: r2^(-3/2) is a normal number
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
         const double e = fma(-(r2 * y), y, 1.0);
-        const double g = m * (y * y * y);
-        return fma(g * e, fma(1.875, e, 1.5), g);
+        const double g = y * y * y;
+        return m * fma(g * e, fma(1.875, e, 1.5), g);
     }
     return m / (r2 * sqrt(r2));
 }
