@@ -978,21 +978,22 @@ void sph_kernel_values(int n, const double* r, const double* h, double* w, doubl
     GF_CHECK_LAUNCH();
 }
 
-// The two float64 passes with L lanes per particle, on any neighbour source.
+// The two float64 passes with L lanes per particle, on any neighbour source. timed: as stages of the
+// profiler, which creates events and keeps them.
 template <class Idx, int L, class Src>
 void sph_launch(int n, int k, int ld, const Src& src, const int* order, const Idx* nb, const double* h,
                 const double* u, double gamma, double alpha, double beta, double* rho, SphRec* rec, double* pr2,
                 double* cs, double* acc, double* dudt, double* dt_i, cudaStream_t s, float* divv, Subset sub,
-                uint32_t* status) {
+                uint32_t* status, bool timed) {
     constexpr int threads = kSphThreads<L>;
     const int grid = div_up((long long)n * L, threads);
     {
-        ProfScope ps(kStSphDensity, s);
+        ProfScope ps(timed ? kStSphDensity : -1, s);
         k_sph_density<Idx, L><<<grid, threads, 0, s>>>(n, k, ld, src, order, nb, h, u, gamma, 5.0 * alpha, rho, rec,
                                                         pr2, cs, sub, status);
         GF_CHECK_LAUNCH();
     }
-    ProfScope ps(kStSphForce, s);
+    ProfScope ps(timed ? kStSphForce : -1, s);
     k_sph_force<Idx, L><<<grid, threads, 0, s>>>(n, k, ld, src, order, nb, h, alpha, beta, acc, dudt, dt_i, divv,
                                                   sub, status);
     GF_CHECK_LAUNCH();
@@ -1018,7 +1019,8 @@ void sph_forces(SphScratch& S, int n, int k, int ld, const int* order, const dou
     GF_CHECK_LAUNCH();
     auto go = [&](auto lanes) {
         sph_launch<Idx, decltype(lanes)::value>(n, k, ld, PackedSrc{rec}, order, nb, h, u, gamma, alpha, beta, rho,
-                                                rec, nullptr, nullptr, acc, dudt, dt_i, s, divv, sub, ctx().d_status);
+                                                rec, nullptr, nullptr, acc, dudt, dt_i, s, divv, sub, ctx().d_status,
+                                                true);
     };
     if (!sub.idx && n <= kSphEightLanes)
         go(std::integral_constant<int, 8>());
@@ -1249,7 +1251,7 @@ extern "C" int gf_sph_forces_noalloc_dev(int n, int k, const double* pos, const 
     try {
         sph_launch<int64_t, 4>(n, k, k, PlainSrc{pos, vel, mass, h, rho, pr2, cs, 5.0 * alpha}, nullptr, nb, h, u,
                                gamma, alpha, beta, rho, nullptr, pr2, cs, acc, dudt, dt_i, s, nullptr, Subset(),
-                               nullptr);
+                               nullptr, false);
     } catch (const Error& err) {
         return noalloc_fail(err.code, err.what());
     }
