@@ -64,6 +64,9 @@ struct DevBuf {
     }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
+    // How many T fit (0 after a failed growth).
+    template <class T>
+    size_t holds() const { return bytes / sizeof(T); }
     void release() {
         if (p) cudaFree(p);
         p = nullptr;

@@ -1516,8 +1516,10 @@ void Octree::build(int n_, const double* pos, const double* mass, double theta, 
         radix_sort_pairs(k0, pm, key_alt.as<uint64_t>(), perm_alt.as<int>(), n, 0, 63, s, &scratch);
     }
 
+    // The owners' bound is the buffer's own size: node_cap is raised before the node buffers grow, and
+    // a growth that fails leaves it above what they hold.
     StartScan starts{KeyView{k0, nullptr, nullptr}, n, leaf_max, ldepth.get<int8_t>(n), dsplit.get<int8_t>(n), nb,
-                     node_owner.as<int>(), node_owner.p ? node_cap : 0, cnt};
+                     node_owner.as<int>(), int(std::min(size_t(node_cap), node_owner.holds<int>())), cnt};
     // Deep cells (> 8 particles in one level-21 cell) need extension keys. A regular build
     // finds out on the host; a captured one always computes them (zero outside deep runs,
     // where they leave every common-prefix length the tree uses unchanged).
