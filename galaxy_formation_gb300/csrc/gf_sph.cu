@@ -353,6 +353,12 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
         ok = (bad & ((1u << kLanes) - 1u)) == 0u;
     }
     if (!on || s != 0) return;
+    if (fabs(ei.sp) > DBL_MAX || ei.sp != ei.sp) {  // no number times an empty sum: a particle alone is not heated
+        const Idx* row = nb + size_t(i) * ld;
+        bool alone = true;
+        for (int jj = 0; jj < k; ++jj) alone = alone && row[jj] == i;
+        if (alone) du = 0.0;
+    }
     if (!ok) {
         raise_status(status, GF_ERR_ARG);
         ax = ay = az = du = nan64();
