@@ -168,7 +168,7 @@ constexpr int kRsWarps = kRsThreads / 32;
 // Keys per thread: 8, or 4 up to kOsFewKeys keys, where a tile's own latency counts and tiles of
 // 2048 would leave SMs idle. Eight passes with 4 / 8 / 16 per thread: 60k keys 76 / 88 / 115 us, 100k
 // 76 / 93 / 122, 200k 104 / 92 / 125, 1M 252 / 208 / 199, 4M 742 / 572 / 613.
-constexpr int kOsMinItems = 4;
+constexpr int kOsItems = 8, kOsMinItems = 4;
 constexpr int kOsFewKeys = 144 * 1024;
 constexpr int kOsMaxPasses = 8;
 constexpr unsigned kOsAgg = 1u << 30;         // look-back flags: the tile's own count,
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kRsThreads) k_os_hist(const uint64_t* __restri
 }
 
 // One pass: tiles in ticket order; status[tile * 256 + d] holds the flag and value of digit d.
-template <int kOsItems>
+template <int kItems>
 __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     const uint64_t* __restrict__ kin, const int* __restrict__ vin, uint64_t* __restrict__ kout,
     int* __restrict__ vout, int n, int shift, const int* __restrict__ tot, unsigned* __restrict__ status,
@@ -202,8 +202,8 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     __shared__ int s_base[256];
     __shared__ int s_warp[33];
     __shared__ int s_tile;
-    constexpr int kOsWarpItems = 32 * kOsItems;  // consecutive keys per warp
-    constexpr int kOsTile = kRsThreads * kOsItems;
+    constexpr int kOsWarpItems = 32 * kItems;  // consecutive keys per warp
+    constexpr int kOsTile = kRsThreads * kItems;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1);
     for (int w = 0; w < kRsWarps; ++w) s_cnt[w][threadIdx.x] = 0;
@@ -211,19 +211,19 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     const int gbase = block_excl_scan(tot[threadIdx.x], s_warp, nullptr);  // synchronises
     const int tile = s_tile;
     const int base = tile * kOsTile + warp * kOsWarpItems;
-    uint64_t k[kOsItems];
-    int v[kOsItems];
-    int rank[kOsItems];
+    uint64_t k[kItems];
+    int v[kItems];
+    int rank[kItems];
     const unsigned lt = lanemask_lt();
 #pragma unroll
-    for (int s = 0; s < kOsItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         const int i = base + s * 32 + lane;
         const bool ok = i < n;
         k[s] = ok ? kin[i] : 0ull;
         v[s] = ok ? vin[i] : 0;
     }
 #pragma unroll
-    for (int s = 0; s < kOsItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         const int i = base + s * 32 + lane;
         const bool ok = i < n;
         const unsigned d = ok ? unsigned((k[s] >> shift) & 255u) : 256u;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     s_base[d] = gbase + excl;
     __syncthreads();
 #pragma unroll
-    for (int s = 0; s < kOsItems; ++s) {
+    for (int s = 0; s < kItems; ++s) {
         const int i = base + s * 32 + lane;
         if (i < n) {
             const unsigned dg = unsigned((k[s] >> shift) & 255u);
@@ -291,10 +291,12 @@ __global__ void __launch_bounds__(kRsThreads) k_os_pass(
     }
 }
 
-// Scratch of a one-sweep sort of n pairs: digit totals [8][256], tickets [8], tile status
-// [8][tiles][256].
+// Scratch of one-sweep sorts of up to n pairs: digit totals [8][256], tickets [8], tile status
+// [8][tiles][256], the tiles those of n pairs or of the largest sort with small tiles.
 size_t os_scratch_ints(int n) {
-    const size_t tiles = size_t(div_up(std::max(n, 1), kRsThreads * kOsMinItems));
+    n = std::max(n, 1);
+    const size_t tiles = size_t(std::max(div_up(std::min(n, kOsFewKeys), kRsThreads * kOsMinItems),
+                                         div_up(n, kRsThreads * kOsItems)));
     return size_t(kOsMaxPasses) * 256 + 64 + size_t(kOsMaxPasses) * tiles * 256;
 }
 
@@ -310,7 +312,7 @@ void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_a
     if (n > int(kOsValue)) throw Error(GF_ERR_CAPACITY, "radix sort of more than 2^30 - 1 keys");
     const int npass = div_up(bit_hi - bit_lo, 8);
     if (npass < 1 || npass > kOsMaxPasses) throw Error(GF_ERR_ARG, "radix sort bit range");
-    const int items = n <= kOsFewKeys ? kOsMinItems : 8;
+    const int items = n <= kOsFewKeys ? kOsMinItems : kOsItems;
     const int tiles = div_up(n, kRsThreads * items);
     int* hist = (sc ? sc->sort_tmp : g_ctx.sort_tmp).get<int>(os_scratch_ints(n));
     int* tickets = hist + kOsMaxPasses * 256;
@@ -330,7 +332,7 @@ void radix_sort_pairs(uint64_t* keys, int* vals, uint64_t* keys_alt, int* vals_a
         if (items == kOsMinItems)
             pass(k_os_pass<kOsMinItems>);
         else
-            pass(k_os_pass<8>);
+            pass(k_os_pass<kOsItems>);
         GF_CHECK_LAUNCH();
         std::swap(ka, kb);
         std::swap(va, vb);
