@@ -169,8 +169,9 @@ __device__ __forceinline__ int pop_round(int* stack, int& sp, int (&node)[NPL]) 
 __device__ __forceinline__ unsigned exponent_of(double x) { return unsigned(__double2hiint(x)) >> 20; }
 
 // r and 1/r of r2 >= 0 (1/r capped at 1e30). y, the hardware's approximation of 1/sqrt(r2), has
-// e = 1 - r2 y^2 of about 2^-20; the roots are r2 y and y times (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 + ...,
-// each rounded once at the end.
+// e = 1 - r2 y^2 of about 2^-20; the roots are r2 y and y times (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 + ...
+// (the binomial series, a Householder step of third order). Within a unit in the last place: half from the
+// last rounding, a quarter to half from that of r2 y.
 __device__ __forceinline__ void inv_root(double r2, double& r, double& inv_r) {
     if (exponent_of(r2) - 825u < 1160u) {  // 2^-198 <= r2 < 2^962
         double y;
@@ -198,7 +199,10 @@ __device__ __forceinline__ double root(double r2) {
     return sqrt(r2);
 }
 
-// 1/x of a normal x far from the ends of the range: seed y with e = 1 - x y, y (1 + e + e^2 + ...).
+// 1/x of an x in that range (neither zero, negative, subnormal, infinite nor NaN): seed y with
+// e = 1 - x y, y (1 + e + e^2 + ...).
+__device__ __forceinline__ bool in_inverse_range(double x) { return exponent_of(x) - 123u < 1800u; }  // 2^-900..2^900
+
 __device__ __forceinline__ double inverse(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
                 const double den = fma(hs, hs, r2), rs = rhoi + src.rho(j);
                 const double prod = den * rs;
                 double x, xr;  // mu / 10, and that over rs
-                if (exponent_of(prod) - 123u < 1800u) {
+                if (in_inverse_range(prod)) {
                     xr = num * inverse(prod);
                     x = xr * rs;
                 } else {

@@ -1082,7 +1082,7 @@ struct Moments64Args {
 
 // 1/M of a node's mass (0 for a massless node).
 __device__ __forceinline__ double inverse_mass(double M) {
-    return exponent_of(M) - 123u < 1800u ? inverse(M) : M > 0 ? __drcp_rn(M) : 0.0;
+    return in_inverse_range(M) ? inverse(M) : M > 0 ? __drcp_rn(M) : 0.0;
 }
 
 // open_r of a node whose centre of mass lies at squared distance o2 from its cell's centre.
