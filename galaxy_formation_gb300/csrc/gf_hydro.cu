@@ -715,6 +715,10 @@ void ForceEngine::hydro(const ForceArgs& a, cudaStream_t s) {
     if (!have_nb) {  // full search, 48 candidates (sph.py:165-169), written into the cache
         vsel_ = vsel.get<int>(ng);  // the neighbour that fixes each h (k_smoothing measures it)
         const int kq = std::min(kCand, ng);
+        // a search that throws half way leaves neither a cache nor a visiting order behind
+        const bool same_gas = order_ng == ng;
+        cache_valid = false;
+        order_ng = -1;
         nb = cache.get<int>(size_t(ng) * kCand);
         float* rg = nullptr;
         if (have_hprev && (hguess == 0 || hguess == 2)) {  // previous h
@@ -732,7 +736,7 @@ void ForceEngine::hydro(const ForceArgs& a, cudaStream_t s) {
         GF_CUDA(cudaMemsetAsync(&sc->knn_iters, 0, sizeof(unsigned long long), s));
         // the gas of the last full search, moved (same count): rebuild without a host round trip
         knn_exact(knn_tree, ng, gp, kq, rg, nullptr, nullptr, &sc->knn_iters, s, nb, kCand, d31, kNgb - 1,
-                  features ? &hg : nullptr, order_ng == ng, vsel_, hguess == 1);
+                  features ? &hg : nullptr, same_gas, vsel_, hguess == 1);
         if (collect) {
             const long long take = std::min<long long>(ng, (collect_cap - collect_n) / 2);  // two rows each
             if (take > 0) {
