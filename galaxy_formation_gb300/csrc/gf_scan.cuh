@@ -172,7 +172,7 @@ void scan_with(const F& f, int n, int* total, cudaStream_t s, ScanScratch* sc) {
         GF_CHECK_LAUNCH();
         if (tiles <= kScanDirectTiles) {
             k_scan_tiles<F, kItems, false><<<tiles, kScanThreads, 0, s>>>(f, n, sums, total);
-        } else {
+        } else if constexpr (kItems == kScanItems) {  // (the small tiles are taken while they are that few)
             scan_sums(sums, tiles, total, s);
             k_scan_tiles<F, kItems, true><<<tiles, kScanThreads, 0, s>>>(f, n, sums, nullptr);
         }

@@ -385,8 +385,6 @@ __global__ void __launch_bounds__(kSphThreads<kLanes>) k_sph_force(int n, int k,
                                                                                   // (a feature of the h guess)
 }
 
-// ------------------------------------------------------------------- warp bitonic sorts
-
 // --------------------------------------------------------------- knn_from_candidates
 
 constexpr int kCandWarps = 8;

@@ -20,10 +20,11 @@
 //      depth-first order, and `next` is the id of the first node starting after the cell.
 //      Cells that still hold > 8 particles at level 21 get extension keys (levels 22..48,
 //      exact chain) and are re-sorted in shared memory.
-//   5. leaves re-sorted by index (the reference never partitions a leaf).
-//   6. moments bottom-up in one launch (the last child to arrive computes its parent,
-//      children summed in octant order), float64 sums of the same terms as the reference,
-//      rounded to the same float32 node record.
+//   5. node emission, where a leaf's thread also puts its particles in index order (the
+//      reference never partitions a leaf).
+//   6. moments bottom-up in one launch (the last child to arrive completes its parent), float64
+//      sums of the same terms as the reference (a parent's first four children and its last four
+//      apart, then both), rounded to the same float32 node record.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -247,14 +248,14 @@ __global__ void k_keys(const double* __restrict__ pos, int n, const RootBox* __r
 
 // Bounding box, keys and their radix sort in one launch, for sets that fit the shared memory of one
 // cluster: kSmallCtas blocks hold m consecutive positions each; 8-bit passes rank the keys
-// as the one-sweep sort does (match-any per warp, warps in key order), add up the blocks' digit
+// as the one-sweep sort does (ballots per warp, warps in key order), add up the blocks' digit
 // counts through distributed shared memory and scatter keys and indices straight into the block
 // that holds their new position. Two cluster barriers a pass take the place of a launch, a digit
-// histogram and a look-back. A pass costs about 12,000 cycles at 10k keys, half of it barriers and
-// their latencies, and grows with the keys per block (match-any, scattered remote stores), so the
-// chain of 12 launches is as fast from about 28k keys on: Engine.gravity with the chain / with this
-// launch 325 / 267 us at 5k particles, 350 / 302 at 10k, 366 / 354 at 24k, 375 / 381 at 32k (blocks of
-// 512 threads instead of 1024, whose barriers are longer: 2 % faster builds).
+// histogram and a look-back. The launch's time grows with the keys per block (scattered remote
+// stores), where the chain of 12 launches hardly changes: 25 us at 2k keys, 39 at 10k and 70 at 28k,
+// against 75 for the chain's sort alone at 50k. Engine.gravity of 28,672 / 28,673 particles, the last count with
+// this launch and the first with the chain: 325 / 352 us. (Blocks of 512 threads instead of 1024,
+// whose barriers are longer: 2 % faster builds.)
 static_assert(kKeyLevels == 21, "eight 8-bit passes over a 63-bit key");
 constexpr int kSmallCtas = 8;
 constexpr int kSmallThreads = 512;
@@ -268,7 +269,8 @@ constexpr int kSmallMax = kSmallCtas * kSmallMaxPer;        // 28,672 particles
 // (coincident particles, cores 10^4 times smaller than the box) sends the whole set through all eight
 // digits. Engine.gravity of a 2k / 10k / 24k cloud with eight passes 154 / 226 / 268 us, with five
 // and the runs 150 / 217 / 253 (with four 148 / 213 / 246, but 385 instead of 325 us for a concentrated
-// 28k set whose core then takes all twelve); 10k in groups of 20, which take all thirteen, 457 -> 482.
+// 28k set whose core then takes all twelve). Such a set pays for both sorts, 63 instead of 39 us at 10k:
+// gravity of 10k / 28k particles in groups of 20 within 10^-6 396 / 469 us.
 constexpr int kSmallTopPasses = 5, kSmallTopShift = 63 - 8 * kSmallTopPasses, kSmallRun = 16;
 
 constexpr size_t small_sort_smem(int m) {
@@ -392,7 +394,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
             __syncwarp();
         }
         __syncthreads();
-        // four threads per digit: exclusive prefix over the warps; the block's count of every digit
+        // two threads per digit: exclusive prefix over the warps; the block's count of every digit
         // goes to all blocks
         const int d = tid & 255, part = tid >> 8;
         constexpr int kParts = kSmallThreads / 256, kPart = kSmallWarps / kParts;
@@ -627,8 +629,8 @@ __device__ int run_begin(const KeyView& K, int i, int lev) {
 // ---------------------------------------------------------------------------- emit
 
 // Node emission, one thread per node. Position i starts the nodes of depths ds[i] .. ld[i]
-// (ids nbase[i] ..); k_node_owner writes, for every node id, the position that starts it, and
-// k_emit fills the node: the cube centre by the float64 halving chain from the root along
+// (ids nbase[i] ..); the scan that numbers the nodes writes, for every node id, the position that
+// starts it (k_node_owner again, after the node buffers have grown), and k_emit fills the node: the cube centre by the float64 halving chain from the root along
 // i's octant digits (cpp/nbody.cpp:92-96), the particle range [i, end) with end the first
 // position whose prefix leaves the node's, `next` = the first node starting at end, the leaf
 // flag and the parent (the previous node of the chain, or the deepest node at depth d - 1 of
@@ -637,7 +639,7 @@ __device__ int run_begin(const KeyView& K, int i, int lev) {
 // A leaf's thread also puts its particles in increasing index order (the reference's stable
 // partitions never reorder a leaf), the nodes of each depth are counted for the breadth-first
 // numbering, and that pass's look-back statuses are cleared.
-__global__ void k_node_owner(int n, StartScan S) {  // after the node buffers have grown
+__global__ void k_node_owner(int n, StartScan S) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) S.put(i, S.again(i), S.nbase[i]);
 }
@@ -1505,9 +1507,9 @@ void Octree::small_sort(const double* pos, cudaStream_t s) {
                                      int(small_sort_smem(kSmallMaxPer))));
         attr = true;
     }
-    const int m = std::max(2, div_up(n, kSmallCtas));
+    const int m = std::max(2, div_up(n, kSmallCtas));  // at least 2: the reciprocal then has 32 bits
     // floor(t / m) = mulhi(t, div_m) for every t below kSmallMax: t m < 2^32
-    const unsigned div_m = m > 1 ? unsigned((0x100000000ull + m - 1) / m) : 0u;
+    const unsigned div_m = unsigned((0x100000000ull + m - 1) / m);
     k_small_sort<<<kSmallCtas, kSmallThreads, small_sort_smem(m), s>>>(
         pos, n, m, div_m, double(theta_f), root.as<RootBox>(), key.as<uint64_t>(), perm.as<int>(),
         counts.as<TreeCounts>(), ctx().d_status);
@@ -1673,8 +1675,6 @@ void Octree::refit(const double* pos, const double* mass, cudaStream_t s, cudaSt
     ProfScope ps(kStTreeRefit, s);
     const int grid = div_up(n, kThreads);
     const int span = std::max(node_cap, nn);
-    const int ngrid = div_up(span, kThreads);
-    const int* nn_dev = &counts.as<TreeCounts>()->total_nodes;
     float4* pp = p4.as<float4>();
     float* pd = pdisp.get<float>(n);
     k_gather<<<grid, kThreads, 0, s>>>(n, perm.as<int>(), pos, mass, xbuild.as<double>(), pp, pd,
