@@ -36,8 +36,15 @@ constexpr int kWalkWarps = 4;
 // particles per lane). Thresholds of 2, 4 and 8 measured the same.
 constexpr int kSplitItems = 4;
 // The kernel that can do so also evaluates in batches and takes four blocks per SM, which costs
-// throughput where there are many items: it runs up to this many particles (Engine.gravity at
-// 10k: 386 -> 351 us, sub-steps at 200k 3493 -> 3150 us; at 4M it would take 7230-7350 us, not 7070).
+// throughput where there are many items: it runs up to this many particles, where walks of 6 % of a
+// cloud break even. Few active particles gain at any count, all of them only below 200k. The walk alone in us,
+// with / without it:
+//            all active     6 % active    0.3 % active
+//     100k    172 /  180      74 / 100       68 /  76
+//     200k    317 /  295      96 / 113       68 /  92
+//     400k    524 /  487     141 / 145       78 / 111
+//     800k    979 /  932     258 / 240       84 /  96
+//     1.6M   2270 / 2033     414 / 379       84 / 113
 constexpr int kSplitParticles = 400000;
 constexpr int kStackCap = 1024;   // child ranges per warp
 constexpr int kTileCap = 256;     // interaction entries per warp
